@@ -281,6 +281,20 @@ int swv_block_sparse_attn_fwd(const void* q, const int64_t q_strides[4], const v
                               int kv_group, float* lse, void* o, const int64_t o_strides[4], int o_dtype, int B,
                               int H, int Tq, int Tk, int D, int* status, void* stream);
 
+/* The same with long lists divided over several CTAs (a row block that attends everything, such as
+ * the one holding the CLS tokens, otherwise runs alone past the end of the launch).  `nnz` is the
+ * number of entries of col_idx; the workspace (16-byte aligned, swv_block_sparse_workspace_bytes of the
+ * same sizes, 0 when no list can be long enough) takes the partial rows and is free again when the
+ * launch has completed.
+ */
+int swv_block_sparse_workspace_bytes(int B, int H, int Tq, int Tk, int D, int block, int64_t nnz, size_t* bytes);
+int swv_block_sparse_attn_ws_fwd(const void* q, const int64_t q_strides[4], const void* k, const int64_t k_strides[4],
+                                 const void* v, const int64_t v_strides[4], const int32_t* row_ptr,
+                                 const int32_t* col_idx, int64_t nnz, int block, int mode, int num_cls, int window,
+                                 int dilation, int kv_group, float* lse, void* o, const int64_t o_strides[4],
+                                 int o_dtype, int B, int H, int Tq, int Tk, int D, void* workspace,
+                                 size_t workspace_bytes, int* status, void* stream);
+
 /* Mean pooling of overlapping token windows, y[b,h,c,:] = mean_{i<window} x[b,h,c*stride+i,:],
  * c < (T-window)/stride + 1: the compressed keys and values of the NSA compressed branch
  * (no counterpart in the reference, which only names NSA as an intent,

@@ -19,7 +19,7 @@ EXPORTS = [
     "swv_nsa_importance_bytes", "swv_nsa_select_blocks_fwd", "swv_nsa_selected_attn_fwd", "swv_nsa_combine_fwd",
     "swv_nsa_workspace_bytes", "swv_nsa_attn_fwd", "swv_dsa_attn_scratch_bytes", "swv_dsa_attn_masked_count_fwd",
     "swv_dsa_attn_bwd", "swv_dsa_indexer_bwd", "swv_dsa_prologue_fwd", "swv_dsa_attn_lists_fwd",
-    "swv_dsa_attn_lists_scratch_bytes", "swv_dsa_workspace_bytes_topk",
+    "swv_dsa_attn_lists_scratch_bytes", "swv_dsa_workspace_bytes_topk", "swv_block_sparse_workspace_bytes", "swv_block_sparse_attn_ws_fwd",
 ]
 
 
@@ -51,6 +51,10 @@ def _load():
     lib.swv_block_sparse_attn_fwd.argtypes = [
         c_void_p, i64p, c_void_p, i64p, c_void_p, i64p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
         c_int, c_void_p, c_void_p, i64p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
+    lib.swv_block_sparse_workspace_bytes.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int, c_int64, POINTER(c_size_t)]
+    lib.swv_block_sparse_attn_ws_fwd.argtypes = [
+        c_void_p, i64p, c_void_p, i64p, c_void_p, i64p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int,
+        c_int, c_void_p, c_void_p, i64p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p, c_void_p]
     lib.swv_pool_tokens.argtypes = [c_void_p, i64p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
     lib.swv_rope2d_apply.argtypes = [
         c_void_p, i64p, c_void_p, i64p, c_int, c_void_p, c_int64, c_int, c_int, c_float, c_float, c_int, c_void_p]

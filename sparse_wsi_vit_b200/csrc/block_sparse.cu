@@ -10,19 +10,25 @@
 //             query i sees key j iff  i < C  or  j < C  or
 //             (|i - j| <= W*d and (i - j) % d == 0)      (C CLS tokens first, window W, dilation d)
 //             -- exactly the mask static_sparse_attention.py:159-176 builds.
-// One CTA owns (batch, head, one query block).  The score tile is M = 128 query rows by
-// N = BS keys (BS = 64: the 64 rows behind the block are computed and dropped).
-//   warp 0     : TMA producer (Q once; K, V blocks of the list through 2-stage rings)
-//   warp 1     : UMMA issuer: S(j) = Q K(j)^T into one of TWO score buffers, O += P(j) V(j) with
-//                P read from TMEM; S(j+2) is issued as soon as the softmax has read S(j), so the
-//                tensor pipe works one tile ahead of the softmax
-//   warps 2..9 : online softmax, two threads per query row (one per half of the key columns), ONE
-//                pass per tile: exponentials are
-//                taken against the current stabiliser while the tile's maximum is tracked; only
-//                if some row's maximum exceeds its stabiliser by more than 2^8 is the stabiliser
-//                raised, O (in TMEM) rescaled and the pass repeated (S stays intact: P has its
-//                own columns)
-// TMEM: S fp32 [0,BS) and [BS,2BS) | P (bf16x2) [2BS, 2.5BS) and [2.5BS, 3BS) | O fp32 [3BS, 3BS+D).
+// A CTA owns (batch, head, one query block) or, of a query block whose list is long, one chunk of
+// the list.  The score tile is M = 128 query rows by N = BS keys (BS = 64: the 64 rows behind the
+// block are computed by the tensor core and skipped by the softmax).
+//   warp 0     : TMA producer (Q once; K, V blocks of the list through rings)
+//   warp 1     : UMMA issuer: S(j) = Q K(j)^T, then O += P(j) V(j) with P read from TMEM
+//   warps 2..5 : online softmax, one thread per query row: the row's BS scores are read into registers
+//                once, their maximum is taken, and P is written as bf16 pairs over the first half of the
+//                score columns, in two halves, so that PV starts under the second half's exponentials.
+//                The stabiliser is raised (and O in TMEM rescaled) only when a row's maximum exceeds it
+//                by 2^8.
+// TMEM: S fp32 [0,BS), P (bf16x2) [0,BS/2) over it | O fp32 [BS, BS+D).
+// With P on top of S a CTA needs at most 256 columns and 100 KiB of shared memory, so TWO CTAs share
+// an SM: one CTA's softmax runs under the other's products.  Bound at 128 x 128 x 128 tiles: the chain
+// QK -> softmax -> PV of each CTA (4100 cycles a tile, two tiles in flight; products 1024, exponentials
+// 1024 of the SM's time per tile); 32768 tokens, 16 heads, 5 % of the blocks: 0.82 -> 0.79 ms against one
+// CTA with two score and two probability buffers and eight softmax warps.  Token patterns are evaluated
+// as whole mask words (one arithmetic range per 32 keys; testing every pair took four times the tile's
+// time: 2.5 -> 1.0 ms for the 65536-token sliding window), and lists far longer than the mean are divided
+// (a CLS block over 33 key blocks, 6 heads: 252 -> 44 us).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -47,94 +53,144 @@ struct BsaParams {
   int64_t osb, osh, ost;
   int o_dtype;
   float scale_log2;
+  // Long lists: a query block with more than `chunk` key blocks is divided over ceil(n / chunk) CTAs
+  // (chunk = 0: never).  The first `extra` CTAs of every (batch, head) serve the second and later
+  // chunks.  Partial rows go to `part_o` / `part_ml` (indexed by the chunk's unit), the CTA that
+  // takes the last ticket of the row block adds them up.
+  int chunk, extra;
+  float* part_o;            // [B*H][nQB + extra][BS rows][D] unnormalised fp32 rows
+  float2* part_ml;          // [B*H][nQB + extra][BS rows] (stabiliser, probability sum)
+  uint32_t* tickets;        // [B*H][nQB], zero before the launch
   int* status;
 };
+
+constexpr int kBsaThreads = 192;
 
 struct BsaCtl {
   uint64_t q_full;
   uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2];
-  uint64_t s_full[2], p_full[2], pv_done[2];   // per score / probability buffer (tile parity)
+  uint64_t s_full, p_full[2], pv_done;         // p_full: first and second half of the tile's keys
   uint32_t tmem_base;
   uint32_t abort_flag;
-  float xm[2][kTile][2];                       // per tile parity and row: the tile maximum seen by each column half
-  float xl[kTile][2];                          // per row: the probability sum of each column half
+  int unit[3];                                 // query block, chunk, number of extra units before the query block
+  uint32_t ticket;
+  int scan[kBsaThreads / 32];
 };
 
 template <int BS, int D>
 struct BsaCfg {
+  static constexpr int kStages = BS * D > 8192 ? 1 : 2;   // 128 x 128 blocks: one stage, so that two CTAs fit
   static constexpr int kQBytes = kTile * D * 2;     // 128 query rows
   static constexpr int kKVBytes = BS * D * 2;       // one key / value block
   static constexpr int kOffK = kQBytes;
-  static constexpr int kOffV = kOffK + 2 * kKVBytes;
-  static constexpr int kOffCtl = kOffV + 2 * kKVBytes;
-  static constexpr uint32_t kColP = 2 * BS;          // two probability buffers of BS/2 columns
-  static constexpr uint32_t kColO = 3 * BS;
-  static constexpr uint32_t kTmemCols = (3 * BS + D <= 256) ? 256 : 512;
-  // at least 80 KiB so that no more than two CTAs (2 x 256 TMEM columns) share an SM
+  static constexpr int kOffV = kOffK + kStages * kKVBytes;
+  static constexpr int kOffCtl = kOffV + kStages * kKVBytes;
+  static constexpr uint32_t kColO = BS;
+  static constexpr uint32_t kTmemCols = (BS + D <= 128) ? 128 : 256;
+  static constexpr int kCtas = kTmemCols == 128 ? 3 : 2;  // resident CTAs (registers: 112 and 168 per thread)
+  // at least 80 KiB where 256 columns are used so that no third CTA waits for TMEM
   static constexpr size_t kSmemNeed = 1024 + kOffCtl + sizeof(BsaCtl) + 64;
-  static constexpr size_t kSmem = kSmemNeed > 80 * 1024 ? kSmemNeed : 80 * 1024;
+  static constexpr size_t kSmem = (kTmemCols == 256 && kSmemNeed < 80 * 1024) ? 80 * 1024 : kSmemNeed;
 };
 
-// One softmax pass of a thread over its row of the score tile: p = 2^(s*sc + neg_m) for the kept
-// columns, written as bf16 pairs; returns the row's maximum raw score over the kept columns and
-// the sum of the probabilities.  Loads run one 16-column unit ahead.
-template <int BS, bool MASKED>
-__device__ __forceinline__ void bsa_pass(uint32_t s_col, uint32_t p_col, const uint32_t (&keep)[(BS + 31) / 32], float sc,
-                                         float neg_m, float& mt_out, float& l_out) {
-  const float ninf = -__int_as_float(0x7f800000);
-  float mt0 = ninf, mt1 = ninf, l0 = 0.f, l1 = 0.f;
-  uint32_t sa[16], sb[16];
-  tmem_ld16(s_col, sa);
-#pragma unroll
-  for (int u = 0; u < BS / 16; ++u) {
-    tc_wait_ld();
-    if (u + 1 < BS / 16) {
-      if (u & 1) tmem_ld16(s_col + (u + 1) * 16, sa);
-      else tmem_ld16(s_col + (u + 1) * 16, sb);
+// bits [0, n) of a word, n clamped to [0, 32]
+__device__ __forceinline__ uint32_t low_bits(int n) { return n >= 32 ? 0xFFFFFFFFu : (n <= 0 ? 0u : (1u << n) - 1u); }
+
+// Token-level pattern of the reference's static attention (mode 1) for query `qi` and the 32 keys
+// base..base+31 as a bit mask: the CLS keys, and the window's arithmetic progression.  With window 0 a
+// patch sees the CLS keys only, not itself (static_sparse_attention.py:92-95).
+__device__ __forceinline__ uint32_t static_pattern_word(int qi, int base, int C, int reach, int d) {
+  if (qi < C) return 0xFFFFFFFFu;
+  uint32_t w = low_bits(C - base);
+  if (reach > 0) {
+    uint32_t win = low_bits(qi + reach - base + 1) & ~low_bits(qi - reach - base);
+    if (d > 1 && win != 0u) {
+      int ph = (qi - base) % d;
+      if (ph < 0) ph += d;
+      uint32_t comb = ph < 32 ? 1u << ph : 0u;
+      for (int s = d; s < 32; s <<= 1) comb |= comb << s;
+      win &= comb;
     }
-    const uint32_t w = MASKED ? keep[u >> 1] >> ((u & 1) * 16) : 0xFFFFu;   // (BS = 32: one word)
-    uint32_t packed[8];
-#pragma unroll
-    for (int i = 0; i < 16; i += 2) {
-      const float s0 = __uint_as_float((u & 1) ? sb[i] : sa[i]);
-      const float s1 = __uint_as_float((u & 1) ? sb[i + 1] : sa[i + 1]);
-      float p0 = ex2_approx(fmaf(s0, sc, neg_m));
-      float p1 = ex2_approx(fmaf(s1, sc, neg_m));
-      if (MASKED) {
-        const bool k0 = (w & (1u << i)) != 0u, k1 = (w & (2u << i)) != 0u;
-        mt0 = fmaxf(mt0, k0 ? s0 : ninf);
-        mt1 = fmaxf(mt1, k1 ? s1 : ninf);
-        p0 = k0 ? p0 : 0.f;
-        p1 = k1 ? p1 : 0.f;
-      } else {
-        mt0 = fmaxf(mt0, s0);
-        mt1 = fmaxf(mt1, s1);
-      }
-      l0 += p0;
-      l1 += p1;
-      packed[i >> 1] = pack_bf16x2(p0, p1);
-    }
-    tmem_st8(p_col + u * 8, packed);
+    w |= win;
   }
-  mt_out = fmaxf(mt0, mt1);
-  l_out = l0 + l1;
+  return w;
 }
 
+// max of three / packed pair arithmetic: half the instructions of the scalar forms
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ void fma_pair(float& x, float& y, float a, float b, float sc, float add) {
+  asm("{\n\t.reg .b64 v, s, d;\n\tmov.b64 v, {%2, %3};\n\tmov.b64 s, {%4, %4};\n\tmov.b64 d, {%5, %5};\n\t"
+      "fma.rn.f32x2 v, v, s, d;\n\tmov.b64 {%0, %1}, v;\n\t}"
+      : "=f"(x), "=f"(y)
+      : "f"(a), "f"(b), "f"(sc), "f"(add));
+}
+__device__ __forceinline__ void add_pair(float& x, float& y, float a, float b) {
+  asm("{\n\t.reg .b64 v, s;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 s, {%2, %3};\n\tadd.rn.f32x2 v, v, s;\n\tmov.b64 {%0, %1}, v;\n\t}"
+      : "+f"(x), "+f"(y)
+      : "f"(a), "f"(b));
+}
 
-// Token-level pattern of the reference's static attention (mode 1).
-// With window 0 a patch sees the CLS keys only, not itself (static_sparse_attention.py:92-95).
-__device__ __forceinline__ bool static_pattern(int qi, int kj, int C, int reach, int d) {
-  if (qi < C || kj < C) return true;
-  const int diff = qi - kj;
-  const int ad = diff < 0 ? -diff : diff;
-  return reach > 0 && ad <= reach && (ad % d) == 0;
+// The (query block, chunk) of extra unit `e`: query block r contributes ceil(len_r / chunk) - 1 extra
+// units, in query-block order.  All threads of the CTA take part; returns false past the last unit.
+__device__ __forceinline__ bool bsa_find_extra(const BsaParams& p, int e, BsaCtl* ctl) {
+  if (threadIdx.x == 0) ctl->unit[0] = -1;
+  int before = 0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r0 = 0; r0 < p.nQB; r0 += blockDim.x) {
+    const int r = r0 + threadIdx.x;
+    int n = 0;
+    if (r < p.nQB) n = max(0, (p.row_ptr[r + 1] - p.row_ptr[r] + p.chunk - 1) / p.chunk - 1);
+    int inc = n;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, inc, off);
+      if (lane >= off) inc += t;
+    }
+    if (lane == 31) ctl->scan[warp] = inc;
+    __syncthreads();
+    int base = before, total = 0;
+    for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) {
+      if (w < warp) base += ctl->scan[w];
+      total += ctl->scan[w];
+    }
+    const int first = base + inc - n;
+    if (n > 0 && e >= first && e < first + n) {
+      ctl->unit[0] = r;
+      ctl->unit[1] = e - first + 1;
+      ctl->unit[2] = first;
+    }
+    __syncthreads();
+    if (ctl->unit[0] >= 0) return true;
+    before += total;
+    if (e < before) break;      // (cannot happen: the owner was found above)
+  }
+  return false;
+}
+
+// Number of extra units of the query blocks before `qb` (for the workspace slots of its chunks).
+__device__ __forceinline__ int bsa_extra_before(const BsaParams& p, int qb, BsaCtl* ctl) {
+  int n = 0;
+  for (int r = threadIdx.x; r < qb; r += blockDim.x)
+    n += max(0, (p.row_ptr[r + 1] - p.row_ptr[r] + p.chunk - 1) / p.chunk - 1);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) n += __shfl_xor_sync(0xffffffffu, n, off);
+  if ((threadIdx.x & 31) == 0) ctl->scan[threadIdx.x >> 5] = n;
+  __syncthreads();
+  int t = 0;
+  for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += ctl->scan[w];
+  return t;
 }
 
 template <int BS, int D>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(kBsaThreads, BsaCfg<BS, D>::kCtas)
     block_sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                              const __grid_constant__ CUtensorMap tm_v, const BsaParams p) {
   using Cfg = BsaCfg<BS, D>;
+  constexpr int NST = Cfg::kStages;
   constexpr uint32_t kIdescQK = make_idesc(/*bf16*/ 1, kTile, BS, 0, 0);
   constexpr uint32_t kIdescPV = make_idesc(/*bf16*/ 1, kTile, D, 0, /*V is MN-major*/ 1);
   constexpr float kStep = 8.0f;
@@ -145,27 +201,53 @@ __global__ void __launch_bounds__(320, 1)
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  // query blocks fastest, heads slowest: the CTAs in flight at any time work on one or two heads,
-  // whose keys and values stay in L2 (all heads' K/V together can exceed it)
-  const int qb = blockIdx.x % p.nQB;
-  const int h = (blockIdx.x / p.nQB) % p.H;
-  const int b = blockIdx.x / (p.H * p.nQB);
-  const int list0 = p.row_ptr[qb];
-  const int nblk = p.row_ptr[qb + 1] - list0;
+  // the later chunks of long lists first (they are the longest-running units), then query blocks
+  // fastest, heads slowest: the CTAs in flight at any time work on one or two heads, whose keys and
+  // values stay in L2 (all heads' K/V together can exceed it)
+  int qb, bh, ch = 0, nch = 1, ubase = 0;
+  const int n_extra = p.extra * p.B * p.H;
+  if (static_cast<int>(blockIdx.x) < n_extra) {
+    bh = blockIdx.x / p.extra;
+    if (!bsa_find_extra(p, blockIdx.x % p.extra, ctl)) return;
+    qb = ctl->unit[0];
+    ch = ctl->unit[1];
+    ubase = ctl->unit[2];
+  } else {
+    const int u = blockIdx.x - n_extra;
+    qb = u % p.nQB;
+    bh = u / p.nQB;
+  }
+  const int h = bh % p.H;
+  const int b = bh / p.H;
+  int list0 = p.row_ptr[qb];
+  int nblk = p.row_ptr[qb + 1] - list0;
+  bool peek = false;
+  int first_blk = 0;
+  if (p.chunk > 0 && nblk > p.chunk) {
+    nch = (nblk + p.chunk - 1) / p.chunk;
+    if (ch == 0) ubase = bsa_extra_before(p, qb, ctl);
+    const int a = static_cast<int>(static_cast<int64_t>(nblk) * ch / nch);
+    const int z = static_cast<int>(static_cast<int64_t>(nblk) * (ch + 1) / nch);
+    // A later chunk looks at the list's first block before its own: it starts from the same stabiliser
+    // as the first chunk, so its probabilities round to bf16 exactly as they would in one sweep.
+    peek = ch > 0;
+    first_blk = list0;
+    list0 += a - (peek ? 1 : 0);
+    nblk = z - a + (peek ? 1 : 0);
+  }
 
   if (threadIdx.x == 0) {
     mbar_init(&ctl->q_full, 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < NST; ++s) {
       mbar_init(&ctl->k_full[s], 1);
       mbar_init(&ctl->k_empty[s], 1);
       mbar_init(&ctl->v_full[s], 1);
       mbar_init(&ctl->v_empty[s], 1);
     }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&ctl->s_full[s], 1);
-      mbar_init(&ctl->p_full[s], 8);
-      mbar_init(&ctl->pv_done[s], 1);
-    }
+    mbar_init(&ctl->s_full, 1);
+    mbar_init(&ctl->p_full[0], 4);
+    mbar_init(&ctl->p_full[1], 4);
+    mbar_init(&ctl->pv_done, 1);
     ctl->abort_flag = 0;
     fence_barrier_init();
   }
@@ -191,9 +273,9 @@ __global__ void __launch_bounds__(320, 1)
         tma_load_4d(smem + c * (kTile * 128), &tm_q, &ctl->q_full, c * 64, qb * BS, h, b);
       const int hk = h / p.kv_group;
       for (int j = 0; j < nblk; ++j) {
-        const int s = j & 1;
-        const uint32_t par = ((j >> 1) & 1) ^ 1;
-        const int key0 = checked_index(p.col_idx[list0 + j], (p.Tk + BS - 1) / BS, p.status) * BS;
+        const int s = j % NST;
+        const uint32_t par = ((j / NST) & 1) ^ 1;
+        const int key0 = checked_index(p.col_idx[peek && j == 0 ? first_blk : list0 + j], (p.Tk + BS - 1) / BS, p.status) * BS;
         if (!mbar_wait_bounded(&ctl->k_empty[s], par, abort_flag)) {
           record_status(p.status, kDevWaitStageEmpty);
           break;
@@ -222,12 +304,17 @@ __global__ void __launch_bounds__(320, 1)
       const uint32_t v_addr = smem_u32(smem + Cfg::kOffV);
       bool ok = mbar_wait_bounded(&ctl->q_full, 0, abort_flag);
       if (!ok) record_status(p.status, kDevWaitQ);
-
-      auto issue_qk = [&](int j) -> bool {
-        const int s = j & 1;
-        if (!mbar_wait_bounded(&ctl->k_full[s], (j >> 1) & 1, abort_flag)) {
+      for (int j = 0; ok && j < nblk; ++j) {
+        const int s = j % NST;
+        const uint32_t par = (j / NST) & 1;
+        if (!mbar_wait_bounded(&ctl->k_full[s], par, abort_flag)) {
           record_status(p.status, kDevWaitTmaFull);
-          return false;
+          break;
+        }
+        // S(j) overwrites the columns PV(j-1) reads P from
+        if (j > 0 && !mbar_wait_bounded(&ctl->pv_done, (j - 1) & 1, abort_flag)) {
+          record_status(p.status, kDevWaitPvDone);
+          break;
         }
         tc_fence_after();
         const uint64_t da = smem_desc_sw128(q_addr);
@@ -237,125 +324,105 @@ __global__ void __launch_bounds__(320, 1)
           // 64-element halves of the head dimension are separate swizzled tiles
           const uint64_t offa = (ks >> 2) * (kTile * 128 / 16) + (ks & 3) * 2;
           const uint64_t offb = (ks >> 2) * (BS * 128 / 16) + (ks & 3) * 2;
-          umma_f16_ss(tmem_base + s * BS, da + offa, db + offb, kIdescQK, ks > 0);
+          umma_f16_ss(tmem_base, da + offa, db + offb, kIdescQK, ks > 0);
         }
         umma_commit(&ctl->k_empty[s]);
-        umma_commit(&ctl->s_full[s]);
-        return true;
-      };
-
-      if (ok) ok = issue_qk(0);
-      if (ok && nblk > 1) ok = issue_qk(1);
-      for (int j = 0; ok && j < nblk; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait_bounded(&ctl->v_full[s], (j >> 1) & 1, abort_flag)) {
+        umma_commit(&ctl->s_full);
+        if (!mbar_wait_bounded(&ctl->v_full[s], par, abort_flag)) {
           record_status(p.status, kDevWaitTmaFull);
           break;
         }
-        if (!mbar_wait_bounded(&ctl->p_full[s], (j >> 1) & 1, abort_flag)) {
-          record_status(p.status, kDevWaitPReady);
-          break;
-        }
-        tc_fence_after();
         // V block: rows = keys (128 bytes per 64 head-dim elements), column halves BS*128 bytes apart
         const uint64_t dv = smem_desc_sw128(v_addr + s * Cfg::kKVBytes, BS * 128);
 #pragma unroll
-        for (int ks = 0; ks < BS / 16; ++ks)
-          umma_f16_ts(tmem_base + Cfg::kColO, tmem_base + Cfg::kColP + s * (BS / 2) + ks * 8, dv + ks * 128, kIdescPV,
-                      (j > 0 || ks > 0));
+        for (int half = 0; half < 2; ++half) {
+          if (ok && !mbar_wait_bounded(&ctl->p_full[half], j & 1, abort_flag)) {
+            record_status(p.status, kDevWaitPReady);
+            ok = false;
+          }
+          if (!ok) break;
+          tc_fence_after();
+#pragma unroll
+          for (int ks = half * (BS / 32); ks < (half + 1) * (BS / 32); ++ks)
+            umma_f16_ts(tmem_base + Cfg::kColO, tmem_base + ks * 8, dv + ks * 128, kIdescPV, (j > 0 || ks > 0));
+        }
+        if (!ok) break;
         umma_commit(&ctl->v_empty[s]);
-        umma_commit(&ctl->pv_done[s]);
-        // the softmax has read S(j) (it delivered P(j)): its buffer takes S(j+2)
-        if (j + 2 < nblk) ok = issue_qk(j + 2);
+        umma_commit(&ctl->pv_done);
       }
     }
   } else {
     // ----------------------------------------------------------------- softmax
-    // Eight warps: warp (quarter, half) owns 32 query rows and half of the tile's key columns.  The
-    // two warps of a row quarter exchange their tile maxima through shared memory (one named
-    // barrier per tile), so both take the same decision on raising the stabiliser; each keeps the
-    // probability sum of its columns and rescales / writes its half of the output channels.
-    constexpr int HC = BS / 2;                 // key columns per warp
-    constexpr int DH = D / 2;                  // output channels per warp
     const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;
     const int row = quarter * 32 + lane;
     const int qrow = qb * BS + row;
+    const bool live = quarter * 32 < BS;       // BS = 64: the upper two row quarters hold no query
     const bool row_ok = row < BS && qrow < p.Tq;
-    const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    const uint32_t o_col = lane_base + Cfg::kColO + half * DH;
+    const uint32_t s_col = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t o_col = s_col + Cfg::kColO;
     const float sc = p.scale_log2;
     const float ninf = -__int_as_float(0x7f800000);
     const int reach = p.window * p.dilation;
     const int dil = p.dilation > 0 ? p.dilation : 1;
 
-    float m_used = ninf, l = 0.f;
+    float m_used = ninf;
+    float lh[2] = {0.f, 0.f};                  // probability sums of the two halves of the key columns
     bool ok = true;
+    int key_next = nblk > 0 ? p.col_idx[peek ? first_blk : list0] : 0;
     for (int j = 0; j < nblk; ++j) {
-      const int key0 = checked_index(p.col_idx[list0 + j], (p.Tk + BS - 1) / BS, p.status) * BS;
-      const int sb = j & 1;
-      const uint32_t s_col = lane_base + sb * BS + half * HC;
-      const uint32_t p_col = lane_base + Cfg::kColP + sb * (BS / 2) + half * (HC / 2);
-      // S(j) computed; P's buffer no longer read by PV(j-2).  (A wait that gave up keeps looping
-      // without work: both warps of a quarter pass the same barriers.)
-      if (ok && (!mbar_wait_bounded(&ctl->s_full[sb], (j >> 1) & 1, abort_flag) ||
-                 (j >= 2 && !mbar_wait_bounded(&ctl->pv_done[sb], ((j >> 1) & 1) ^ 1, abort_flag)))) {
+      const int key0 = checked_index(key_next, (p.Tk + BS - 1) / BS, p.status) * BS;
+      if (j + 1 < nblk) key_next = p.col_idx[list0 + j + 1];
+      // S(j) computed, which also means that PV(j-1) has retired (the issuer waited for it)
+      if (!mbar_wait_bounded(&ctl->s_full, j & 1, abort_flag)) {
         record_status(p.status, kDevWaitAccFull);
         ok = false;
       }
+      if (!__all_sync(0xffffffffu, ok)) {        // (the whole warp gives up together)
+        ok = false;
+        break;
+      }
       tc_fence_after();
-      // which of its columns the row attends (bit i of word c = column half*HC + 32c + i)
-      // Token-pattern mode: a block whose every (query, key) pair lies inside the window (no CLS
-      // row or column involved, dilation 1) needs no per-element pattern test.
-      bool inside = false;
-      if (p.mode != 0 && dil == 1 && qb * BS >= p.num_cls && key0 >= p.num_cls) {
-        const int q0 = qb * BS, far = max(q0 + BS - 1 - key0, key0 + BS - 1 - q0);
-        inside = far <= reach;
-      }
-      const bool masked = (p.mode != 0 && !inside) || key0 + BS > p.Tk;
-      uint32_t keep[(HC + 31) / 32];
+      if (live) {
+        uint32_t s[BS];
 #pragma unroll
-      for (int c = 0; c < (HC + 31) / 32; ++c) {
-        uint32_t w = 0xFFFFFFFFu;
-        const int base = key0 + half * HC + c * 32;
-        if (p.mode != 0 && !inside) {
-          w = 0;
-#pragma unroll 4
-          for (int i = 0; i < 32; ++i) {
-            const int kj = base + i;
-            if (kj < p.Tk && static_pattern(qrow, kj, p.num_cls, reach, dil)) w |= 1u << i;
-          }
-        } else if (masked) {
-          const int nv = p.Tk - base;
-          w = nv >= 32 ? 0xFFFFFFFFu : (nv <= 0 ? 0u : ((1u << nv) - 1u));
+        for (int c = 0; c < BS / 32; ++c) tmem_ld32(s_col + c * 32, *reinterpret_cast<uint32_t(*)[32]>(s + c * 32));
+        tc_wait_ld();
+        // Which columns the row attends.  Token-pattern mode: a block whose every (query, key) pair
+        // lies inside the window (no CLS row or column involved, dilation 1) needs no mask.
+        bool inside = false;
+        if (p.mode != 0 && dil == 1 && qb * BS >= p.num_cls && key0 >= p.num_cls) {
+          const int q0 = qb * BS, far = max(q0 + BS - 1 - key0, key0 + BS - 1 - q0);
+          inside = far <= reach;
         }
-        keep[c] = w;
-      }
-
-      // rows that have attended nothing yet have m_used = -inf; their stabiliser is 0 for now
-      float mt = ninf, lt = 0.f;
-      if (ok) {
-        if (masked) bsa_pass<HC, true>(s_col, p_col, keep, sc, (m_used == ninf) ? 0.f : -m_used, mt, lt);
-        else bsa_pass<HC, false>(s_col, p_col, keep, sc, (m_used == ninf) ? 0.f : -m_used, mt, lt);
-      }
-      ctl->xm[sb][row][half] = mt;
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
-      const float m_new = fmaxf(m_used, fmaxf(ctl->xm[sb][row][0], ctl->xm[sb][row][1]) * sc);
-      if (__any_sync(0xffffffffu, m_new > m_used + kStep)) {
-        // raise the stabiliser, rescale what has been accumulated, repeat the pass
-        const float factor = (m_new == m_used) ? 1.f : ex2_approx(m_used - m_new);
-        l *= factor;
-        m_used = m_new;
-        if (j > 0) {
-          // O of the tiles before this one is complete once PV(j-1) retired
-          if (ok && !mbar_wait_bounded(&ctl->pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag)) {
-            record_status(p.status, kDevWaitPvDone);
-            ok = false;
+        if ((p.mode != 0 && !inside) || key0 + BS > p.Tk) {
+#pragma unroll
+          for (int c = 0; c < BS / 32; ++c) {
+            const int base = key0 + c * 32;
+            uint32_t w = low_bits(p.Tk - base);
+            if (p.mode != 0 && !inside) w &= static_pattern_word(qrow, base, p.num_cls, reach, dil);
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (!((w >> i) & 1u)) s[c * 32 + i] = __float_as_uint(ninf);
           }
-          if (ok) {
-            tc_fence_after();
+        }
+        float m0 = ninf, m1 = ninf, m2 = ninf, m3 = ninf;
+#pragma unroll
+        for (int i = 0; i < BS; i += 8) {
+          m0 = max3(m0, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+          m1 = max3(m1, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
+          m2 = max3(m2, __uint_as_float(s[i + 4]), __uint_as_float(s[i + 5]));
+          m3 = max3(m3, __uint_as_float(s[i + 6]), __uint_as_float(s[i + 7]));
+        }
+        const float m_new = fmaxf(m_used, fmaxf(max3(m0, m1, m2), m3) * sc);
+        if (__any_sync(0xffffffffu, m_new > m_used + kStep)) {
+          // raise the stabiliser, rescale what has been accumulated
+          const float factor = (m_new == m_used) ? 1.f : ex2_approx(m_used - m_new);
+          lh[0] *= factor;
+          lh[1] *= factor;
+          m_used = m_new;
+          if (j > 0) {
 #pragma unroll 1
-            for (int c = 0; c < DH / 16; ++c) {
+            for (int c = 0; c < D / 16; ++c) {
               uint32_t o[16];
               tmem_ld16(o_col + c * 16, o);
               tc_wait_ld();
@@ -363,40 +430,118 @@ __global__ void __launch_bounds__(320, 1)
               for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
               tmem_st16(o_col + c * 16, o);
             }
-            tc_wait_st();
           }
         }
-        if (ok) {
-          if (masked) bsa_pass<HC, true>(s_col, p_col, keep, sc, (m_used == ninf) ? 0.f : -m_used, mt, lt);
-          else bsa_pass<HC, false>(s_col, p_col, keep, sc, (m_used == ninf) ? 0.f : -m_used, mt, lt);
+        // rows that have attended nothing yet have m_used = -inf; their stabiliser is 0 for now
+        // (the looked-at block of a later chunk contributes nothing)
+        const float neg_m = peek && j == 0 ? ninf : ((m_used == ninf) ? 0.f : -m_used);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          float l0 = 0.f, l1 = 0.f;
+#pragma unroll
+          for (int u = half * (BS / 32); u < (half + 1) * (BS / 32); ++u) {
+            uint32_t packed[8];
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              float x0, x1;
+              fma_pair(x0, x1, __uint_as_float(s[u * 16 + i]), __uint_as_float(s[u * 16 + i + 1]), sc, neg_m);
+              x0 = ex2_approx(x0);
+              x1 = ex2_approx(x1);
+              add_pair(l0, l1, x0, x1);
+              packed[i >> 1] = pack_bf16x2(x0, x1);
+            }
+            tmem_st8(s_col + u * 8, packed);
+          }
+          lh[half] += l0 + l1;
+          tc_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl->p_full[half]);
         }
+      } else if (lane == 0) {
+        mbar_arrive(&ctl->p_full[0]);
+        mbar_arrive(&ctl->p_full[1]);
       }
-      l += lt;
-      tc_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (ok && lane == 0) mbar_arrive(&ctl->p_full[sb]);
     }
 
-    if (nblk > 0 && ok && !mbar_wait_bounded(&ctl->pv_done[(nblk - 1) & 1], ((nblk - 1) >> 1) & 1, abort_flag)) {
+    if (nblk > 0 && ok && !mbar_wait_bounded(&ctl->pv_done, (nblk - 1) & 1, abort_flag)) {
       record_status(p.status, kDevWaitPvDone);
       ok = false;
     }
-    // the row's probability sum: both column halves
-    ctl->xl[row][half] = l;
-    asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
-    l = ctl->xl[row][0] + ctl->xl[row][1];
-    if (ok) {
-      tc_fence_after();
+    float l = lh[0] + lh[1];
+    tc_fence_after();
+
+    // One chunk of a long list: leave the unnormalised rows, take a ticket; the last CTA of the query
+    // block goes on with the sum over all chunks.
+    const int64_t units = p.nQB + p.extra;
+    bool writer = true;
+    if (nch > 1) {
+      const int64_t u = bh * units + (ch == 0 ? qb : p.nQB + ubase + ch - 1);
+      if (ok) {
+        if (row_ok) p.part_ml[u * BS + row] = make_float2(m_used, l);
+        float* po = p.part_o + (u * BS + row) * D;
+#pragma unroll 1
+        for (int c = 0; c < D / 16; ++c) {
+          uint32_t o[16];
+          tmem_ld16(o_col + c * 16, o);
+          tc_wait_ld();
+          if (!row_ok) continue;
+#pragma unroll
+          for (int i = 0; i < 16; i += 4)
+            *reinterpret_cast<uint4*>(po + c * 16 + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+        }
+      }
+      __threadfence();
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (threadIdx.x == 64) ctl->ticket = atomicAdd(p.tickets + static_cast<int64_t>(bh) * p.nQB + qb, 1u);
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      writer = ctl->ticket + 1 == static_cast<uint32_t>(nch);
+      if (writer) __threadfence();
+    }
+    if (ok && writer) {
+      float wgt_m = m_used;
+      if (nch > 1 && row_ok) {
+        for (int c = 0; c < nch; ++c) {
+          const int64_t u = bh * units + (c == 0 ? qb : p.nQB + ubase + c - 1);
+          wgt_m = fmaxf(wgt_m, __ldcg(p.part_ml + u * BS + row).x);
+        }
+        l = 0.f;
+        for (int c = 0; c < nch; ++c) {
+          const int64_t u = bh * units + (c == 0 ? qb : p.nQB + ubase + c - 1);
+          const float2 ml = __ldcg(p.part_ml + u * BS + row);
+          if (ml.x != ninf) l += ml.y * ex2_approx(ml.x - wgt_m);
+        }
+      }
       const float inv = l > 0.f ? 1.f / l : 0.f;
-      if (p.lse != nullptr && row_ok && half == 0) {
+      if (p.lse != nullptr && row_ok) {
         p.lse[(static_cast<int64_t>(b) * p.H + h) * p.Tq + qrow] =
-            l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : ninf;
+            l > 0.f ? (wgt_m + log2f(l)) * 0.6931471805599453f : ninf;
       }
 #pragma unroll 1
-      for (int c = 0; c < DH / 16; ++c) {
+      for (int c = 0; c < D / 16; ++c) {
         uint32_t o[16];
-        if (nblk > 0) {
+        if (nch > 1) {
+          float acc[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+          for (int k = 0; row_ok && k < nch; ++k) {
+            const int64_t u = bh * units + (k == 0 ? qb : p.nQB + ubase + k - 1);
+            const float mk = __ldcg(p.part_ml + u * BS + row).x;
+            if (mk == ninf) continue;
+            const float f = ex2_approx(mk - wgt_m);
+            const float4* po = reinterpret_cast<const float4*>(p.part_o + (u * BS + row) * D + c * 16);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float4 v = __ldcg(po + i);
+              acc[4 * i] = fmaf(v.x, f, acc[4 * i]);
+              acc[4 * i + 1] = fmaf(v.y, f, acc[4 * i + 1]);
+              acc[4 * i + 2] = fmaf(v.z, f, acc[4 * i + 2]);
+              acc[4 * i + 3] = fmaf(v.w, f, acc[4 * i + 3]);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(acc[i]);
+        } else if (nblk > 0) {
           tmem_ld16(o_col + c * 16, o);
           tc_wait_ld();
         } else {
@@ -410,8 +555,7 @@ __global__ void __launch_bounds__(320, 1)
           const float gl = p.gate[((static_cast<int64_t>(b) * p.Tq + qrow) * p.H + h) * 3 + p.gate_idx];
           const float gs = 1.f / (1.f + __expf(-gl));
           const float* arow = p.acc_in == nullptr ? nullptr
-                                                  : p.acc_in + ((static_cast<int64_t>(b) * p.H + h) * p.Tq + qrow) * D +
-                                                        half * DH + c * 16;
+                                                  : p.acc_in + ((static_cast<int64_t>(b) * p.H + h) * p.Tq + qrow) * D + c * 16;
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const float a = __uint_as_float(o[i]) * inv;
@@ -420,7 +564,7 @@ __global__ void __launch_bounds__(320, 1)
         }
         const float inv_w = p.gate != nullptr ? 1.f : inv;      // (already applied above)
         if (p.o_dtype == SWV_F32) {
-          float* orow = static_cast<float*>(p.o) + b * p.osb + h * p.osh + qrow * p.ost + half * DH + c * 16;
+          float* orow = static_cast<float*>(p.o) + b * p.osb + h * p.osh + qrow * p.ost + c * 16;
 #pragma unroll
           for (int i = 0; i < 16; i += 4) {
             *reinterpret_cast<float4*>(orow + i) =
@@ -428,7 +572,7 @@ __global__ void __launch_bounds__(320, 1)
                             __uint_as_float(o[i + 2]) * inv_w, __uint_as_float(o[i + 3]) * inv_w);
           }
         } else {
-          uint16_t* orow = static_cast<uint16_t*>(p.o) + b * p.osb + h * p.osh + qrow * p.ost + half * DH + c * 16;
+          uint16_t* orow = static_cast<uint16_t*>(p.o) + b * p.osb + h * p.osh + qrow * p.ost + c * 16;
 #pragma unroll
           for (int i = 0; i < 16; i += 8) {
             uint32_t w4[4];
@@ -544,9 +688,43 @@ static int launch_bsa(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   using Cfg = BsaCfg<BS, D>;
   SWV_CUDA_OK(cudaFuncSetAttribute(block_sparse_attn_kernel<BS, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(Cfg::kSmem)));
-  const unsigned grid = static_cast<unsigned>(p.B) * p.nQB * p.H;
-  block_sparse_attn_kernel<BS, D><<<grid, 320, Cfg::kSmem, st>>>(tq, tk, tv, p);
+  const unsigned grid = static_cast<unsigned>(p.B) * (p.nQB + p.extra) * p.H;
+  block_sparse_attn_kernel<BS, D><<<grid, kBsaThreads, Cfg::kSmem, st>>>(tq, tk, tv, p);
   SWV_CUDA_OK(cudaGetLastError());
+  return SWV_OK;
+}
+
+// How long lists are divided, from the sizes the host knows (`nnz` = entries of col_idx).  A chunk is
+// never shorter than 8 key blocks (a partial row block costs about one block's time to write and read
+// back), than twice the mean list (regular lists stay whole), or than an even share of all work over
+// the resident CTAs (a list below that does not reach past the end of the launch).
+struct BsaSplit {
+  int chunk = 0, extra = 0;
+  size_t o_bytes = 0, ml_bytes = 0, ticket_bytes = 0;
+};
+static BsaSplit bsa_split(int B, int H, int nQB, int nKB, int block, int D, int64_t nnz) {
+  BsaSplit s;
+  if (nnz <= 0) return s;
+  const int64_t slots = static_cast<int64_t>(sm_count()) * (block + D <= 128 ? 3 : 2);
+  const int64_t mean2 = (2 * nnz + nQB - 1) / nQB, share = (nnz * B * H + slots - 1) / slots;
+  const int64_t chunk = mean2 > share ? (mean2 > 8 ? mean2 : 8) : (share > 8 ? share : 8);
+  if (chunk >= nKB) return s;                       // no list can be longer
+  s.chunk = static_cast<int>(chunk);
+  s.extra = static_cast<int>(nnz / chunk);          // sum over rows of ceil(n / chunk) - 1 <= nnz / chunk
+  if (s.extra == 0) s.chunk = 0;
+  const size_t rows = static_cast<size_t>(B) * H * (nQB + s.extra) * block;
+  s.o_bytes = rows * D * sizeof(float);
+  s.ml_bytes = rows * sizeof(float2);
+  s.ticket_bytes = static_cast<size_t>(B) * H * nQB * sizeof(uint32_t);
+  return s;
+}
+
+int block_sparse_workspace_bytes_impl(int B, int H, int Tq, int Tk, int D, int block, int64_t nnz, size_t* bytes) {
+  if (!bytes) return SWV_ERR_NULL;
+  if (B < 1 || H < 1 || Tq < 1 || Tk < 1 || nnz < 0) return SWV_ERR_SHAPE;
+  if ((block != 64 && block != 128) || (D != 64 && D != 128)) return SWV_ERR_UNSUPPORTED;
+  const BsaSplit s = bsa_split(B, H, (Tq + block - 1) / block, (Tk + block - 1) / block, block, D, nnz);
+  *bytes = s.extra > 0 ? s.o_bytes + s.ml_bytes + s.ticket_bytes : 0;
   return SWV_OK;
 }
 
@@ -554,7 +732,8 @@ int block_sparse_attn_impl(const void* q, const int64_t* qs, const void* k, cons
                            const int64_t* vs, const int32_t* row_ptr, const int32_t* col_idx, int block, int mode,
                            int num_cls, int window, int dilation, int kv_group, float* lse, void* o,
                            const int64_t* os, int o_dtype, int B, int H, int Tq, int Tk, int D, int* status,
-                           cudaStream_t st, const float* gate, int gate_idx, const float* acc_in) {
+                           cudaStream_t st, const float* gate, int gate_idx, const float* acc_in, int64_t nnz,
+                           void* workspace, size_t workspace_bytes) {
   if (!q || !k || !v || !row_ptr || !col_idx || !o || !status || !qs || !ks || !vs || !os) return SWV_ERR_NULL;
   if (B < 1 || H < 1 || Tq < 1 || Tk < 1) return SWV_ERR_SHAPE;
   if (kv_group < 1 || H % kv_group != 0) return SWV_ERR_SHAPE;
@@ -592,6 +771,21 @@ int block_sparse_attn_impl(const void* q, const int64_t* qs, const void* k, cons
   p.o = o; p.osb = os[0]; p.osh = os[1]; p.ost = os[2]; p.o_dtype = o_dtype;
   p.scale_log2 = 1.4426950408889634f / sqrtf(static_cast<float>(D));
   p.status = status;
+  p.chunk = 0; p.extra = 0;
+  p.part_o = nullptr; p.part_ml = nullptr; p.tickets = nullptr;
+  if (workspace != nullptr) {
+    const BsaSplit s = bsa_split(B, H, p.nQB, (Tk + block - 1) / block, block, D, nnz);
+    if (s.extra > 0) {
+      if (workspace_bytes < s.o_bytes + s.ml_bytes + s.ticket_bytes) return SWV_ERR_WORKSPACE;
+      if (!bsa_aligned16(workspace)) return SWV_ERR_ALIGN;
+      uint8_t* w = static_cast<uint8_t*>(workspace);
+      p.chunk = s.chunk; p.extra = s.extra;
+      p.part_o = reinterpret_cast<float*>(w);
+      p.part_ml = reinterpret_cast<float2*>(w + s.o_bytes);
+      p.tickets = reinterpret_cast<uint32_t*>(w + s.o_bytes + s.ml_bytes);
+      SWV_CUDA_OK(cudaMemsetAsync(p.tickets, 0, s.ticket_bytes, st));
+    }
+  }
   if (block == 64 && D == 64) return launch_bsa<64, 64>(tq, tk, tv, p, st);
   if (block == 64 && D == 128) return launch_bsa<64, 128>(tq, tk, tv, p, st);
   if (block == 128 && D == 64) return launch_bsa<128, 64>(tq, tk, tv, p, st);

@@ -35,7 +35,9 @@ int block_sparse_attn_impl(const void* q, const int64_t* qs, const void* k, cons
                            const int64_t* vs, const int32_t* row_ptr, const int32_t* col_idx, int block, int mode,
                            int num_cls, int window, int dilation, int kv_group, float* lse, void* o,
                            const int64_t* os, int o_dtype, int B, int H, int Tq, int Tk, int D, int* status,
-                           cudaStream_t st, const float* gate, int gate_idx, const float* acc_in);
+                           cudaStream_t st, const float* gate, int gate_idx, const float* acc_in, int64_t nnz,
+                           void* workspace, size_t workspace_bytes);
+int block_sparse_workspace_bytes_impl(int B, int H, int Tq, int Tk, int D, int block, int64_t nnz, size_t* bytes);
 int pool_tokens_impl(const void* x, const int64_t* xs, void* y, int B, int H, int T, int D, int win, int stride,
                      cudaStream_t st);
 int rope2d_impl(const void* x, const int64_t* xs, void* y, const int64_t* ys, int dtype, const float* coords,
@@ -215,7 +217,23 @@ int swv_block_sparse_attn_fwd(const void* q, const int64_t q_strides[4], const v
                               int H, int Tq, int Tk, int D, int* status, void* stream) {
   return swv::block_sparse_attn_impl(q, q_strides, k, k_strides, v, v_strides, row_ptr, col_idx, block, mode, num_cls,
                                      window, dilation, kv_group, lse, o, o_strides, o_dtype, B, H, Tq, Tk, D, status,
-                                     static_cast<cudaStream_t>(stream), nullptr, 0, nullptr);
+                                     static_cast<cudaStream_t>(stream), nullptr, 0, nullptr, 0, nullptr, 0);
+}
+
+int swv_block_sparse_workspace_bytes(int B, int H, int Tq, int Tk, int D, int block, int64_t nnz, size_t* bytes) {
+  return swv::block_sparse_workspace_bytes_impl(B, H, Tq, Tk, D, block, nnz, bytes);
+}
+
+int swv_block_sparse_attn_ws_fwd(const void* q, const int64_t q_strides[4], const void* k, const int64_t k_strides[4],
+                                 const void* v, const int64_t v_strides[4], const int32_t* row_ptr,
+                                 const int32_t* col_idx, int64_t nnz, int block, int mode, int num_cls, int window,
+                                 int dilation, int kv_group, float* lse, void* o, const int64_t o_strides[4],
+                                 int o_dtype, int B, int H, int Tq, int Tk, int D, void* workspace,
+                                 size_t workspace_bytes, int* status, void* stream) {
+  return swv::block_sparse_attn_impl(q, q_strides, k, k_strides, v, v_strides, row_ptr, col_idx, block, mode, num_cls,
+                                     window, dilation, kv_group, lse, o, o_strides, o_dtype, B, H, Tq, Tk, D, status,
+                                     static_cast<cudaStream_t>(stream), nullptr, 0, nullptr, nnz, workspace,
+                                     workspace_bytes);
 }
 
 int swv_pool_tokens(const void* x, const int64_t x_strides[4], void* y, int B, int H, int T, int D, int window,

@@ -798,7 +798,8 @@ int block_sparse_attn_impl(const void* q, const int64_t* qs, const void* k, cons
                            const int64_t* vs, const int32_t* row_ptr, const int32_t* col_idx, int block, int mode,
                            int num_cls, int window, int dilation, int kv_group, float* lse, void* o,
                            const int64_t* os, int o_dtype, int B, int H, int Tq, int Tk, int D, int* status,
-                           cudaStream_t st, const float* gate, int gate_idx, const float* acc_in);
+                           cudaStream_t st, const float* gate, int gate_idx, const float* acc_in, int64_t nnz,
+                           void* workspace, size_t workspace_bytes);
 
 struct NsaLayout {
   size_t kc, vc, acc, lse, imp, blocks, full_ptr, full_col, win_ptr, win_col, total;
@@ -881,7 +882,7 @@ int nsa_attn_impl(const void* q, const int64_t* qs, const void* k, const int64_t
   // its own.
   // compressed branch (all compressed tokens, log-sum-exp kept for the selection)
   rc = block_sparse_attn_impl(q, qs, kc, cs, vc, cs, full_ptr, full_col, kTile, 0, 0, 0, 1, G, lse, acc, os,
-                              SWV_F32, B, Hq, T, L.nC, D, status, st, gate, 0, nullptr);
+                              SWV_F32, B, Hq, T, L.nC, D, status, st, gate, 0, nullptr, 0, nullptr, 0);
   if (rc != SWV_OK) return rc;
   // selection + selected branch
   size_t imp_bytes = 0;
@@ -893,7 +894,7 @@ int nsa_attn_impl(const void* q, const int64_t* qs, const void* k, const int64_t
   if (rc != SWV_OK) return rc;
   // sliding-window branch: token pattern |i - j| <= window / 2 inside the listed blocks
   rc = block_sparse_attn_impl(q, qs, k, ks, v, vs, win_ptr, win_col, kTile, 1, 0, reach, 1, G, nullptr, out, os,
-                              out_dtype, B, Hq, T, T, D, status, st, gate, 2, acc);
+                              out_dtype, B, Hq, T, T, D, status, st, gate, 2, acc, 0, nullptr, 0);
   if (rc != SWV_OK) return rc;
   if (blocks_out != nullptr)
     SWV_CUDA_OK(cudaMemcpyAsync(blocks_out, blocks, static_cast<size_t>(B) * Hkv * T * L.k_eff * 4,

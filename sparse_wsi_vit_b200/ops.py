@@ -513,11 +513,16 @@ def block_sparse_attention(q, k, v, row_ptr, col_idx, block, mode=0, num_cls=0, 
     o = torch.empty((B, H, Tq, D), dtype=out_dtype, device=dev)
     lse = torch.empty((B, H, Tq), dtype=torch.float32, device=dev) if return_lse else None
     st = status_word(dev)
-    rc = lib.swv_block_sparse_attn_fwd(
+    nnz = col_idx.numel()
+    nws = ctypes.c_size_t()
+    check(lib.swv_block_sparse_workspace_bytes(B, H, Tq, Tk, D, block, nnz, ctypes.byref(nws)),
+          "swv_block_sparse_workspace_bytes")
+    ws = torch.empty(nws.value, dtype=torch.uint8, device=dev) if nws.value else None
+    rc = lib.swv_block_sparse_attn_ws_fwd(
         q.data_ptr(), strides(q), k.data_ptr(), strides(k), v.data_ptr(), strides(v), row_ptr.data_ptr(),
-        col_idx.data_ptr(), block, mode, num_cls, window, dilation, kv_group,
+        col_idx.data_ptr(), nnz, block, mode, num_cls, window, dilation, kv_group,
         lse.data_ptr() if return_lse else None, o.data_ptr(), strides(o), dtype_code(o.dtype),
-        B, H, Tq, Tk, D, st.data_ptr(), _stream(dev))
+        B, H, Tq, Tk, D, None if ws is None else ws.data_ptr(), nws.value, st.data_ptr(), _stream(dev))
     check(rc, "swv_block_sparse_attn_fwd")
     if _CHECK:
         check_status(dev, "swv_block_sparse_attn_fwd")

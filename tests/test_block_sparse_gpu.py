@@ -57,6 +57,27 @@ def test_block_mask_vs_oracle(swv, T, H, D, block):
     _check_vs_oracle(swv, q, k, v, rp, ci, block)
 
 
+@pytest.mark.parametrize("nb,D,block,long_rows", [(40, 64, 64, (0,)), (21, 128, 128, (3, 20)), (35, 64, 128, (0, 1, 34)),
+                                                  (19, 128, 64, (18,))])
+def test_long_lists_are_divided(swv, nb, D, block, long_rows):
+    """A few query blocks that attend everything among short ones (an empty one too): their lists are
+    divided over several CTAs and the partial rows added up by the last of them; the last block is
+    ragged.  Rows outside the long ones must not notice."""
+    T = nb * block - 37
+    rows = [list(range(nb)) if r in long_rows else ([] if r == 5 else sorted({r, (7 * r) % nb})) for r in range(nb)]
+    rp, ci = swv.patterns._to_csr(rows)
+    q, k, v = _qkv(T, 2, D, seed=nb)
+    o = _check_vs_oracle(swv, q, k, v, rp, ci, block)
+    again = swv.block_sparse_attention(*_dev(q, k, v), torch.from_numpy(rp).to(DEV), torch.from_numpy(ci).to(DEV), block,
+                                       out_dtype=torch.float32, return_lse=True)
+    assert torch.equal(o, again[0])
+    mask = S.expand_block_mask(rp, ci, block, T, T, rows=None)
+    s = (q[0].float() @ k[0].float().transpose(1, 2)) / D ** 0.5
+    ref = torch.logsumexp(s.masked_fill(~mask, float("-inf")), dim=-1)
+    seen = mask.any(-1)
+    assert (again[1][0].cpu() - ref)[:, seen].abs().max() < 1e-3
+
+
 def test_empty_rows_and_full_list(swv):
     T, H, D, block = 512, 2, 64, 128
     q, k, v = _qkv(T, H, D, seed=3)
