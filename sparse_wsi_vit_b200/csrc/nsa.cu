@@ -14,7 +14,7 @@
 //                           (TMA rings -> tcgen05 -> two TMEM accumulators), eight epilogue warps
 //                           turn scores into probabilities and add them up per selection block.
 //   nsa_select_kernel     : one warp per (b, g, t): iterative arg-max over the importance row.
-//   nsa_selected_attn_mma_kernel : one warp per (b, g, t), the G heads as rows of mma.sync tiles: every
+//   nsa_selected_attn_mma_kernel : one warp per (b, g, t), the G heads as columns of mma.sync tiles: every
 //                           selected key / value row is read once for the whole group
 //                           (nsa_selected_attn_kernel: the same on CUDA cores, for unaligned layouts).
 //   nsa_combine_kernel    : out = sum_b sigmoid(gate_b) * O_b.
@@ -35,7 +35,7 @@ struct NsaImpParams {
 };
 
 struct NsaImpCtl {
-  uint64_t q_full[2], q_empty[2], k_full[2], k_empty[2], acc_full[2], acc_empty[2];
+  uint64_t q_full[2], q_empty[2], k_full, k_empty, acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   uint32_t abort_flag;
 };
@@ -45,15 +45,19 @@ constexpr int kNsaMaxGroup = 16;
 template <int D>
 struct NsaImpCfg {
   static constexpr int kTileBytes = kTile * D * 2;
-  static constexpr int kOffK = 2 * kTileBytes;
-  static constexpr int kOffLse = 4 * kTileBytes;
+  static constexpr int kOffK = 2 * kTileBytes;          // (two Q stages, one K stage: a K tile serves G products)
+  static constexpr int kOffLse = 3 * kTileBytes;
   static constexpr int kOffCtl = kOffLse + kNsaMaxGroup * kTile * 4;
   static constexpr size_t kSmem = 1024 + kOffCtl + sizeof(NsaImpCtl) + 64;
 };
 
 // R = compressed tokens per selection block (selection block size / compression stride).
+// Two CTAs per SM (104 KiB, 256 TMEM columns each): the exponentials are the bound (one per score,
+// 1024 of the SM's cycles per 128x128 tile against 512 of tensor time), and the eight epilogue warps of
+// one CTA alone leave their unit idle at every tile's hand-over (65536 tokens, 16 heads, D = 128:
+// 1.60 -> 1.34 ms).
 template <int D, int R>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(320, 2)
     nsa_importance_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                           const NsaImpParams p) {
   using Cfg = NsaImpCfg<D>;
@@ -77,11 +81,11 @@ __global__ void __launch_bounds__(320, 1)
     for (int s = 0; s < 2; ++s) {
       mbar_init(&ctl->q_full[s], 1);
       mbar_init(&ctl->q_empty[s], 1);
-      mbar_init(&ctl->k_full[s], 1);
-      mbar_init(&ctl->k_empty[s], 1);
       mbar_init(&ctl->acc_full[s], 1);
       mbar_init(&ctl->acc_empty[s], 8);
     }
+    mbar_init(&ctl->k_full, 1);
+    mbar_init(&ctl->k_empty, 1);
     ctl->abort_flag = 0;
     fence_barrier_init();
   }
@@ -112,16 +116,14 @@ __global__ void __launch_bounds__(320, 1)
           tma_load_4d(smem + s * Cfg::kTileBytes + c * (kTile * 128), &tm_q, &ctl->q_full[s], c * 64, qt * kTile,
                       g * G + hh, b);
         if (hh == 0) {
-          const int ks = jt & 1;
-          if (!mbar_wait_bounded(&ctl->k_empty[ks], ((jt >> 1) & 1) ^ 1, abort_flag)) {
+          if (!mbar_wait_bounded(&ctl->k_empty, (jt & 1) ^ 1, abort_flag)) {
             record_status(p.status, kDevWaitStageEmpty);
             break;
           }
-          mbar_expect_tx(&ctl->k_full[ks], Cfg::kTileBytes);
+          mbar_expect_tx(&ctl->k_full, Cfg::kTileBytes);
 #pragma unroll
           for (int c = 0; c < D / 64; ++c)
-            tma_load_4d(smem + Cfg::kOffK + ks * Cfg::kTileBytes + c * (kTile * 128), &tm_k, &ctl->k_full[ks], c * 64,
-                        jt * kTile, g, b);
+            tma_load_4d(smem + Cfg::kOffK + c * (kTile * 128), &tm_k, &ctl->k_full, c * 64, jt * kTile, g, b);
         }
       }
     }
@@ -131,9 +133,9 @@ __global__ void __launch_bounds__(320, 1)
       const uint32_t q_addr = smem_u32(smem);
       const uint32_t k_addr = smem_u32(smem + Cfg::kOffK);
       for (int it = 0; it < nIt; ++it) {
-        const int jt = it / G, hh = it - jt * G, s = it & 1, ks = jt & 1;
+        const int jt = it / G, hh = it - jt * G, s = it & 1;
         if (!mbar_wait_bounded(&ctl->q_full[s], (it >> 1) & 1, abort_flag) ||
-            (hh == 0 && !mbar_wait_bounded(&ctl->k_full[ks], (jt >> 1) & 1, abort_flag))) {
+            (hh == 0 && !mbar_wait_bounded(&ctl->k_full, jt & 1, abort_flag))) {
           record_status(p.status, kDevWaitTmaFull);
           break;
         }
@@ -143,7 +145,7 @@ __global__ void __launch_bounds__(320, 1)
         }
         tc_fence_after();
         const uint64_t da = smem_desc_sw128(q_addr + s * Cfg::kTileBytes);
-        const uint64_t db = smem_desc_sw128(k_addr + ks * Cfg::kTileBytes);
+        const uint64_t db = smem_desc_sw128(k_addr);
 #pragma unroll
         for (int k16 = 0; k16 < D / 16; ++k16) {
           // 64-element halves of the head dimension are separate swizzled tiles
@@ -151,7 +153,7 @@ __global__ void __launch_bounds__(320, 1)
           umma_f16_ss(tmem_base + s * kTile, da + off, db + off, kIdesc, k16 > 0);
         }
         umma_commit(&ctl->q_empty[s]);
-        if (hh == G - 1) umma_commit(&ctl->k_empty[ks]);
+        if (hh == G - 1) umma_commit(&ctl->k_empty);
         umma_commit(&ctl->acc_full[s]);
       }
     }
@@ -235,19 +237,18 @@ __global__ void __launch_bounds__(320, 1)
 }
 
 // ------------------------------------------------------------------- select
-// One warp per (b, g, t).  Importance values are >= 0; taken entries are marked -1, entries
-// behind the last selection block -2.  Ties go to the lower block index; output ascending.
-__global__ void __launch_bounds__(128) nsa_select_kernel(const float* __restrict__ imp, int n_pad, int n_s, int k_eff,
-                                                         int64_t rows, int32_t* __restrict__ blocks) {
-  extern __shared__ float sel_sm[];
-  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t r = static_cast<int64_t>(blockIdx.x) * 4 + wib;
-  if (r >= rows) return;
-  const int n = (n_s + 31) & ~31;                     // scanned range, a multiple of 32
-  float* v = sel_sm + wib * n;
-  const float* src = imp + r * n_pad;
-  for (int i = lane; i < n; i += 32) v[i] = i < n_s ? (i < n_pad ? src[i] : 0.f) : -2.f;
-  __syncwarp();
+// One warp per (b, g, t).  Importance values are >= 0; entries behind the last selection block count as
+// -2.  Ties go to the lower block index; output ascending.
+//
+// Short form (k_eff <= 32, at most 32 * NPL blocks, the row in registers, entry i * 32 + lane): the
+// k-th largest of the 32 lane maxima is a lower bound of the k-th largest entry, and on real rows only a
+// few dozen entries reach it.  They are compacted in index order, and each counts how many of the others
+// come before it.  A row with more than 64 of them (plateaus of equal values) takes the arg-max loop.
+// Bound by instruction issue, ~500 per row of 1024 entries; the loop below needs ~2500 (65536 tokens, 2
+// kv heads, 1024 blocks: 0.64 -> 0.17 ms).
+constexpr int kSelCand = 64;
+
+__device__ __forceinline__ void nsa_argmax_loop(float* v, int n, int k_eff, int lane, int32_t* dst) {
   for (int s = 0; s < k_eff; ++s) {
     float best = -3.f;
     int bi = 0x7fffffff;
@@ -267,10 +268,9 @@ __global__ void __launch_bounds__(128) nsa_select_kernel(const float* __restrict
         bi = oi;
       }
     }
-    if (lane == 0) v[bi] = -1.f;
+    if (lane == 0) v[bi] = -1.f;                      // taken
     __syncwarp();
   }
-  int32_t* dst = blocks + r * k_eff;
   int cnt = 0;
   for (int i0 = 0; i0 < n; i0 += 32) {
     const bool taken = v[i0 + lane] == -1.f;
@@ -278,6 +278,90 @@ __global__ void __launch_bounds__(128) nsa_select_kernel(const float* __restrict
     if (taken) dst[cnt + __popc(m & ((1u << lane) - 1u))] = i0 + lane;
     cnt += __popc(m);
   }
+}
+
+template <int NPL>
+__global__ void __launch_bounds__(128) nsa_select_short_kernel(const float* __restrict__ imp, int n_pad, int n_s,
+                                                               int k_eff, int64_t rows, int32_t* __restrict__ blocks) {
+  __shared__ float row_sm[4][NPL * 32];               // the arg-max loop's copy; first kSelCand: candidate values
+  __shared__ int idx_sm[4][kSelCand];
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t r = static_cast<int64_t>(blockIdx.x) * 4 + wib;
+  if (r >= rows) return;
+  const float* src = imp + r * n_pad;
+  float v[NPL];
+  float mx = -2.f;
+#pragma unroll
+  for (int i = 0; i < NPL; ++i) {
+    const int e = i * 32 + lane;
+    v[i] = e < n_s ? (e < n_pad ? __ldg(src + e) : 0.f) : -2.f;
+    mx = fmaxf(mx, v[i]);
+  }
+  // the k-th largest lane maximum: the one whose rank (ties by lane) is k - 1
+  int rank = 0;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    const float o = __shfl_sync(0xffffffffu, mx, j);
+    rank += (o > mx || (o == mx && j < lane)) ? 1 : 0;
+  }
+  const float bound = __shfl_sync(0xffffffffu, mx, __ffs(__ballot_sync(0xffffffffu, rank == k_eff - 1)) - 1);
+  float* cv = row_sm[wib];
+  int* ci = idx_sm[wib];
+  int n = 0;
+#pragma unroll
+  for (int i = 0; i < NPL; ++i) {
+    const bool in = v[i] >= bound;
+    const uint32_t m = __ballot_sync(0xffffffffu, in);
+    if (m != 0u) {
+      const int pos = n + __popc(m & ((1u << lane) - 1u));
+      if (in && pos < kSelCand) {
+        cv[pos] = v[i];
+        ci[pos] = i * 32 + lane;
+      }
+      n += __popc(m);
+    }
+  }
+  int32_t* dst = blocks + r * k_eff;
+  __syncwarp();
+  if (n > kSelCand) {
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) cv[i * 32 + lane] = v[i];
+    __syncwarp();
+    nsa_argmax_loop(cv, NPL * 32, k_eff, lane, dst);
+    return;
+  }
+  float a[2];
+  int before[2] = {0, 0};
+#pragma unroll
+  for (int c = 0; c < 2; ++c) a[c] = c * 32 + lane < n ? cv[c * 32 + lane] : -3.f;
+  for (int j = 0; j < n; ++j) {
+    const float o = cv[j];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) before[c] += (o > a[c] || (o == a[c] && j < c * 32 + lane)) ? 1 : 0;
+  }
+  int cnt = 0;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const bool sel = c * 32 + lane < n && before[c] < k_eff;
+    const uint32_t m = __ballot_sync(0xffffffffu, sel);
+    if (sel) dst[cnt + __popc(m & ((1u << lane) - 1u))] = ci[c * 32 + lane];
+    cnt += __popc(m);
+  }
+}
+
+// Any size: the row in shared memory, iterative arg-max.
+__global__ void __launch_bounds__(128) nsa_select_kernel(const float* __restrict__ imp, int n_pad, int n_s, int k_eff,
+                                                         int64_t rows, int32_t* __restrict__ blocks) {
+  extern __shared__ float sel_sm[];
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t r = static_cast<int64_t>(blockIdx.x) * 4 + wib;
+  if (r >= rows) return;
+  const int n = (n_s + 31) & ~31;                     // scanned range, a multiple of 32
+  float* v = sel_sm + wib * n;
+  const float* src = imp + r * n_pad;
+  for (int i = lane; i < n; i += 32) v[i] = i < n_s ? (i < n_pad ? src[i] : 0.f) : -2.f;
+  __syncwarp();
+  nsa_argmax_loop(v, n, k_eff, lane, blocks + r * k_eff);
 }
 
 // ------------------------------------------------------- selected attention
@@ -432,12 +516,20 @@ __global__ void __launch_bounds__(128) nsa_selected_attn_kernel(const NsaSelPara
 
 // ---------------------------------------- selected attention on mma.sync tiles
 // The same operator with the two products on warp-level tensor-core tiles (m16n8k16, bf16 in, fp32
-// accumulate): the G <= 8 heads of the kv group are the rows of a 16-row tile (the other rows are
-// zero), so one tile multiplies all heads of a query with 8 keys (scores) or 8 channels (output).
-// tcgen05 tiles are 128 rows tall and would be 6 % used here; the limit of this kernel is the
-// gather of the selected key / value rows from L2 anyway.  One warp per (b, g, t); keys in chunks
-// of 16, copied with cp.async into a per-warp double buffer (rows padded to D*2 + 16 bytes so that
-// ldmatrix reads are free of bank conflicts).
+// accumulate).  Both products are computed transposed, so that the G <= 8 heads of the kv group are
+// the N = 8 columns of a tile and no row of it is padding:
+//   S^T (keys x heads)     = K (16 keys x 16 channels)   * Q^T
+//   O^T (channels x heads) = V^T (16 channels x 16 keys) * P^T
+// (tcgen05 tiles are 128 rows tall and would be 6 % used here.)  One warp per (b, g, t), warps
+// persistent; every warp streams its selected blocks 32 keys at a time through its own two-stage
+// rings (16-byte cp.async pieces, 16-byte chunks swizzled by row so that ldmatrix reads are free of
+// bank conflicts), one stream across query boundaries.  A K stage is refilled as soon as the scores are
+// taken, a V stage after the second product, so most of the 224 KiB of shared memory is loads in
+// flight: the bound is the L2 -> SM path (every selected row crosses it once per group, 8 FLOP per byte;
+// 17.5 TB/s measured for such blocks) with the shared-memory port close behind (each byte is written
+// and read once).  65536 tokens, 2 kv heads, 16 blocks of 64, D = 128: 7.1 -> 4.6 ms, 15 TB/s (the loads
+// alone take 4.0 ms).  The same rings filled by TMA boxes of 32 keys x 64 channels ran at 9.4 TB/s with
+// the products left out: one 4 KiB box per 125 cycles and SM.
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -452,155 +544,253 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t add
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
-// d += a (16x16, row) * b (16x8, col); the tile's rows 8..15 are zero: a1 = a3 = 0
-__device__ __forceinline__ void mma_16816_top(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+// d += a (16x16, row) * b (16x8, col)
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
                "{%0, %1, %2, %3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// transposes an 8x8 tile of 16-bit elements held as one mma fragment register
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
 }
 
 template <int D>
-__global__ void __launch_bounds__(128) nsa_selected_attn_mma_kernel(const NsaSelParams p) {
-  constexpr int kRowBytes = D * 2 + 16;              // padded key / value row
-  constexpr int kChunk = 16;                         // keys per step
-  constexpr int kBufBytes = kChunk * kRowBytes;      // one K or V chunk
-  extern __shared__ __align__(16) uint8_t sel_smem[];   // [4 warps][2 buffers][K chunk, V chunk]
+struct NsaSelCfg {
+  static constexpr int kStep = 32;                           // keys per step
+  static constexpr int kHalfBytes = kStep * 128;             // 64 channels of a step
+  static constexpr int kStageBytes = kStep * D * 2;
+  static constexpr int kWarps = D == 128 ? 7 : 12;
+  static constexpr int kWarpBytes = 4 * kStageBytes;         // two K and two V stages
+  static constexpr size_t kSmem = static_cast<size_t>(kWarps) * kWarpBytes;
+};
+
+template <int D>
+__global__ void __launch_bounds__(32 * NsaSelCfg<D>::kWarps, 1)
+    nsa_selected_attn_mma_kernel(const NsaSelParams p) {
+  using Cfg = NsaSelCfg<D>;
+  extern __shared__ __align__(128) uint8_t sel_smem[];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g4 = lane >> 2, t4 = lane & 3;           // fragment row / column-pair indices
-  const int64_t wid = static_cast<int64_t>(blockIdx.x) * 4 + wib;
-  const int64_t total = static_cast<int64_t>(p.B) * p.Hkv * p.Tq;
-  if (wid >= total) return;
-  const int t = static_cast<int>(wid % p.Tq);
-  const int g = static_cast<int>((wid / p.Tq) % p.Hkv);
-  const int b = static_cast<int>(wid / (static_cast<int64_t>(p.Tq) * p.Hkv));
+  const int g4 = lane >> 2, t4 = lane & 3;                   // fragment row / column-pair indices
+  const uint32_t sbase = smem_u32(sel_smem) + wib * Cfg::kWarpBytes;
+
   const int G = p.G;
-  const uint32_t sbase = smem_u32(sel_smem) + wib * (4 * kBufBytes);
-  const __nv_bfloat16* kbase = p.k + b * p.ks[0] + g * p.ks[1];
-  const __nv_bfloat16* vbase = p.v + b * p.vs[0] + g * p.vs[1];
-  const int32_t* blk = p.blocks + ((static_cast<int64_t>(b) * p.Hkv + g) * p.Tq + t) * p.n_sel;
+  const int64_t total = static_cast<int64_t>(p.B) * p.Hkv * p.Tq;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * Cfg::kWarps;
+  const int steps_per_block = p.sel_block / Cfg::kStep;
+  const int n_steps = p.n_sel * steps_per_block;
   const float ninf = -__int_as_float(0x7f800000);
+  const float sc = p.scale_log2;
 
-  // Q fragments: row g4 = head g4 of the group (zero for g4 >= G), 16 channels per k-step
-  uint32_t qa0[D / 16], qa2[D / 16];
-  {
-    const __nv_bfloat16* qrow = p.q + b * p.qs[0] + (g * G + min(g4, G - 1)) * p.qs[1] + t * p.qs[2];
-#pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks) {
-      const uint32_t lo = *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 2 * t4);
-      const uint32_t hi = *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 8 + 2 * t4);
-      qa0[ks] = g4 < G ? lo : 0u;
-      qa2[ks] = g4 < G ? hi : 0u;
-    }
-  }
-
-  const int chunks_per_block = p.sel_block / kChunk;
-  const int n_chunks = p.n_sel * chunks_per_block;
-  // copies chunk c (16 key rows and 16 value rows) into buffer c & 1
-  auto issue = [&](int c) {
-    const int key0 = blk[c / chunks_per_block] * p.sel_block + (c % chunks_per_block) * kChunk;
-    const uint32_t dst = sbase + (c & 1) * (2 * kBufBytes);
-    constexpr int kPieces = kChunk * (D * 2 / 16);   // 16-byte pieces per chunk
-#pragma unroll
-    for (int i = 0; i < kPieces / 32; ++i) {
-      const int piece = i * 32 + lane;
-      const int r = piece / (D * 2 / 16), cpi = piece % (D * 2 / 16);
-      const int key = min(key0 + r, p.Tk - 1);
-      cp_async16(dst + r * kRowBytes + cpi * 16, kbase + static_cast<int64_t>(key) * p.ks[2] + cpi * 8);
-      cp_async16(dst + kBufBytes + r * kRowBytes + cpi * 16, vbase + static_cast<int64_t>(key) * p.vs[2] + cpi * 8);
-    }
-    cp_async_commit();
+  // The copies' positions (K and V streams), running ahead of the products: query row, its list of
+  // blocks and its K / V base (recomputed only when the row changes), block within the list, step
+  // within the block; the next block index is loaded one step before it is used.
+  constexpr int CPR = D / 8;                                 // 16-byte chunks per row
+  constexpr int RPI = 32 / CPR;                              // rows per copy instruction
+  const int crow = lane / CPR, cchunk = lane % CPR;
+  // stage layout: [64-channel half][key][8 chunks], chunk c of row r at position c ^ (r & 7)
+  const uint32_t cdst = sbase + (cchunk >> 3) * Cfg::kHalfBytes + crow * 128;
+  struct Stream {
+    int64_t row;
+    const int32_t* list;
+    const __nv_bfloat16* base;
+    int in_list, in_block, blk;
+  } str[2];
+  auto open_row = [&](int which, int64_t r) {
+    Stream& x = str[which];
+    x.row = r;
+    x.in_list = x.in_block = 0;
+    if (r >= total) return;
+    const int bg = static_cast<int>(r / p.Tq);
+    const int g = bg % p.Hkv, b = bg / p.Hkv;
+    x.list = p.blocks + r * p.n_sel;
+    x.base = (which ? p.v + b * p.vs[0] + g * p.vs[1] : p.k + b * p.ks[0] + g * p.ks[1]) + cchunk * 8;
+    x.blk = __ldg(x.list);
   };
-
-  float o[D / 8][4];
+  auto issue = [&](int which, int stage) {                   // which: 0 = K, 1 = V
+    Stream& x = str[which];
+    if (x.row < total) {
+      const int key0 = x.blk * p.sel_block + x.in_block * Cfg::kStep;
+      const int64_t rs = which ? p.vs[2] : p.ks[2];
+      const uint32_t dst = cdst + (which * 2 + stage) * Cfg::kStageBytes;
+      if (key0 + Cfg::kStep <= p.Tk) {
+        const __nv_bfloat16* src = x.base + (key0 + crow) * rs;
 #pragma unroll
-  for (int n = 0; n < D / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-  float m = ninf, l = 0.f;
-
-  issue(0);
-  for (int c = 0; c < n_chunks; ++c) {
-    if (c + 1 < n_chunks) {
-      issue(c + 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+        for (int i = 0; i < Cfg::kStep / RPI; ++i) {
+          const int row = i * RPI + crow;
+          cp_async16(dst + i * RPI * 128 + (((cchunk & 7) ^ (row & 7)) << 4), src);
+          src += RPI * rs;
+        }
+      } else {
+#pragma unroll 1
+        for (int i = 0; i < Cfg::kStep / RPI; ++i) {
+          const int row = i * RPI + crow;
+          cp_async16(dst + i * RPI * 128 + (((cchunk & 7) ^ (row & 7)) << 4), x.base + min(key0 + row, p.Tk - 1) * rs);
+        }
+      }
+      if (++x.in_block == steps_per_block) {
+        x.in_block = 0;
+        if (++x.in_list == p.n_sel) open_row(which, x.row + stride);
+        else x.blk = __ldg(x.list + x.in_list);
+      }
     }
-    __syncwarp();
-    const uint32_t kb = sbase + (c & 1) * (2 * kBufBytes);
-    const uint32_t vb = kb + kBufBytes;
-    const int key0 = blk[c / chunks_per_block] * p.sel_block + (c % chunks_per_block) * kChunk;
+    cp_async_commit();                                       // (an empty group past the end keeps the count)
+  };
+  open_row(0, static_cast<int64_t>(blockIdx.x) * Cfg::kWarps + wib);
+  open_row(1, str[0].row);
+  issue(0, 0);
+  issue(1, 0);
+  issue(0, 1);
+  issue(1, 1);
 
-    // ---- scores: s[nt][0..1] = head g4 against keys key0 + 8*nt + 2*t4 (+1)
-    float s[2][4];
+  int it = 0;                                                // steps consumed by this warp
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * Cfg::kWarps + wib; r < total; r += stride) {
+    const int bg = static_cast<int>(r / p.Tq);
+    const int t = static_cast<int>(r - static_cast<int64_t>(bg) * p.Tq);
+    const int g = bg % p.Hkv, b = bg / p.Hkv;
+    // Q^T fragments: column g4 = head g4 of the group (zero for g4 >= G), 16 channels per k-step
+    uint32_t qb0[D / 16], qb1[D / 16];
+    {
+      const __nv_bfloat16* qrow = p.q + b * p.qs[0] + (g * G + min(g4, G - 1)) * p.qs[1] + t * p.qs[2];
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+      for (int ks = 0; ks < D / 16; ++ks) {
+        const uint32_t lo = *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 2 * t4);
+        const uint32_t hi = *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 8 + 2 * t4);
+        qb0[ks] = g4 < G ? lo : 0u;
+        qb1[ks] = g4 < G ? hi : 0u;
+      }
+    }
+    float o[D / 16][4];                                      // channels (g4, g4 + 8) x heads (2 t4, 2 t4 + 1)
 #pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks) {
-      // four 8x8 matrices: (keys 0-7 | 8-15) x (channels 16ks..+7 | +8..+15)
-      uint32_t kf[4];
+    for (int n = 0; n < D / 16; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+    float m[2] = {ninf, ninf}, l[2] = {0.f, 0.f};            // heads 2 t4, 2 t4 + 1
+    const int32_t* list = p.blocks + r * p.n_sel;
+    int key0 = __ldg(list) * p.sel_block, in_block = 0;
+    int blk_next = p.n_sel > 1 ? __ldg(++list) : 0;          // (loaded a block ahead of its use)
+    for (int step = 0; step < n_steps; ++step, ++it) {
+      const int stage = it & 1;
+      const uint32_t kb = sbase + stage * Cfg::kStageBytes;
+      const uint32_t vb = sbase + (2 + stage) * Cfg::kStageBytes;
+      cp_async_wait<3>();                                    // K of this step (three younger groups)
+      __syncwarp();
+      // ---- scores: s[mt]: keys key0 + 16 mt + (g4 | g4 + 8) x heads 2 t4, 2 t4 + 1
+      float s[2][4];
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt) s[mt][0] = s[mt][1] = s[mt][2] = s[mt][3] = 0.f;
       const int mat = lane >> 3, mr = lane & 7;
-      ldmatrix_x4(kf, kb + ((mat >> 1) * 8 + mr) * kRowBytes + ks * 32 + (mat & 1) * 16);
-      mma_16816_top(s[0], qa0[ks], qa2[ks], kf[0], kf[1]);
-      mma_16816_top(s[1], qa0[ks], qa2[ks], kf[2], kf[3]);
-    }
-    // ---- online softmax of row g4 (log2 domain); the four lanes of a row hold 4 keys each
-    float sv[4];
-    float mx = ninf;
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
+      for (int ks = 0; ks < D / 16; ++ks) {
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+          // four 8x8 matrices: (keys 0-7 | 8-15) of (channels 0-7), then of (channels 8-15)
+          uint32_t kf[4];
+          const int row = mt * 16 + (mat & 1) * 8 + mr, chunk = (ks & 3) * 2 + (mat >> 1);
+          ldmatrix_x4(kf, kb + (ks >> 2) * Cfg::kHalfBytes + row * 128 + ((chunk ^ mr) << 4));
+          mma_16816(s[mt], kf, qb0[ks], qb1[ks]);
+        }
+      }
+      __syncwarp();
+      issue(0, stage);                                       // K stage read: refill it
+      // ---- online softmax per head (log2 domain) over the 32 keys
+      if (key0 + Cfg::kStep > p.Tk) {
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (key0 + mt * 16 + (e >> 1) * 8 + g4 >= p.Tk) s[mt][e] = ninf;
+        }
+      }
+      // The stabiliser is raised only when some score exceeds it by 2^8 (always at the first step): one
+      // vote instead of a maximum over the lanes that hold a head's keys.
+      float mx[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) mx[e] = fmaxf(fmaxf(s[0][e], s[0][e + 2]), fmaxf(s[1][e], s[1][e + 2])) * sc;
+      if (__any_sync(0xffffffffu, mx[0] > m[0] + 8.f || mx[1] > m[1] + 8.f)) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 4));
+          mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 8));
+          mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 16));
+          const float m_new = fmaxf(m[e], mx[e]);
+          const float alpha = (m[e] == m_new) ? 1.f : ex2_approx(m[e] - m_new);
+          m[e] = m_new;
+          l[e] *= alpha;
+#pragma unroll
+          for (int n = 0; n < D / 16; ++n) {
+            o[n][e] *= alpha;
+            o[n][e + 2] *= alpha;
+          }
+        }
+      }
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int key = key0 + nt * 8 + 2 * t4 + e;
-        sv[nt * 2 + e] = key < p.Tk ? s[nt][e] * p.scale_log2 : ninf;
-        mx = fmaxf(mx, sv[nt * 2 + e]);
+        const float neg = m[e] == ninf ? 0.f : -m[e];        // (no key seen yet: every score is -inf)
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+          s[mt][e] = ex2_approx(fmaf(s[mt][e], sc, neg));
+          s[mt][e + 2] = ex2_approx(fmaf(s[mt][e + 2], sc, neg));
+        }
+        l[e] += (s[0][e] + s[0][e + 2]) + (s[1][e] + s[1][e + 2]);
+      }
+      uint32_t pb[2][2];                                     // P^T fragments: keys 2 t4, 2 t4 + 1 (+ 8) of head g4
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt) {
+        pb[mt][0] = movmatrix_trans(pack_bf16x2(s[mt][0], s[mt][1]));
+        pb[mt][1] = movmatrix_trans(pack_bf16x2(s[mt][2], s[mt][3]));
+      }
+      // ---- O^T += V^T P^T
+      cp_async_wait<3>();                                    // V of this step
+      __syncwarp();
+#pragma unroll
+      for (int n = 0; n < D / 16; ++n) {
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+          // four 8x8 matrices, transposed on load: (channels 0-7 | 8-15) of (keys 0-7), then of (keys 8-15)
+          uint32_t vf[4];
+          const int row = mt * 16 + (mat >> 1) * 8 + mr, chunk = (n & 3) * 2 + (mat & 1);
+          ldmatrix_x4_trans(vf, vb + (n >> 2) * Cfg::kHalfBytes + row * 128 + ((chunk ^ mr) << 4));
+          mma_16816(o[n], vf, pb[mt][0], pb[mt][1]);
+        }
+      }
+      __syncwarp();
+      issue(1, stage);
+      key0 += Cfg::kStep;
+      if (++in_block == steps_per_block) {
+        in_block = 0;
+        key0 = blk_next * p.sel_block;
+        if (step + 1 + steps_per_block < n_steps) blk_next = __ldg(++list);
       }
     }
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    const float m_new = fmaxf(m, mx);
-    const float alpha = (m == m_new) ? 1.f : ex2_approx(m - m_new);      // m_new = -inf only if m is too
-    float pr[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) pr[e] = (m_new == ninf) ? 0.f : ex2_approx(sv[e] - m_new);
-    l = l * alpha + (pr[0] + pr[1]) + (pr[2] + pr[3]);
-    m = m_new;
-    const uint32_t pa0 = pack_bf16x2(pr[0], pr[1]);   // keys 2*t4, +1 of the first eight
-    const uint32_t pa2 = pack_bf16x2(pr[2], pr[3]);   // of the second eight
-    // ---- O = O * alpha + P V
+    for (int e = 0; e < 2; ++e) {
+      l[e] += __shfl_xor_sync(0xffffffffu, l[e], 4);
+      l[e] += __shfl_xor_sync(0xffffffffu, l[e], 8);
+      l[e] += __shfl_xor_sync(0xffffffffu, l[e], 16);
+      const int hh = 2 * t4 + e;
+      if (hh < G) {
+        const float inv = l[e] > 0.f ? 1.f / l[e] : 0.f;
+        float* dst = p.o + ((static_cast<int64_t>(b) * p.Hq + g * G + hh) * p.Tq + t) * D + g4;
+        float x[D / 8];
 #pragma unroll
-    for (int n2 = 0; n2 < D / 16; ++n2) {
-      // four 8x8 matrices, transposed on load: (keys 0-7 | 8-15) x (channels 16*n2..+7 | +8..+15)
-      uint32_t vf[4];
-      const int mat = lane >> 3, mr = lane & 7;
-      ldmatrix_x4_trans(vf, vb + ((mat & 1) * 8 + mr) * kRowBytes + n2 * 32 + (mat >> 1) * 16);
+        for (int n = 0; n < D / 8; ++n) x[n] = o[n >> 1][e + (n & 1) * 2] * inv;
+        if (p.gate != nullptr) {
+          const float gl = p.gate[((static_cast<int64_t>(b) * p.Tq + t) * p.Hq + g * G + hh) * 3 + 1];
+          const float gs = 1.f / (1.f + __expf(-gl));
+          float a[D / 8];                                    // (all loads before the first store)
 #pragma unroll
-      for (int h2 = 0; h2 < 2; ++h2) {
-        float (&acc)[4] = o[n2 * 2 + h2];
-        acc[0] *= alpha;
-        acc[1] *= alpha;
-        mma_16816_top(acc, pa0, pa2, vf[h2 * 2], vf[h2 * 2 + 1]);
+          for (int n = 0; n < D / 8; ++n) a[n] = dst[n * 8];
+#pragma unroll
+          for (int n = 0; n < D / 8; ++n) x[n] = fmaf(gs, x[n], a[n]);
+        }
+#pragma unroll
+        for (int n = 0; n < D / 8; ++n) dst[n * 8] = x[n];
       }
     }
-    __syncwarp();   // the buffer is refilled two chunks later
   }
-  l += __shfl_xor_sync(0xffffffffu, l, 1);
-  l += __shfl_xor_sync(0xffffffffu, l, 2);
-  if (g4 < G) {
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-    float* dst = p.o + ((static_cast<int64_t>(b) * p.Hq + g * G + g4) * p.Tq + t) * D + 2 * t4;
-    if (p.gate != nullptr) {
-      const float gl = p.gate[((static_cast<int64_t>(b) * p.Tq + t) * p.Hq + g * G + g4) * 3 + 1];
-      const float gs = 1.f / (1.f + __expf(-gl));
-#pragma unroll
-      for (int n = 0; n < D / 8; ++n) {
-        const float2 a = *reinterpret_cast<const float2*>(dst + n * 8);
-        *reinterpret_cast<float2*>(dst + n * 8) = make_float2(fmaf(gs, o[n][0] * inv, a.x), fmaf(gs, o[n][1] * inv, a.y));
-      }
-    } else {
-#pragma unroll
-      for (int n = 0; n < D / 8; ++n) *reinterpret_cast<float2*>(dst + n * 8) = make_float2(o[n][0] * inv, o[n][1] * inv);
-    }
-  }
+  cp_async_wait<0>();
 }
 
 // ------------------------------------------------------------------ combine
@@ -625,6 +815,18 @@ __global__ void nsa_combine_kernel(const float* __restrict__ o_cmp, const float*
 
 // --------------------------------------------------------------------- host
 static bool nsa_aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+template <int D>
+static int launch_selected(const NsaSelParams& p, cudaStream_t st) {
+  using Cfg = NsaSelCfg<D>;
+  SWV_CUDA_OK(cudaFuncSetAttribute(nsa_selected_attn_mma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(Cfg::kSmem)));
+  const int64_t total = static_cast<int64_t>(p.B) * p.Hkv * p.Tq, need = (total + Cfg::kWarps - 1) / Cfg::kWarps;
+  const unsigned grid = static_cast<unsigned>(need < sm_count() ? need : sm_count());
+  nsa_selected_attn_mma_kernel<D><<<grid, 32 * Cfg::kWarps, Cfg::kSmem, st>>>(p);
+  SWV_CUDA_OK(cudaGetLastError());
+  return SWV_OK;
+}
 
 template <int D, int R>
 static int launch_importance(const CUtensorMap& tq, const CUtensorMap& tk, const NsaImpParams& p, cudaStream_t st) {
@@ -696,13 +898,19 @@ int nsa_select_blocks_impl(const void* q, const int64_t* qs, const void* kc, con
 
   const int64_t rows = static_cast<int64_t>(B) * Hkv * Tq;
   const int n = (n_s + 31) & ~31;
+  const unsigned sel_grid = static_cast<unsigned>((rows + 3) / 4);
+  if (k_eff <= 32 && n_s <= 1024) {
+    if (n_s <= 256) nsa_select_short_kernel<8><<<sel_grid, 128, 0, st>>>(importance, p.n_pad, n_s, k_eff, rows, blocks);
+    else nsa_select_short_kernel<32><<<sel_grid, 128, 0, st>>>(importance, p.n_pad, n_s, k_eff, rows, blocks);
+    SWV_CUDA_OK(cudaGetLastError());
+    return SWV_OK;
+  }
   const size_t sm = static_cast<size_t>(4) * n * 4;
   if (sm > 200 * 1024) return SWV_ERR_UNSUPPORTED;
   if (sm > 48 * 1024)
     SWV_CUDA_OK(cudaFuncSetAttribute(nsa_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(sm)));
-  nsa_select_kernel<<<static_cast<unsigned>((rows + 3) / 4), 128, sm, st>>>(importance, p.n_pad, n_s, k_eff, rows,
-                                                                            blocks);
+  nsa_select_kernel<<<sel_grid, 128, sm, st>>>(importance, p.n_pad, n_s, k_eff, rows, blocks);
   SWV_CUDA_OK(cudaGetLastError());
   return SWV_OK;
 }
@@ -729,21 +937,10 @@ int nsa_selected_attn_impl(const void* q, const int64_t* qs, const void* k, cons
   const int64_t total = static_cast<int64_t>(B) * Hkv * Tq;
   const unsigned grid = static_cast<unsigned>((total + 3) / 4);
   // tensor-core tiles when the layout allows 16-byte row copies (the usual case), else CUDA cores
-  const bool mma_ok = sel_block % 16 == 0 && nsa_aligned16(q) && (qs[0] * 2) % 4 == 0 && (qs[1] * 2) % 4 == 0 &&
+  const bool mma_ok = nsa_aligned16(q) && (qs[0] * 2) % 4 == 0 && (qs[1] * 2) % 4 == 0 &&
                       (qs[2] * 2) % 4 == 0;
-  if (mma_ok) {
-    if (D == 64) {
-      const size_t sm = 4 * 4 * 16 * (64 * 2 + 16);
-      SWV_CUDA_OK(cudaFuncSetAttribute(nsa_selected_attn_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(sm)));
-      nsa_selected_attn_mma_kernel<64><<<grid, 128, sm, st>>>(p);
-    } else {
-      const size_t sm = 4 * 4 * 16 * (128 * 2 + 16);
-      SWV_CUDA_OK(cudaFuncSetAttribute(nsa_selected_attn_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(sm)));
-      nsa_selected_attn_mma_kernel<128><<<grid, 128, sm, st>>>(p);
-    }
-  } else if (D == 64) {
+  if (mma_ok) return D == 64 ? launch_selected<64>(p, st) : launch_selected<128>(p, st);
+  if (D == 64) {
     nsa_selected_attn_kernel<64, 8><<<grid, 128, 0, st>>>(p);
   } else {
     nsa_selected_attn_kernel<128, 8><<<grid, 128, 0, st>>>(p);

@@ -90,3 +90,24 @@ def test_nsa_single_call_equals_stepwise():
     # same kernels and the same order of additions; the fused epilogues contract g * o + acc into one
     # FMA where the stand-alone gate kernel may round the product first
     assert (one - parts[0]).abs().max() < 1e-5
+
+
+@pytest.mark.parametrize("T", [300, 6000, 17000, 66000])
+def test_selection_on_plateaus_takes_the_lowest_blocks(T):
+    """Zero queries: every compressed token is equally important, so all full blocks tie and the lowest
+    indices must be taken.  More ties than the short selection's candidate buffer holds (its arg-max
+    fallback), the two register sizes of the short form, and more blocks than it takes."""
+    import sparse_wsi_vit_b200 as swv
+    from sparse_wsi_vit_b200.nsa import nsa_attention
+    g = torch.Generator().manual_seed(T)
+    q = torch.zeros(1, 2, T, 64, dtype=torch.bfloat16, device=DEV)
+    k, v = (torch.randn(1, 1, T, 64, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
+    gate = torch.zeros(1, T, 2, 3, device=DEV)
+    _, _, o_sel, _, blocks = nsa_attention(q, k, v, gate, window=128, return_parts=True)
+    swv.check_status(DEV)
+    n = min(16, -(-T // 64))
+    assert bool((blocks[0, 0] == torch.arange(n, device=DEV)).all())
+    # equal scores: the selected branch is the mean of the selected values; P is 1 before normalisation,
+    # so only the bf16 rounding of the inputs and the fp32 sums are left
+    mean = v[0, 0, :min(T, n * 64)].float().mean(0)
+    assert (o_sel[0] - mean).abs().max() < 1e-4
