@@ -20,6 +20,7 @@ EXPORTS = [
     "swv_nsa_workspace_bytes", "swv_nsa_attn_fwd", "swv_dsa_attn_scratch_bytes", "swv_dsa_attn_masked_count_fwd",
     "swv_dsa_attn_bwd", "swv_dsa_indexer_bwd", "swv_dsa_prologue_fwd", "swv_dsa_attn_lists_fwd",
     "swv_dsa_attn_lists_scratch_bytes", "swv_dsa_workspace_bytes_topk", "swv_block_sparse_workspace_bytes", "swv_block_sparse_attn_ws_fwd",
+    "swv_dsa_module_bwd_bytes", "swv_dsa_module_bwd",
 ]
 
 
@@ -79,6 +80,10 @@ def _load():
     lib.swv_dsa_indexer_bwd.argtypes = [
         c_void_p, i64p, c_void_p, i64p, c_void_p, i64p, c_int, c_void_p, c_void_p, i64p, c_void_p, i64p, c_void_p,
         c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
+    lib.swv_dsa_module_bwd_bytes.argtypes = [c_int, c_int, c_int, c_int, POINTER(c_size_t)]
+    lib.swv_dsa_module_bwd.argtypes = (
+        [c_void_p, i64p] * 5 + [c_int] + [c_void_p, i64p] * 2 + [c_int] + [c_void_p] * 12 + [c_int] * 8 +
+        [c_void_p, c_size_t, c_void_p, c_void_p])
     lib.swv_dsa_prologue_fwd.argtypes = [
         c_void_p, i64p, c_void_p, i64p, c_int, c_void_p, i64p, c_void_p, i64p, c_int, c_void_p, c_void_p, c_float,
         c_float, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]

@@ -56,7 +56,16 @@ int dsa_attn_bwd_impl(const void* d_out, const int64_t* dos, const void* q, cons
                       const int64_t* ks, const void* v, const int64_t* vs, int dtype, const void* o,
                       const int64_t* os, int o_dtype, const int32_t* idx, const int64_t* is, const float* valid,
                       const int64_t* vls, const float* rw, const int64_t* rs, float* dq, float* dk, float* dv,
-                      float* drw, int B, int H, int Tq, int Tk, int D, int top_k, int* status, cudaStream_t st);
+                      float* drw, int B, int H, int Tq, int Tk, int D, int top_k, int* status, cudaStream_t st,
+                      const int* run_if);
+int dsa_module_bwd_bytes_impl(int B, int H, int Tq, int Tk, size_t* bytes);
+int dsa_module_bwd_impl(const void* d_out, const int64_t* dos, const void* q, const int64_t* qs, const void* k,
+                        const int64_t* ks, const void* v, const int64_t* vs, const void* o, const int64_t* os,
+                        int o_dtype, const void* q_idx, const int64_t* qis, const void* k_idx, const int64_t* kis,
+                        int idx_dtype, const float* w, const int32_t* idx, const float* valid, const float* scores,
+                        const uint32_t* maskbits, float* dq, float* dk, float* dv, float* drw, float* dq_idx,
+                        float* dk_idx, float* dw, int B, int H, int Tq, int Tk, int D, int IH, int ID, int top_k,
+                        void* workspace, size_t workspace_bytes, int* status, cudaStream_t st);
 int dsa_indexer_bwd_impl(const float* d_scores, const int64_t* dss, const void* q_idx, const int64_t* qs,
                          const void* k_idx, const int64_t* ks, int dtype, const float* w, const int32_t* idx,
                          const int64_t* is, const float* valid, const int64_t* vls, float* dq, float* dk, float* dw,
@@ -150,7 +159,25 @@ int swv_dsa_attn_bwd(const void* d_out, const int64_t d_out_strides[4], const vo
                      int Tk, int D, int top_k, int* status, void* stream) {
   return swv::dsa_attn_bwd_impl(d_out, d_out_strides, q, q_strides, k, k_strides, v, v_strides, qkv_dtype, o, o_strides,
                                 o_dtype, idx, idx_strides, valid, valid_strides, rw, rw_strides, dq, dk, dv, drw, B, H,
-                                Tq, Tk, D, top_k, status, static_cast<cudaStream_t>(stream));
+                                Tq, Tk, D, top_k, status, static_cast<cudaStream_t>(stream), nullptr);
+}
+
+int swv_dsa_module_bwd_bytes(int B, int H, int Tq, int Tk, size_t* bytes) {
+  return swv::dsa_module_bwd_bytes_impl(B, H, Tq, Tk, bytes);
+}
+
+int swv_dsa_module_bwd(const void* d_out, const int64_t d_out_strides[4], const void* q, const int64_t q_strides[4],
+                       const void* k, const int64_t k_strides[4], const void* v, const int64_t v_strides[4],
+                       const void* o, const int64_t o_strides[4], int o_dtype, const void* q_idx,
+                       const int64_t q_idx_strides[4], const void* k_idx, const int64_t k_idx_strides[4], int idx_dtype,
+                       const float* w, const int32_t* idx, const float* valid, const float* scores,
+                       const uint32_t* maskbits, float* dq, float* dk, float* dv, float* drw, float* dq_idx,
+                       float* dk_idx, float* dw, int B, int H, int Tq, int Tk, int D, int IH, int ID, int top_k,
+                       void* workspace, size_t workspace_bytes, int* status, void* stream) {
+  return swv::dsa_module_bwd_impl(d_out, d_out_strides, q, q_strides, k, k_strides, v, v_strides, o, o_strides, o_dtype,
+                                  q_idx, q_idx_strides, k_idx, k_idx_strides, idx_dtype, w, idx, valid, scores, maskbits,
+                                  dq, dk, dv, drw, dq_idx, dk_idx, dw, B, H, Tq, Tk, D, IH, ID, top_k, workspace,
+                                  workspace_bytes, status, static_cast<cudaStream_t>(stream));
 }
 
 int swv_dsa_indexer_bwd(const float* d_scores, const int64_t d_scores_strides[3], const void* q_idx,

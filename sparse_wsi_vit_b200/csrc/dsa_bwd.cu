@@ -83,6 +83,7 @@ struct AttnBwdParams {
   float *dq, *dk, *dv, *drw;      // fp32 contiguous: (B,H,Tq,D), (B,H,Tk,D), (B,H,Tk,D), (B,Tq,K)
   int B, H, Tq, Tk, D, top_k;
   float scale;
+  const int* run_if;              // when given and zero: the tile kernels have the work, return at once
   int* status;
 };
 
@@ -94,6 +95,7 @@ constexpr int kBwdWarps = 4;
 template <typename T, typename TO, int DPL, bool CACHE>
 __global__ void __launch_bounds__(32 * kBwdWarps) dsa_attn_bwd_kernel(const AttnBwdParams p) {
   constexpr int DMAX = 32 * DPL;
+  if (p.run_if != nullptr && *p.run_if == 0) return;
   extern __shared__ float bw_smem[];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* qsm = bw_smem + wib * (2 * DMAX + (CACHE ? p.top_k : 0));
@@ -275,7 +277,8 @@ int dsa_attn_bwd_impl(const void* d_out, const int64_t* dos, const void* q, cons
                       const int64_t* ks, const void* v, const int64_t* vs, int dtype, const void* o,
                       const int64_t* os, int o_dtype, const int32_t* idx, const int64_t* is, const float* valid,
                       const int64_t* vls, const float* rw, const int64_t* rs, float* dq, float* dk, float* dv,
-                      float* drw, int B, int H, int Tq, int Tk, int D, int top_k, int* status, cudaStream_t st) {
+                      float* drw, int B, int H, int Tq, int Tk, int D, int top_k, int* status, cudaStream_t st,
+                      const int* run_if) {
   if (!d_out || !q || !k || !v || !o || !idx || !valid || !rw || !dq || !dk || !dv || !drw || !status || !dos || !qs ||
       !ks || !vs || !os || !is || !vls || !rs)
     return SWV_ERR_NULL;
@@ -292,6 +295,7 @@ int dsa_attn_bwd_impl(const void* d_out, const int64_t* dos, const void* q, cons
   p.dq = dq; p.dk = dk; p.dv = dv; p.drw = drw;
   p.B = B; p.H = H; p.Tq = Tq; p.Tk = Tk; p.D = D; p.top_k = top_k;
   p.scale = 1.0f / sqrtf(static_cast<float>(D));
+  p.run_if = run_if;
   p.status = status;
   const size_t kv_bytes = static_cast<size_t>(B) * H * Tk * D * sizeof(float);
   SWV_CUDA_OK(cudaMemsetAsync(dk, 0, kv_bytes, st));

@@ -1,0 +1,950 @@
+// Backward of a DSA layer on the tensor cores, for selections this library's own indexer made
+// (ascending key lists with their membership bitmask): gradients of the routing-weighted attention
+// (src/sparse_wsi_vit/models/deepseek_sparse_attention_kernels/kernels.py:569-762) and of the indexer
+// (:128-339), the same formulas as the list kernels in dsa_bwd.cu, which serve every other case.
+//
+//   sm_ij = exp(logit_ij - m_i) / max(l_i, 1e-6)     P_ij = sm_ij w_ij          (member pairs only)
+//   g_ij  = sm_ij (dO_i . v_j - D_i)                 dS_ij = w_ij g_ij
+//   dV_j = sum_i P_ij dO_i    dK_j = scale sum_i dS_ij q_i    dQ_i = scale sum_j dS_ij k_j
+//   drw_ij = sum_heads g_ij   dq_idx = W sum_j drw_ij k_idx_j   dk_idx = W sum_i drw_ij q_idx_i
+//
+// Three sweeps over 128 x 64 tiles of (lane side) x (streamed side), one kernel:
+//   kStats : lanes = queries, keys streamed: exact row maximum and l in fp32 -> lse_i = m_i + log2 max(l_i, 1e-6)
+//   kDkv   : lanes = keys, queries streamed: dV, dK in TMEM accumulators; drw by reductions into the lists
+//   kDq    : lanes = queries, keys streamed: dQ in a TMEM accumulator
+// Every tile's logits S, routing weights R (TF32, from the collapsed indexer vectors: the forward's own
+// products) and dP = dO V^T come from tcgen05 products into one of two TMEM buffers; eight warps turn
+// them into P and dS, which go back into the very columns they came from, as the A operand (TMEM) of the
+// gradient products.  P and dS are fp32 values: each is split into THREE bf16 terms (24 bits) that are
+// multiplied one after the other, so no product sees fewer bits than the CUDA-core form.  q, k, v are
+// bf16; dO must be exact in bf16 as well (it is whenever the next layer ran in bf16) -- where it is not,
+// these kernels return at once and the list kernel runs.
+//
+// Bound: the tensor pipe.  An M128 x N64 x K16 instruction takes ~60 cycles, so a 128 x 128 tile of one
+// head costs 128 (kDkv), 80 (kDq) and 24 (kStats) of them; exponentials and splits run beside them.
+// The list kernels move 3 rows and reduce 2 per selected pair (43.8 ms at 16384 tokens, 8 heads,
+// top-2048); at one key in 8 the tiles do 8 times the kept products and are still far ahead.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <type_traits>
+
+#include "common.cuh"
+
+namespace swv {
+namespace {
+
+enum { kStats = 0, kDkv = 1, kDq = 2 };
+constexpr int kNW = 64;                 // streamed rows per tile
+constexpr int kBwdStages = 4;
+constexpr int kHd = 64;                 // head dimension
+constexpr int kLBytes = kTile * kHd * 2;            // 16 KiB: lane-side bf16 tile
+constexpr int kLRBytes = kTile * kIdxDim * 4;       // 32 KiB: lane-side collapsed indexer vectors
+constexpr int kSBytes = kNW * kHd * 2;              // 8 KiB
+constexpr int kSRBytes = kNW * kIdxDim * 4;         // 16 KiB
+constexpr int kOffL2 = kLBytes;
+constexpr int kOffLR = 2 * kLBytes;
+constexpr int kOffStage = 2 * kLBytes + kLRBytes;
+constexpr int kStageB = 2 * kSBytes + kSRBytes;
+constexpr int kOffCols = kOffStage + kBwdStages * kStageB;
+
+// per streamed query (kDkv), double-buffered: stabiliser, D, membership words and list positions
+struct BwdCols {
+  float lse[kNW], di[kNW];
+  uint32_t word[4][kNW], base[4][kNW];
+};
+struct BwdCtl {
+  uint64_t l_full, full[kBwdStages], empty[kBwdStages];
+  uint64_t in_full[2], p_ready[2], acc_done, acc_final;   // acc_done: per tile (issuer); acc_final: once
+  uint32_t tmem_base, abort_flag;
+  float xm[kTile][2], xl[kTile][2], xe[kTile][2];
+};
+constexpr int kOffBwdCtl = kOffCols + 2 * static_cast<int>(sizeof(BwdCols));
+constexpr size_t kBwdSmem = 1024 + kOffBwdCtl + sizeof(BwdCtl) + 64;
+constexpr uint32_t kBufCols = 192;      // S 64 | R 64 | dP 64
+constexpr uint32_t kColAcc = 384;       // dV (or dQ) 64 | dK 64
+
+struct BwdTileParams {
+  int B, H, Tq, Tk, nQT, nKT, top_k;
+  const uint32_t* maskbits;
+  const uint16_t* off;      // [B][nKT + 1][Tq] first list slot of row i with a key in tile kt or later
+  const float* di;          // (B,H,Tq)
+  float* lse;               // (B,H,Tq): log2 domain
+  float *dq, *dk, *dv, *drw;
+  float scale, c2;          // 1/sqrt(D), and times log2 e
+  const int* skip_if;       // non-zero: nothing to do here
+  int* status;
+};
+
+// a pair of fp32 values as three bf16 pairs whose sum is the pair
+__device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack_bf16x2(a, b);
+  a -= __uint_as_float(hi << 16);
+  b -= __uint_as_float(hi & 0xffff0000u);
+  mid = pack_bf16x2(a, b);
+  a -= __uint_as_float(mid << 16);
+  b -= __uint_as_float(mid & 0xffff0000u);
+  lo = pack_bf16x2(a, b);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(320, 1)
+    dsa_bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_l1, const __grid_constant__ CUtensorMap tm_l2,
+                         const __grid_constant__ CUtensorMap tm_lr, const __grid_constant__ CUtensorMap tm_s1,
+                         const __grid_constant__ CUtensorMap tm_s2, const __grid_constant__ CUtensorMap tm_sr,
+                         const BwdTileParams p) {
+  constexpr uint32_t kIdescQK = make_idesc(/*bf16*/ 1, kTile, kNW, 0, 0);
+  constexpr uint32_t kIdescR = make_idesc(/*tf32*/ 2, kTile, kNW, 0, 0);
+  constexpr uint32_t kIdescAcc = make_idesc(/*bf16*/ 1, kTile, kHd, 0, /*B is MN-major*/ 1);
+  if (p.skip_if != nullptr && *p.skip_if != 0) return;
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  BwdCols* cols = reinterpret_cast<BwdCols*>(smem + kOffCols);
+  BwdCtl* ctl = reinterpret_cast<BwdCtl*>(smem + kOffBwdCtl);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nLT = MODE == kDkv ? p.nKT : p.nQT;
+  const int lt = blockIdx.x % nLT;                       // lane-side tile
+  const int h = (blockIdx.x / nLT) % p.H;
+  const int b = blockIdx.x / (nLT * p.H);
+  const int nS = ((MODE == kDkv ? p.Tq : p.Tk) + kNW - 1) / kNW;   // streamed tiles
+
+  if (threadIdx.x == 0) {
+    mbar_init(&ctl->l_full, 1);
+    for (int s = 0; s < kBwdStages; ++s) {
+      mbar_init(&ctl->full[s], 1);
+      mbar_init(&ctl->empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&ctl->in_full[s], 1);
+      mbar_init(&ctl->p_ready[s], 8);
+    }
+    mbar_init(&ctl->acc_done, 1);
+    mbar_init(&ctl->acc_final, 1);
+    ctl->abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&ctl->tmem_base, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = ctl->tmem_base;
+  volatile uint32_t* abort_flag = &ctl->abort_flag;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      mbar_expect_tx(&ctl->l_full, kLBytes * (MODE == kStats ? 1 : 2) + kLRBytes);
+      tma_load_4d(smem, &tm_l1, &ctl->l_full, 0, lt * kTile, h, b);
+      if (MODE != kStats) tma_load_4d(smem + kOffL2, &tm_l2, &ctl->l_full, 0, lt * kTile, h, b);
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        tma_load_3d(smem + kOffLR + c * (kLRBytes / 2), &tm_lr, &ctl->l_full, c * 32, lt * kTile, b);
+      for (int t = 0; t < nS; ++t) {
+        const int s = t % kBwdStages;
+        if (!mbar_wait_bounded(&ctl->empty[s], ((t / kBwdStages) & 1) ^ 1, abort_flag)) {
+          record_status(p.status, kDevWaitStageEmpty);
+          break;
+        }
+        uint8_t* st = smem + kOffStage + s * kStageB;
+        mbar_expect_tx(&ctl->full[s], kSBytes * (MODE == kStats ? 1 : 2) + kSRBytes);
+        tma_load_4d(st, &tm_s1, &ctl->full[s], 0, t * kNW, h, b);
+        if (MODE != kStats) tma_load_4d(st + kSBytes, &tm_s2, &ctl->full[s], 0, t * kNW, h, b);
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+          tma_load_3d(st + 2 * kSBytes + c * (kSRBytes / 2), &tm_sr, &ctl->full[s], c * 32, t * kNW, b);
+      }
+    }
+  } else if (warp == 1) {
+    // -------------------------------------------------------------- MMA issuer
+    if (lane == 0) {
+      const uint32_t l1 = smem_u32(smem), l2 = l1 + kOffL2, lr = l1 + kOffLR, st0 = l1 + kOffStage;
+      bool ok = mbar_wait_bounded(&ctl->l_full, 0, abort_flag);
+      if (!ok) record_status(p.status, kDevWaitQ);
+      // the gradient products of tile t
+      auto accumulate = [&](int t) -> bool {
+        if (!mbar_wait_bounded(&ctl->p_ready[t & 1], (t >> 1) & 1, abort_flag)) {
+          record_status(p.status, kDevWaitPReady);
+          return false;
+        }
+        tc_fence_after();
+        const uint32_t buf = tmem_base + (t & 1) * kBufCols;
+        const uint32_t st = st0 + (t % kBwdStages) * kStageB;
+        const uint64_t d1 = smem_desc_sw128(st), d2 = smem_desc_sw128(st + kSBytes);
+#pragma unroll
+        for (int ks = 0; ks < kNW / 16; ++ks) {
+          // where the eight warps left the terms of these 16 streamed rows (see the epilogue)
+          const uint32_t cs = buf + 16 * ks, cr = cs + 64, cp = cs + 128;
+          const bool acc = t > 0 || ks > 0;
+          if (MODE == kDkv) {
+            umma_f16_ts(tmem_base + kColAcc, cs, d2 + ks * 128, kIdescAcc, acc);
+            umma_f16_ts(tmem_base + kColAcc, cs + 8, d2 + ks * 128, kIdescAcc, 1);
+            umma_f16_ts(tmem_base + kColAcc, cr, d2 + ks * 128, kIdescAcc, 1);
+          }
+          const uint32_t a2 = tmem_base + kColAcc + (MODE == kDkv ? 64 : 0);
+          umma_f16_ts(a2, cr + 8, d1 + ks * 128, kIdescAcc, acc);
+          umma_f16_ts(a2, cp, d1 + ks * 128, kIdescAcc, 1);
+          umma_f16_ts(a2, cp + 8, d1 + ks * 128, kIdescAcc, 1);
+        }
+        umma_commit(&ctl->empty[t % kBwdStages]);
+        umma_commit(&ctl->acc_done);
+        return true;
+      };
+      for (int t = 0; ok && t < nS; ++t) {
+        const int s = t % kBwdStages;
+        if (!mbar_wait_bounded(&ctl->full[s], (t / kBwdStages) & 1, abort_flag)) {
+          record_status(p.status, kDevWaitTmaFull);
+          ok = false;
+          break;
+        }
+        // the buffer's columns are free: tile t - 2 has been multiplied (kStats: read)
+        if (t >= 2 && !(MODE == kStats ? mbar_wait_bounded(&ctl->p_ready[t & 1], ((t >> 1) & 1) ^ 1, abort_flag)
+                                       : mbar_wait_bounded(&ctl->acc_done, t & 1, abort_flag))) {
+          record_status(p.status, kDevWaitAccEmpty);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t st = st0 + s * kStageB;
+        const uint32_t buf = tmem_base + (t & 1) * kBufCols;
+#pragma unroll
+        for (int ks = 0; ks < kHd / 16; ++ks)
+          umma_f16_ss(buf, smem_desc_sw128(l1) + ks * 2, smem_desc_sw128(st) + ks * 2, kIdescQK, ks > 0);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)
+          umma_tf32_ss(buf + 64, smem_desc_sw128(lr + (ks >> 2) * (kLRBytes / 2) + (ks & 3) * 32),
+                       smem_desc_sw128(st + 2 * kSBytes + (ks >> 2) * (kSRBytes / 2) + (ks & 3) * 32), kIdescR, ks > 0);
+        if (MODE != kStats) {
+#pragma unroll
+          for (int ks = 0; ks < kHd / 16; ++ks)
+            umma_f16_ss(buf + 128, smem_desc_sw128(l2) + ks * 2, smem_desc_sw128(st + kSBytes) + ks * 2, kIdescQK, ks > 0);
+        } else {
+          umma_commit(&ctl->empty[s]);
+        }
+        umma_commit(&ctl->in_full[t & 1]);
+        if (MODE != kStats && t >= 1) ok = accumulate(t - 1);
+      }
+      if (MODE != kStats && ok && accumulate(nS - 1)) umma_commit(&ctl->acc_final);
+    }
+  } else {
+    // ------------------------------------------------- eight warps: (lane quarter, half of the columns)
+    const int ct = threadIdx.x - 64;
+    const int quarter = warp & 3;
+    const int half = (warp - 2) >> 2;
+    const int row = quarter * 32 + lane;
+    const int lrow = lt * kTile + row;                    // query (kStats, kDq) or key (kDkv)
+    const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
+    const float ninf = -__int_as_float(0x7f800000);
+    const float c2 = p.c2;
+    const int64_t bh = static_cast<int64_t>(b) * p.H + h;
+    const bool row_ok = lrow < (MODE == kDkv ? p.Tk : p.Tq);
+    bool ok = true;
+
+    if constexpr (MODE == kDkv) {
+      // the column data of tile t: this thread's (quarter cq, query cc)
+      const int cq = ct >> 6, cc = ct & 63;
+      uint4 mw;
+      uint32_t off0 = 0;
+      float x0 = 0.f;
+      auto fetch = [&](int t) {
+        const int i = t * kNW + cc;
+        mw = make_uint4(0u, 0u, 0u, 0u);
+        off0 = 0;
+        x0 = cq == 0 ? -ninf : 0.f;                       // rows behind the end: sm = 2^-inf = 0
+        if (t < nS && i < p.Tq) {
+          mw = __ldg(reinterpret_cast<const uint4*>(p.maskbits) +
+                     ((static_cast<int64_t>(b) * p.nQT + (i >> 7)) * p.nKT + lt) * kTile + (i & 127));
+          off0 = __ldg(p.off + (static_cast<int64_t>(b) * (p.nKT + 1) + lt) * p.Tq + i);
+          if (cq < 2) x0 = __ldg((cq == 0 ? p.lse : p.di) + bh * p.Tq + i);
+        }
+      };
+      auto put = [&](int t) {
+        BwdCols& c = cols[t & 1];
+        const uint32_t w[4] = {mw.x, mw.y, mw.z, mw.w};
+        uint32_t mine = w[0], below = 0;
+#pragma unroll
+        for (int q = 1; q < 4; ++q) {
+          if (q <= cq) below += __popc(w[q - 1]);
+          if (q == cq) mine = w[q];
+        }
+        c.word[cq][cc] = mine;
+        c.base[cq][cc] = (static_cast<uint32_t>(b) * p.Tq + t * kNW + cc) * p.top_k + off0 + below;
+        if (cq == 0) c.lse[cc] = x0;
+        if (cq == 1) c.di[cc] = x0;
+      };
+      fetch(0);
+      put(0);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      const uint32_t lt_mask = (1u << lane) - 1u;
+      for (int t = 0; t < nS; ++t) {
+        const BwdCols& c = cols[t & 1];
+        fetch(t + 1);
+        if (ok && !mbar_wait_bounded(&ctl->in_full[t & 1], (t >> 1) & 1, abort_flag)) {
+          record_status(p.status, kDevWaitAccFull);
+          ok = false;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+          tc_fence_after();
+          const uint32_t buf = tmem_base + lane_off + (t & 1) * kBufCols;
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int c0 = half * 32 + k * 16;            // streamed rows c0 .. c0 + 15 = one k-step of the products
+            uint32_t s[16], r[16], d[16];
+            tmem_ld16(buf + c0, s);
+            tmem_ld16(buf + 64 + c0, r);
+            tmem_ld16(buf + 128 + c0, d);
+            tc_wait_ld();
+            uint32_t pt[3][8], dt[3][8];
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              float pv[2], dv[2];
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const int j = c0 + i + e;
+                const uint32_t word = c.word[quarter][j];
+                const bool member = (word >> lane) & 1u;
+                const float sm = ex2_approx(fmaf(__uint_as_float(s[i + e]), c2, -c.lse[j]));
+                const float x = __uint_as_float(d[i + e]) - c.di[j];
+                if (member) atomicAdd(p.drw + (c.base[quarter][j] + __popc(word & lt_mask)), sm * x);
+                // (selected as a product: sm of a pair that is not a member may be infinite)
+                pv[e] = member ? sm * fmaxf(__uint_as_float(r[i + e]), 0.f) : 0.f;
+                dv[e] = pv[e] * x;
+              }
+              split3(pv[0], pv[1], pt[0][i >> 1], pt[1][i >> 1], pt[2][i >> 1]);
+              split3(dv[0], dv[1], dt[0][i >> 1], dt[1][i >> 1], dt[2][i >> 1]);
+            }
+            tmem_st8(buf + c0, pt[0]);
+            tmem_st8(buf + c0 + 8, pt[1]);
+            tmem_st8(buf + 64 + c0, pt[2]);
+            tmem_st8(buf + 64 + c0 + 8, dt[0]);
+            tmem_st8(buf + 128 + c0, dt[1]);
+            tmem_st8(buf + 128 + c0 + 8, dt[2]);
+          }
+          tc_wait_st();
+          tc_fence_before();
+        }
+        __syncwarp();
+        if (ok && lane == 0) mbar_arrive(&ctl->p_ready[t & 1]);
+        put(t + 1);
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+      }
+    } else {
+      float neg_lse = ninf, di = 0.f;                     // rows behind the end: sm = 0
+      if (MODE == kDq && row_ok) {
+        neg_lse = -__ldg(p.lse + bh * p.Tq + lrow);
+        di = __ldg(p.di + bh * p.Tq + lrow);
+      }
+      float m = ninf, mx = ninf, l = 0.f;                 // kStats: stabiliser, exact maximum, sum
+      const uint32_t* mrow = p.maskbits + ((static_cast<int64_t>(b) * p.nQT + lt) * p.nKT * kTile + row) * 4 + half;
+      auto fetch = [&](int t) -> uint32_t {
+        return (t < nS && row_ok) ? __ldg(mrow + static_cast<int64_t>(t >> 1) * (kTile * 4) + (t & 1) * 2) : 0u;
+      };
+      uint32_t next = fetch(0);
+      for (int t = 0; t < nS; ++t) {
+        const uint32_t word = next;
+        next = fetch(t + 1);
+        if (ok && !mbar_wait_bounded(&ctl->in_full[t & 1], (t >> 1) & 1, abort_flag)) {
+          record_status(p.status, kDevWaitAccFull);
+          ok = false;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t buf = tmem_base + lane_off + (t & 1) * kBufCols;
+        const int c0 = half * 32;
+        if constexpr (MODE == kStats) {
+          uint32_t s[32], r[32];
+          tmem_ld32(buf + c0, s);
+          tmem_ld32(buf + 64 + c0, r);
+          tc_wait_ld();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl->p_ready[t & 1]);
+          float mt = ninf;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            s[i] = ((word >> i) & 1u) ? __float_as_uint(__uint_as_float(s[i]) * c2) : __float_as_uint(ninf);
+            mt = fmaxf(mt, __uint_as_float(s[i]));
+          }
+          mx = fmaxf(mx, mt);
+          if (mt > m + 8.f) {                             // raise the stabiliser when it is 2^8 behind
+            l *= ex2_approx(m - mt);
+            m = mt;
+          }
+          const float neg_m = m == ninf ? 0.f : -m;
+          float l1 = 0.f;
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            l = fmaf(ex2_approx(__uint_as_float(s[i]) + neg_m), fmaxf(__uint_as_float(r[i]), 0.f), l);
+            l1 = fmaf(ex2_approx(__uint_as_float(s[i + 1]) + neg_m), fmaxf(__uint_as_float(r[i + 1]), 0.f), l1);
+          }
+          l += l1;
+        } else {
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int cc = c0 + k * 16;
+            uint32_t s[16], r[16], d[16];
+            tmem_ld16(buf + cc, s);
+            tmem_ld16(buf + 64 + cc, r);
+            tmem_ld16(buf + 128 + cc, d);
+            tc_wait_ld();
+            uint32_t dt[3][8];
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              float dv[2];
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const float sm = ex2_approx(fmaf(__uint_as_float(s[i + e]), c2, neg_lse));
+                const float pv = ((word >> (k * 16 + i + e)) & 1u) ? sm * fmaxf(__uint_as_float(r[i + e]), 0.f) : 0.f;
+                dv[e] = pv * (__uint_as_float(d[i + e]) - di);
+              }
+              split3(dv[0], dv[1], dt[0][i >> 1], dt[1][i >> 1], dt[2][i >> 1]);
+            }
+            tmem_st8(buf + 64 + cc + 8, dt[0]);
+            tmem_st8(buf + 128 + cc, dt[1]);
+            tmem_st8(buf + 128 + cc + 8, dt[2]);
+          }
+          tc_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl->p_ready[t & 1]);
+        }
+      }
+      if constexpr (MODE == kStats) {
+        ctl->xm[row][half] = m;
+        ctl->xe[row][half] = mx;
+        ctl->xl[row][half] = l;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (half == 0 && row_ok && ok) {
+          const float mm = fmaxf(ctl->xe[row][0], ctl->xe[row][1]);
+          float lt_ = 0.f;
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            if (ctl->xm[row][q] != ninf) lt_ = fmaf(ctl->xl[row][q], exp2f(ctl->xm[row][q] - mm), lt_);
+          // a row without members: +inf, all its weights are zero
+          p.lse[bh * p.Tq + lrow] = mm == ninf ? -ninf : mm + log2f(fmaxf(lt_, 1e-6f));
+        }
+      }
+    }
+
+    if constexpr (MODE != kStats) {
+      if (ok && !mbar_wait_bounded(&ctl->acc_final, 0, abort_flag)) {
+        record_status(p.status, kDevWaitPvDone);
+        ok = false;
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) {
+        tc_fence_after();
+#pragma unroll
+        for (int a = 0; a < (MODE == kDkv ? 2 : 1); ++a) {
+          uint32_t o[32];
+          tmem_ld32(tmem_base + lane_off + kColAcc + a * 64 + half * 32, o);
+          tc_wait_ld();
+          if (!row_ok) continue;
+          float* dst = (MODE == kDq ? p.dq : (a == 0 ? p.dv : p.dk)) +
+                       (bh * (MODE == kDkv ? p.Tk : p.Tq) + lrow) * kHd + half * 32;
+          const float f = MODE == kDkv && a == 0 ? 1.f : p.scale;
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<float4*>(dst + i) = make_float4(__uint_as_float(o[i]) * f, __uint_as_float(o[i + 1]) * f,
+                                                              __uint_as_float(o[i + 2]) * f, __uint_as_float(o[i + 3]) * f);
+        }
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    __syncwarp();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// ------------------------------------------------------------------ preparation
+// Per (batch, head, query) row: D = dO . O in fp32 and dO as bf16 (contiguous); `inexact` is raised when
+// some dO has more bits than bf16 holds.  Eight lanes per row.
+template <typename TO>
+__global__ void __launch_bounds__(256)
+    dsa_bwd_prep_kernel(const TO* __restrict__ d_out, int64_t db, int64_t dh, int64_t dt, const TO* __restrict__ o,
+                        int64_t ob, int64_t oh, int64_t ot, int B, int H, int T, __nv_bfloat16* __restrict__ do16,
+                        float* __restrict__ di, int* __restrict__ inexact) {
+  const int64_t r = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) >> 3;
+  const int c = (threadIdx.x & 7) * 8;
+  const bool in = r < static_cast<int64_t>(B) * H * T;
+  float acc = 0.f;
+  bool bad = false;
+  int64_t row = 0;
+  if (in) {
+    // rows in token-major order, the order of the caller's strided views
+    const int h = static_cast<int>(r % H);
+    const int64_t bt = r / H;
+    const int t = static_cast<int>(bt % T), b = static_cast<int>(bt / T);
+    const TO* x = d_out + b * db + h * dh + t * dt + c;
+    const TO* y = o + b * ob + h * oh + t * ot + c;
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      float a[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        a[e] = static_cast<float>(x[i + e]);
+        acc = fmaf(a[e], static_cast<float>(y[i + e]), acc);
+      }
+      w[i >> 1] = pack_bf16x2(a[0], a[1]);
+      bad |= __uint_as_float(w[i >> 1] << 16) != a[0] || __uint_as_float(w[i >> 1] & 0xffff0000u) != a[1];
+    }
+    row = (static_cast<int64_t>(b) * H + h) * T + t;
+    *reinterpret_cast<uint4*>(do16 + row * kHd + c) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+  if (in && c == 0) di[row] = acc;
+  if (sizeof(TO) != 2 || std::is_same<TO, __half>::value) {
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) *inexact = 1;
+  }
+}
+
+// off[b][kt][i] = first slot of row i whose key lies in tile kt or later (kt = 0 .. nKT); one warp per
+// row of the ascending lists (`n` slots are valid in every row).
+__global__ void __launch_bounds__(256)
+    dsa_bwd_offsets_kernel(const int32_t* __restrict__ idx, int top_k, int n, int B, int T, int nKT,
+                           uint16_t* __restrict__ off) {
+  const int64_t r = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (r >= static_cast<int64_t>(B) * T) return;
+  const int b = static_cast<int>(r / T), t = static_cast<int>(r % T);
+  const int32_t* row = idx + r * top_k;
+  uint16_t* dst = off + static_cast<int64_t>(b) * (nKT + 1) * T + t;
+  int carry = -1;                                        // tile of the slot before this group
+  for (int s0 = 0; s0 < n; s0 += 32) {
+    const int s = s0 + lane;
+    const int kt = s < n ? min(max(__ldg(row + s) >> 7, 0), nKT - 1) : nKT;
+    int before = __shfl_up_sync(0xffffffffu, kt, 1);
+    if (lane == 0) before = carry;
+    if (s < n)
+      for (int q = before + 1; q <= kt; ++q) dst[static_cast<int64_t>(q) * T] = static_cast<uint16_t>(s);
+    carry = __shfl_sync(0xffffffffu, kt, min(31, n - 1 - s0));
+  }
+  for (int q = carry + 1 + lane; q <= nKT; q += 32) dst[static_cast<int64_t>(q) * T] = static_cast<uint16_t>(n);
+}
+
+// ------------------------------------------------------------ indexer gradients
+// kLaneQ : lanes = queries of one tile, the key tiles streamed:  dq_idx = W G K_idx, and dW
+// kLaneK : lanes = keys of one tile, the query tiles streamed:   dk_idx = W G^T Q_idx
+// G is the dense 128 x 128 tile of the list gradients: eight warps clear the tile's three bf16 terms in
+// shared memory and scatter the listed pairs into them (two threads per query row), one thread multiplies
+// them with the streamed 128 x E tile of the projections (E = IH * ID, N of the instruction).
+// Bound: those products, 24 instructions of E/2 cycles per tile; the lists are read twice in all.
+struct IdxTileCtl {
+  uint64_t full[2], empty[2], g_full, done;
+  uint32_t tmem_base, abort_flag;
+};
+struct IdxTileParams {
+  int B, Tq, Tk, nQT, nKT, top_k, IH, ID;
+  const int32_t* idx;
+  const float* g;           // (B,Tq,top_k)
+  const uint16_t* off;
+  const float* w;
+  const __nv_bfloat16* q_idx;
+  int64_t qsb, qst;
+  float *dx, *dw;           // dq_idx or dk_idx
+  int* status;
+};
+constexpr int kTermBytes = kTile * kTile * 2;           // one bf16 term of G: two 64-column halves of 16 KiB
+constexpr int kOffB = 3 * kTermBytes;
+constexpr size_t idx_smem(int E, int stages) {
+  return 1024 + kOffB + static_cast<size_t>(stages) * kTile * E * 2 + sizeof(IdxTileCtl) + 64;
+}
+enum { kLaneQ = 0, kLaneK = 1 };
+
+template <int MODE, int E>
+__global__ void __launch_bounds__(320, 1)
+    dsa_idx_bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_b, const IdxTileParams p) {
+  constexpr int NST = 2;
+  constexpr int kBBytes = kTile * E * 2;
+  constexpr uint32_t kIdesc = make_idesc(/*bf16*/ 1, kTile, E, 0, /*B is MN-major*/ 1);
+  constexpr int kPre = 8;                                // list entries a thread loads ahead
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  IdxTileCtl* ctl = reinterpret_cast<IdxTileCtl*>(smem + kOffB + NST * kBBytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nLT = MODE == kLaneQ ? p.nQT : p.nKT, nS = MODE == kLaneQ ? p.nKT : p.nQT;
+  const int lt = blockIdx.x % nLT, b = blockIdx.x / nLT;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NST; ++s) {
+      mbar_init(&ctl->full[s], 1);
+      mbar_init(&ctl->empty[s], 1);
+    }
+    mbar_init(&ctl->g_full, 8);
+    mbar_init(&ctl->done, 1);
+    ctl->abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&ctl->tmem_base, 256);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = ctl->tmem_base;
+  volatile uint32_t* abort_flag = &ctl->abort_flag;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int t = 0; t < nS; ++t) {
+        const int s = t & 1;
+        if (!mbar_wait_bounded(&ctl->empty[s], ((t >> 1) & 1) ^ 1, abort_flag)) {
+          record_status(p.status, kDevWaitStageEmpty);
+          break;
+        }
+        mbar_expect_tx(&ctl->full[s], kBBytes);
+#pragma unroll
+        for (int c = 0; c < E / 64; ++c)
+          tma_load_3d(smem + kOffB + s * kBBytes + c * (kTile * 128), &tm_b, &ctl->full[s], c * 64, t * kTile, b);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t a0 = smem_u32(smem), b0 = a0 + kOffB;
+      for (int t = 0; t < nS; ++t) {
+        const int s = t & 1;
+        if (!mbar_wait_bounded(&ctl->full[s], (t >> 1) & 1, abort_flag)) {
+          record_status(p.status, kDevWaitTmaFull);
+          break;
+        }
+        if (!mbar_wait_bounded(&ctl->g_full, t & 1, abort_flag)) {
+          record_status(p.status, kDevWaitPReady);
+          break;
+        }
+        tc_fence_after();
+        const uint64_t db = smem_desc_sw128(b0 + s * kBBytes, kTile * 128);
+#pragma unroll
+        for (int term = 0; term < 3; ++term) {
+          const uint64_t da = smem_desc_sw128(a0 + term * kTermBytes);
+#pragma unroll
+          for (int ks = 0; ks < kTile / 16; ++ks)
+            umma_f16_ss(tmem_base, da + (ks >> 2) * (kTile * 128 / 16) + (ks & 3) * 2, db + ks * 128, kIdesc,
+                        t > 0 || term > 0 || ks > 0);
+        }
+        umma_commit(&ctl->empty[s]);
+        umma_commit(&ctl->done);
+      }
+    }
+  } else {
+    const int ct = threadIdx.x - 64;
+    const int r = ct >> 1, par = ct & 1;                 // query row of the tile, which half of its entries
+    const uint32_t g_addr = smem_u32(smem);
+    bool ok = true;
+    // the entries of tile t: slots [s0, s1) of the row; this thread takes s0 + par, + 2, ...
+    int s0 = 0, s1 = 0, id[kPre];
+    float gv[kPre];
+    int64_t rowbase = 0;
+    auto fetch = [&](int t) {
+      const int qt = MODE == kLaneQ ? lt : t, kt = MODE == kLaneQ ? t : lt;
+      const int i = qt * kTile + r;
+      s0 = s1 = 0;
+      if (t < nS && i < p.Tq) {
+        const uint16_t* o = p.off + (static_cast<int64_t>(b) * (p.nKT + 1) + kt) * p.Tq + i;
+        rowbase = (static_cast<int64_t>(b) * p.Tq + i) * p.top_k;
+        s0 = __ldg(o) + par;
+        s1 = __ldg(o + p.Tq);
+      }
+#pragma unroll
+      for (int e = 0; e < kPre; ++e) {
+        const bool in = s0 + 2 * e < s1;
+        id[e] = in ? __ldg(p.idx + rowbase + s0 + 2 * e) : 0;
+        gv[e] = in ? __ldg(p.g + rowbase + s0 + 2 * e) : 0.f;
+      }
+    };
+    auto place = [&](int key, float g) {
+      const int j = key & (kTile - 1);
+      const int m = MODE == kLaneQ ? r : j, k = MODE == kLaneQ ? j : r;       // lane-side row, streamed index
+      const uint32_t a = g_addr + (k >> 6) * (kTile * 128) + m * 128 + ((((k & 63) >> 3) ^ (m & 7)) << 4) + (k & 7) * 2;
+      uint32_t hi, mid, lo;
+      split3(g, 0.f, hi, mid, lo);
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(static_cast<uint16_t>(hi)) : "memory");
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(a + kTermBytes), "h"(static_cast<uint16_t>(mid)) : "memory");
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(a + 2 * kTermBytes), "h"(static_cast<uint16_t>(lo)) : "memory");
+    };
+    fetch(0);
+    for (int t = 0; t < nS; ++t) {
+      if (t > 0 && ok && !mbar_wait_bounded(&ctl->done, (t - 1) & 1, abort_flag)) {
+        record_status(p.status, kDevWaitPvDone);
+        ok = false;
+      }
+#pragma unroll
+      for (int i = 0; i < 3 * kTermBytes / 16 / 256; ++i) sts128(g_addr + (i * 256 + ct) * 16, 0u, 0u, 0u, 0u);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+#pragma unroll
+      for (int e = 0; e < kPre; ++e)
+        if (s0 + 2 * e < s1) place(id[e], gv[e]);
+      for (int s = s0 + 2 * kPre; s < s1; s += 2) place(__ldg(p.idx + rowbase + s), __ldg(p.g + rowbase + s));
+      fence_proxy_async_smem();
+      __syncwarp();
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok && lane == 0) mbar_arrive(&ctl->g_full);
+      fetch(t + 1);
+    }
+    if (ok && !mbar_wait_bounded(&ctl->done, (nS - 1) & 1, abort_flag)) {
+      record_status(p.status, kDevWaitPvDone);
+      ok = false;
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok) {
+      tc_fence_after();
+      const int quarter = warp & 3, half = (warp - 2) >> 2;
+      const int lrow = lt * kTile + quarter * 32 + lane;
+      const int T = MODE == kLaneQ ? p.Tq : p.Tk;
+      const bool row_ok = lrow < T;
+      const uint32_t acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (E / 2);
+      float* dst = p.dx + (static_cast<int64_t>(b) * T + lrow) * E + half * (E / 2);
+      const __nv_bfloat16* qrow = p.q_idx + b * p.qsb + lrow * p.qst + half * (E / 2);
+      float dw = 0.f;
+      int head = half * (E / 2) / p.ID;
+#pragma unroll 1
+      for (int c = 0; c < E / 2; c += 16) {
+        uint32_t o[16];
+        tmem_ld16(acc + c, o);
+        tc_wait_ld();
+        uint4 qv[2];
+        if (MODE == kLaneQ && row_ok) {
+          qv[0] = __ldg(reinterpret_cast<const uint4*>(qrow + c));
+          qv[1] = __ldg(reinterpret_cast<const uint4*>(qrow + c) + 1);
+        } else {
+          qv[0] = qv[1] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        const uint32_t qw[8] = {qv[0].x, qv[0].y, qv[0].z, qv[0].w, qv[1].x, qv[1].y, qv[1].z, qv[1].w};
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int e = half * (E / 2) + c + i, hh = e / p.ID;
+          if (MODE == kLaneQ && hh != head) {            // (uniform) the head's sum is complete
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) dw += __shfl_xor_sync(0xffffffffu, dw, off);
+            if (lane == 0) atomicAdd(p.dw + head, dw);
+            dw = 0.f;
+            head = hh;
+          }
+          x[i] = __uint_as_float(o[i]);
+          if (MODE == kLaneQ) dw = fmaf(x[i], __uint_as_float((i & 1) ? qw[i >> 1] & 0xffff0000u : qw[i >> 1] << 16), dw);
+          x[i] *= __ldg(p.w + hh);
+        }
+        if (row_ok) {
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(dst + c + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+        }
+      }
+      if (MODE == kLaneQ) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) dw += __shfl_xor_sync(0xffffffffu, dw, off);
+        if (lane == 0) atomicAdd(p.dw + head, dw);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    __syncwarp();
+    tmem_dealloc(tmem_base, 256);
+  }
+}
+
+size_t up256(size_t x) { return (x + 255) / 256 * 256; }
+struct BwdLayout {
+  size_t do16, di, lse, wq, wk, off, flag, total;
+};
+BwdLayout bwd_layout(int B, int H, int Tq, int Tk) {
+  BwdLayout L;
+  const size_t rows = static_cast<size_t>(B) * H * Tq;
+  const size_t nKT = (Tk + kTile - 1) / kTile;
+  size_t o = 0;
+  L.do16 = o; o += up256(rows * kHd * 2);
+  L.di = o; o += up256(rows * 4);
+  L.lse = o; o += up256(rows * 4);
+  L.wq = o; o += up256(static_cast<size_t>(B) * Tq * kIdxDim * 4);
+  L.wk = o; o += up256(static_cast<size_t>(B) * Tk * kIdxDim * 4);
+  L.off = o; o += up256(static_cast<size_t>(B) * (nKT + 1) * Tq * 2);
+  L.flag = o; o += 256;
+  L.total = o;
+  return L;
+}
+
+template <int MODE>
+int launch_bwd(const CUtensorMap& l1, const CUtensorMap& l2, const CUtensorMap& lr, const CUtensorMap& s1,
+               const CUtensorMap& s2, const CUtensorMap& sr, const BwdTileParams& p, cudaStream_t st) {
+  SWV_CUDA_OK(cudaFuncSetAttribute(dsa_bwd_tiles_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(kBwdSmem)));
+  const unsigned grid = static_cast<unsigned>(p.B) * p.H * (MODE == kDkv ? p.nKT : p.nQT);
+  dsa_bwd_tiles_kernel<MODE><<<grid, 320, kBwdSmem, st>>>(l1, l2, lr, s1, s2, sr, p);
+  SWV_CUDA_OK(cudaGetLastError());
+  return SWV_OK;
+}
+
+template <int MODE, int E>
+int launch_idx(const CUtensorMap& tb, const IdxTileParams& p, cudaStream_t st) {
+  constexpr size_t smem = idx_smem(E, 2);
+  SWV_CUDA_OK(cudaFuncSetAttribute(dsa_idx_bwd_tiles_kernel<MODE, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(smem)));
+  dsa_idx_bwd_tiles_kernel<MODE, E><<<static_cast<unsigned>(p.B) * (MODE == kLaneQ ? p.nQT : p.nKT), 320, smem, st>>>(tb, p);
+  SWV_CUDA_OK(cudaGetLastError());
+  return SWV_OK;
+}
+
+template <typename TO>
+int launch_prep(const void* d_out, const int64_t* ds, const void* o, const int64_t* os, int B, int H, int T, void* do16,
+                float* di, int* flag, cudaStream_t st) {
+  const int64_t threads = static_cast<int64_t>(B) * H * T * 8;
+  dsa_bwd_prep_kernel<TO><<<static_cast<unsigned>((threads + 255) / 256), 256, 0, st>>>(
+      static_cast<const TO*>(d_out), ds[0], ds[1], ds[2], static_cast<const TO*>(o), os[0], os[1], os[2], B, H, T,
+      static_cast<__nv_bfloat16*>(do16), di, flag);
+  SWV_CUDA_OK(cudaGetLastError());
+  return SWV_OK;
+}
+
+bool rows16(const void* p, const int64_t* s, int n) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15) || s[n] != 1) return false;
+  for (int i = 0; i < n; ++i)
+    if ((s[i] * 2) % 16) return false;
+  return true;
+}
+
+}  // namespace
+
+int dsa_collapse_impl(const void* x, const int64_t* s, int dtype, const float* w, float* out, int B, int Tn, int IH,
+                      int ID, cudaStream_t st);
+int dsa_attn_bwd_impl(const void* d_out, const int64_t* dos, const void* q, const int64_t* qs, const void* k,
+                      const int64_t* ks, const void* v, const int64_t* vs, int dtype, const void* o,
+                      const int64_t* os, int o_dtype, const int32_t* idx, const int64_t* is, const float* valid,
+                      const int64_t* vls, const float* rw, const int64_t* rs, float* dq, float* dk, float* dv,
+                      float* drw, int B, int H, int Tq, int Tk, int D, int top_k, int* status, cudaStream_t st,
+                      const int* run_if);
+int dsa_indexer_bwd_impl(const float* d_scores, const int64_t* dss, const void* q_idx, const int64_t* qs,
+                         const void* k_idx, const int64_t* ks, int dtype, const float* w, const int32_t* idx,
+                         const int64_t* is, const float* valid, const int64_t* vls, float* dq, float* dk, float* dw,
+                         int B, int Tq, int Tk, int IH, int ID, int top_k, int* status, cudaStream_t st);
+
+int dsa_module_bwd_bytes_impl(int B, int H, int Tq, int Tk, size_t* bytes) {
+  if (!bytes) return SWV_ERR_NULL;
+  if (B < 1 || H < 1 || Tq < 1 || Tk < 1) return SWV_ERR_SHAPE;
+  *bytes = bwd_layout(B, H, Tq, Tk).total;
+  return SWV_OK;
+}
+
+int dsa_module_bwd_impl(const void* d_out, const int64_t* dos, const void* q, const int64_t* qs, const void* k,
+                        const int64_t* ks, const void* v, const int64_t* vs, const void* o, const int64_t* os,
+                        int o_dtype, const void* q_idx, const int64_t* qis, const void* k_idx, const int64_t* kis,
+                        int idx_dtype, const float* w, const int32_t* idx, const float* valid, const float* scores,
+                        const uint32_t* maskbits, float* dq, float* dk, float* dv, float* drw, float* dq_idx,
+                        float* dk_idx, float* dw, int B, int H, int Tq, int Tk, int D, int IH, int ID, int top_k,
+                        void* workspace, size_t workspace_bytes, int* status, cudaStream_t st) {
+  if (!d_out || !q || !k || !v || !o || !q_idx || !k_idx || !w || !idx || !valid || !scores || !maskbits || !dq || !dk ||
+      !dv || !drw || !dq_idx || !dk_idx || !dw || !workspace || !status)
+    return SWV_ERR_NULL;
+  if (B < 1 || H < 1 || Tq < 1 || Tk < 1 || top_k < 1 || IH < 1 || ID < 1) return SWV_ERR_SHAPE;
+  // list slots are 16-bit offsets, list positions 32-bit
+  if (D != kHd || ID > kIdxDim || top_k > 65535 || static_cast<uint64_t>(B) * Tq * top_k >= (1ull << 32))
+    return SWV_ERR_UNSUPPORTED;
+  if (!rows16(q, qs, 3) || !rows16(k, ks, 3) || !rows16(v, vs, 3) || dos[3] != 1 || os[3] != 1) return SWV_ERR_ALIGN;
+  const BwdLayout L = bwd_layout(B, H, Tq, Tk);
+  if (workspace_bytes < L.total) return SWV_ERR_WORKSPACE;
+  if (reinterpret_cast<uintptr_t>(workspace) & 255) return SWV_ERR_ALIGN;
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  void* do16 = ws + L.do16;
+  float* di = reinterpret_cast<float*>(ws + L.di);
+  float* wq = reinterpret_cast<float*>(ws + L.wq);
+  float* wk = reinterpret_cast<float*>(ws + L.wk);
+  uint16_t* off = reinterpret_cast<uint16_t*>(ws + L.off);
+  int* flag = reinterpret_cast<int*>(ws + L.flag);
+  const int nQT = (Tq + kTile - 1) / kTile, nKT = (Tk + kTile - 1) / kTile;
+  const int64_t ls[3] = {static_cast<int64_t>(Tq) * top_k, top_k, 1};
+
+  int rc;
+  const bool exact = o_dtype == SWV_BF16;
+  if (!exact) SWV_CUDA_OK(cudaMemsetAsync(flag, 0, sizeof(int), st));
+  if (o_dtype == SWV_F32) rc = launch_prep<float>(d_out, dos, o, os, B, H, Tq, do16, di, flag, st);
+  else if (o_dtype == SWV_BF16) rc = launch_prep<__nv_bfloat16>(d_out, dos, o, os, B, H, Tq, do16, di, flag, st);
+  else if (o_dtype == SWV_F16) rc = launch_prep<__half>(d_out, dos, o, os, B, H, Tq, do16, di, flag, st);
+  else return SWV_ERR_DTYPE;
+  if (rc != SWV_OK) return rc;
+  if (exact) {
+    SWV_CUDA_OK(cudaMemsetAsync(drw, 0, static_cast<size_t>(B) * Tq * top_k * sizeof(float), st));
+  } else {
+    // clears dk, dv, drw and, where some dO does not fit bf16, computes them
+    rc = dsa_attn_bwd_impl(d_out, dos, q, qs, k, ks, v, vs, SWV_BF16, o, os, o_dtype, idx, ls, valid, ls, scores, ls, dq,
+                           dk, dv, drw, B, H, Tq, Tk, D, top_k, status, st, flag);
+    if (rc != SWV_OK) return rc;
+  }
+  rc = dsa_collapse_impl(q_idx, qis, idx_dtype, w, wq, B, Tq, IH, ID, st);
+  if (rc != SWV_OK) return rc;
+  rc = dsa_collapse_impl(k_idx, kis, idx_dtype, w, wk, B, Tk, IH, ID, st);
+  if (rc != SWV_OK) return rc;
+  const int64_t rows = static_cast<int64_t>(B) * Tq;
+  dsa_bwd_offsets_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, st>>>(idx, top_k, top_k < Tk ? top_k : Tk, B, Tq,
+                                                                              nKT, off);
+  SWV_CUDA_OK(cudaGetLastError());
+
+  // maps with 128-row boxes (lane side) and 64-row boxes (streamed side)
+  CUtensorMap mq[2], mk[2], mv[2], md[2], mwq[2], mwk[2];
+  const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t box = i == 0 ? kTile : kNW;
+    if ((rc = make_tmap_4d(&mq[i], q, bf, D, Tq, H, B, qs[2] * 2, qs[1] * 2, qs[0] * 2, kHd, box)) != SWV_OK) return rc;
+    if ((rc = make_tmap_4d(&mk[i], k, bf, D, Tk, H, B, ks[2] * 2, ks[1] * 2, ks[0] * 2, kHd, box)) != SWV_OK) return rc;
+    if ((rc = make_tmap_4d(&mv[i], v, bf, D, Tk, H, B, vs[2] * 2, vs[1] * 2, vs[0] * 2, kHd, box)) != SWV_OK) return rc;
+    if ((rc = make_tmap_4d(&md[i], do16, bf, D, Tq, H, B, kHd * 2, static_cast<uint64_t>(Tq) * kHd * 2,
+                           static_cast<uint64_t>(H) * Tq * kHd * 2, kHd, box)) != SWV_OK) return rc;
+    if ((rc = make_tmap_3d(&mwq[i], wq, f32, kIdxDim, Tq, B, kIdxDim * 4, static_cast<uint64_t>(Tq) * kIdxDim * 4, 32,
+                           box)) != SWV_OK) return rc;
+    if ((rc = make_tmap_3d(&mwk[i], wk, f32, kIdxDim, Tk, B, kIdxDim * 4, static_cast<uint64_t>(Tk) * kIdxDim * 4, 32,
+                           box)) != SWV_OK) return rc;
+  }
+  BwdTileParams p;
+  p.B = B; p.H = H; p.Tq = Tq; p.Tk = Tk; p.nQT = nQT; p.nKT = nKT; p.top_k = top_k;
+  p.maskbits = maskbits; p.off = off; p.di = di; p.lse = reinterpret_cast<float*>(ws + L.lse);
+  p.dq = dq; p.dk = dk; p.dv = dv; p.drw = drw;
+  p.scale = 1.0f / sqrtf(static_cast<float>(D));
+  p.c2 = p.scale * 1.4426950408889634f;
+  p.skip_if = exact ? nullptr : flag;
+  p.status = status;
+  if ((rc = launch_bwd<kStats>(mq[0], mq[0], mwq[0], mk[1], mk[1], mwk[1], p, st)) != SWV_OK) return rc;
+  if ((rc = launch_bwd<kDkv>(mk[0], mv[0], mwk[0], mq[1], md[1], mwq[1], p, st)) != SWV_OK) return rc;
+  if ((rc = launch_bwd<kDq>(mq[0], md[0], mwq[0], mk[1], mv[1], mwk[1], p, st)) != SWV_OK) return rc;
+
+  // indexer: tiles for bf16 projections whose heads lie side by side, else the list kernel
+  const int E = IH * ID;
+  const int64_t q3[3] = {qis[0], qis[1], qis[3]}, k3[3] = {kis[0], kis[1], kis[3]};
+  if (idx_dtype == SWV_BF16 && (E == 64 || E == 128 || E == 256) && qis[2] == ID && kis[2] == ID && rows16(q_idx, q3, 2) &&
+      rows16(k_idx, k3, 2)) {
+    CUtensorMap tq, tk;
+    if ((rc = make_tmap_3d(&tq, q_idx, bf, E, Tq, B, qis[1] * 2, qis[0] * 2, 64, kTile)) != SWV_OK) return rc;
+    if ((rc = make_tmap_3d(&tk, k_idx, bf, E, Tk, B, kis[1] * 2, kis[0] * 2, 64, kTile)) != SWV_OK) return rc;
+    SWV_CUDA_OK(cudaMemsetAsync(dw, 0, static_cast<size_t>(IH) * sizeof(float), st));
+    IdxTileParams ip;
+    ip.B = B; ip.Tq = Tq; ip.Tk = Tk; ip.nQT = nQT; ip.nKT = nKT; ip.top_k = top_k; ip.IH = IH; ip.ID = ID;
+    ip.idx = idx; ip.g = drw; ip.off = off; ip.w = w;
+    ip.q_idx = static_cast<const __nv_bfloat16*>(q_idx); ip.qsb = qis[0]; ip.qst = qis[1];
+    ip.dx = dq_idx; ip.dw = dw; ip.status = status;
+    if (E == 64) rc = launch_idx<kLaneQ, 64>(tk, ip, st);
+    else if (E == 128) rc = launch_idx<kLaneQ, 128>(tk, ip, st);
+    else rc = launch_idx<kLaneQ, 256>(tk, ip, st);
+    if (rc != SWV_OK) return rc;
+    ip.dx = dk_idx;
+    if (E == 64) return launch_idx<kLaneK, 64>(tq, ip, st);
+    if (E == 128) return launch_idx<kLaneK, 128>(tq, ip, st);
+    return launch_idx<kLaneK, 256>(tq, ip, st);
+  }
+  return dsa_indexer_bwd_impl(drw, ls, q_idx, qis, k_idx, kis, idx_dtype, w, idx, ls, valid, ls, dq_idx, dk_idx, dw, B, Tq,
+                              Tk, IH, ID, top_k, status, st);
+}
+
+}  // namespace swv

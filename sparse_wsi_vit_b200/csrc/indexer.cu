@@ -1319,6 +1319,16 @@ static void launch_collapse(const void* x, const int64_t* s, const float* w, flo
                                                          Tn, IH, ID);
 }
 
+int dsa_collapse_impl(const void* x, const int64_t* s, int dtype, const float* w, float* out, int B, int Tn, int IH,
+                      int ID, cudaStream_t st) {
+  if (dtype == SWV_F32) launch_collapse<float>(x, s, w, out, B, Tn, IH, ID, st);
+  else if (dtype == SWV_BF16) launch_collapse<__nv_bfloat16>(x, s, w, out, B, Tn, IH, ID, st);
+  else if (dtype == SWV_F16) launch_collapse<__half>(x, s, w, out, B, Tn, IH, ID, st);
+  else return SWV_ERR_DTYPE;
+  SWV_CUDA_OK(cudaGetLastError());
+  return SWV_OK;
+}
+
 int dsa_workspace_bytes_topk_impl(int B, int Tq, int Tk, int top_k, size_t* bytes) {
   if (bytes == nullptr) return SWV_ERR_NULL;
   if (B < 1 || Tq < 1 || Tk < 1 || top_k < 1) return SWV_ERR_SHAPE;

@@ -305,9 +305,16 @@ def dsa_sparse_attention(q, k, v, q_idx, k_idx, w, top_k, out_dtype=None, return
     event after which k and v are complete (they may still be in flight on another
     stream while the indexer runs, which needs only q_idx / k_idx).
     """
+    o, idx, valid, scores, _ = _dsa_forward(q, k, v, q_idx, k_idx, w, top_k, out_dtype, kv_ready, rope)
+    return (o, idx, valid, scores) if return_topk else o
+
+
+def _dsa_forward(q, k, v, q_idx, k_idx, w, top_k, out_dtype=None, kv_ready=None, rope=None):
+    """``dsa_sparse_attention`` that also returns the selection handle (None on the gather path)."""
     B, H, Tq, D = q.shape
     dev = q.device
     out_dtype = out_dtype or q.dtype
+    sel = None
     o = torch.empty((B, H, Tq, D), dtype=out_dtype, device=dev)
     dense = q.dtype == torch.bfloat16 and D == 64
     ws, pre = None, False
@@ -328,7 +335,7 @@ def dsa_sparse_attention(q, k, v, q_idx, k_idx, w, top_k, out_dtype=None, return
         if kv_ready is not None:
             torch.cuda.current_stream(dev).wait_event(kv_ready)
         dsa_attention_gather(q, k, v, idx, valid, scores * valid, o)
-    return (o, idx, valid, scores) if return_topk else o
+    return o, idx, valid, scores, sel
 
 
 def dsa_attention_bwd(d_out, q, k, v, o, idx, valid, rw):
@@ -389,6 +396,40 @@ def dsa_indexer_bwd(d_scores, q_idx, k_idx, w, idx, valid):
     return dq, dk, dw
 
 
+def dsa_module_bwd(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores, mask):
+    """``dsa_attention_bwd`` (with ``rw = scores * valid``) and ``dsa_indexer_bwd`` of its ``drw`` in one call
+    on tensor-core tiles, for lists and bitmask of this library's indexer on the same projections; bf16
+    q, k, v with head_dim 64.  Returns fp32 ``dq, dk, dv, dq_idx, dk_idx, dw``."""
+    _require_cuda(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores, mask)
+    B, H, Tq, D = q.shape
+    Tk, top_k = k.shape[2], idx.shape[-1]
+    IH, ID = q_idx.shape[2:]
+    dev = q.device
+    q, k, v = (t if _tma_ok(t) else t.contiguous() for t in (q, k, v))
+    d_out = d_out if d_out.dtype == o.dtype else d_out.to(o.dtype)
+    if d_out.stride(-1) != 1:
+        d_out = d_out.contiguous()
+    if k_idx.dtype != q_idx.dtype:
+        k_idx = k_idx.to(q_idx.dtype)
+    w32 = w.detach().to(torch.float32).contiguous()
+    f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)
+    dq, dk, dv, drw = f32(B, H, Tq, D), f32(B, H, Tk, D), f32(B, H, Tk, D), f32(B, Tq, top_k)
+    dqi, dki, dw = f32(B, Tq, IH, ID), f32(B, Tk, IH, ID), f32(IH)
+    nws = ctypes.c_size_t()
+    check(lib.swv_dsa_module_bwd_bytes(B, H, Tq, Tk, ctypes.byref(nws)), "swv_dsa_module_bwd_bytes")
+    ws = torch.empty(nws.value, dtype=torch.uint8, device=dev)
+    rc = lib.swv_dsa_module_bwd(
+        d_out.data_ptr(), strides(d_out), q.data_ptr(), strides(q), k.data_ptr(), strides(k), v.data_ptr(), strides(v),
+        o.data_ptr(), strides(o), dtype_code(o.dtype), q_idx.data_ptr(), strides(q_idx), k_idx.data_ptr(), strides(k_idx),
+        dtype_code(q_idx.dtype), w32.data_ptr(), idx.data_ptr(), valid.data_ptr(), scores.data_ptr(), mask.data_ptr(),
+        dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), drw.data_ptr(), dqi.data_ptr(), dki.data_ptr(), dw.data_ptr(),
+        B, H, Tq, Tk, D, IH, ID, top_k, ws.data_ptr(), nws.value, status_word(dev).data_ptr(), _stream(dev))
+    check(rc, "swv_dsa_module_bwd")
+    if _CHECK:
+        check_status(dev, "swv_dsa_module_bwd")
+    return dq, dk, dv, dqi, dki, dw
+
+
 class LightningIndexerFunction(torch.autograd.Function):
     """Same positional signature as the reference (kernels.py:346-352).  The tile
     sizes are accepted and ignored; outputs are allocated here (kernels.py:355-357)."""
@@ -443,18 +484,21 @@ class DSAModuleFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, q_idx, k_idx, w, top_k, out_dtype):
-        o, idx, valid, scores = dsa_sparse_attention(q.detach(), k.detach(), v.detach(), q_idx.detach(),
-                                                     k_idx.detach(), w.detach(), top_k, out_dtype=out_dtype,
-                                                     return_topk=True)
-        ctx.save_for_backward(q, k, v, q_idx, k_idx, w, idx, valid, scores, o)
+        o, idx, valid, scores, sel = _dsa_forward(q.detach(), k.detach(), v.detach(), q_idx.detach(), k_idx.detach(),
+                                                  w.detach(), top_k, out_dtype=out_dtype)
+        ctx.save_for_backward(q, k, v, q_idx, k_idx, w, idx, valid, scores, o, None if sel is None else sel[0])
         return o
 
     @staticmethod
     def backward(ctx, d_out):
-        q, k, v, q_idx, k_idx, w, idx, valid, scores, o = ctx.saved_tensors
-        dq, dk, dv, drw = dsa_attention_bwd(d_out.contiguous(), q, k, v, o, idx, valid, scores * valid)
-        # d scores = d rw * valid; the indexer backward multiplies by valid itself (valid is 0 or 1)
-        dqi, dki, dw = dsa_indexer_bwd(drw, q_idx, k_idx, w, idx, valid)
+        q, k, v, q_idx, k_idx, w, idx, valid, scores, o, mask = ctx.saved_tensors
+        # the tile form addresses lists by 16-bit slots and 32-bit positions
+        if mask is not None and idx.shape[-1] < 65536 and idx.numel() < 1 << 32 and q_idx.shape[-1] <= 64:
+            dq, dk, dv, dqi, dki, dw = dsa_module_bwd(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores, mask)
+        else:
+            dq, dk, dv, drw = dsa_attention_bwd(d_out.contiguous(), q, k, v, o, idx, valid, scores * valid)
+            # d scores = d rw * valid; the indexer backward multiplies by valid itself (valid is 0 or 1)
+            dqi, dki, dw = dsa_indexer_bwd(drw, q_idx, k_idx, w, idx, valid)
         return (dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), dqi.to(q_idx.dtype), dki.to(k_idx.dtype),
                 dw.to(w.dtype), None, None)
 

@@ -156,3 +156,38 @@ def test_encoder_train_steps_reduce_the_loss(swv):
     assert losses[-1] < losses[0], losses
     for n, p_ in net.named_parameters():
         assert p_.grad is not None and torch.isfinite(p_.grad).all(), n
+
+
+@pytest.mark.parametrize("B,T,H,IH,ID,K,o_dtype,exact", [
+    (1, 64, 1, 4, 32, 16, torch.bfloat16, True),      # less than one tile
+    (1, 128, 2, 4, 64, 128, torch.float32, True),     # every key selected, exactly one tile
+    (2, 300, 3, 4, 32, 40, torch.float32, True),      # ragged tiles, batch, fp32 output with bf16-exact gradients
+    (1, 517, 2, 4, 64, 96, torch.float32, False),     # gradients with more bits than bf16: the list kernel takes over
+    (1, 260, 1, 2, 32, 300, torch.bfloat16, True),    # more slots than keys, one 64-channel projection block
+    (1, 391, 2, 3, 64, 33, torch.bfloat16, True),     # 192 projection channels: indexer gradients on the list kernel
+])
+def test_tile_backward_vs_oracle(swv, B, T, H, IH, ID, K, o_dtype, exact):
+    """The tensor-core backward on the selection of the library's own indexer, against the oracle's
+    backward on the same lists: fp32-grade agreement (its factors carry 24 bits), the same tolerance as the
+    CUDA-core kernels."""
+    g = torch.Generator().manual_seed(T + K)
+    bf = torch.bfloat16
+    q = (torch.randn(B, T, H, 64, generator=g) / 8).to(bf).to(DEV).transpose(1, 2)
+    k, v = (torch.randn(B, T, H, 64, generator=g).to(bf).to(DEV).transpose(1, 2) for _ in range(2))
+    qi, ki = ((torch.randn(B, T, IH, ID, generator=g) / ID ** 0.5).to(bf).to(DEV) for _ in range(2))
+    w = torch.randn(IH, generator=g).to(DEV)
+    d_out = torch.randn(B, T, H, 64, generator=g)
+    d_out = (d_out.to(bf) if exact else d_out).to(o_dtype).to(DEV).transpose(1, 2)
+    o, idx, valid, scores, sel = swv.ops._dsa_forward(q, k, v, qi, ki, w, K, out_dtype=o_dtype)
+    got = swv.ops.dsa_module_bwd(d_out, q, k, v, o, qi, ki, w, idx, valid, scores, sel[0])
+    swv.check_status(DEV)
+    c = lambda x: x.detach().float().cpu()
+    dw_ref = torch.zeros(IH)
+    for b in range(B):
+        rw = c(scores)[b] * c(valid)[b]
+        rq, rk, rv, rrw = O.dsa_attention_bwd(c(d_out)[b], c(q)[b], c(k)[b], c(v)[b], c(o)[b], idx[b].cpu(), c(valid)[b], rw)
+        rqi, rki, rdw = O.indexer_bwd(rrw * c(valid)[b], c(qi)[b], c(ki)[b], c(w), idx[b].cpu(), c(valid)[b])
+        for x, r in zip(got, (rq, rk, rv, rqi, rki)):
+            assert _close(x[b], r)
+        dw_ref += rdw
+    assert _close(got[5], dw_ref, rel=1e-3)
