@@ -213,7 +213,7 @@ int swv_dsa_attn_bwd(const void* d_out, const int64_t d_out_strides[4], const vo
  * (B,Tq,top_k) and all gradients fp32 contiguous; ID <= 64; top_k <= 65535; B*Tq*top_k < 2^32.
  * `workspace`: swv_dsa_module_bwd_bytes() bytes, 256-byte aligned.
  */
-int swv_dsa_module_bwd_bytes(int B, int H, int Tq, int Tk, size_t* bytes);
+int swv_dsa_module_bwd_bytes(int B, int H, int Tq, int Tk, int top_k, size_t* bytes);
 int swv_dsa_module_bwd(const void* d_out, const int64_t d_out_strides[4], const void* q, const int64_t q_strides[4],
                        const void* k, const int64_t k_strides[4], const void* v, const int64_t v_strides[4],
                        const void* o, const int64_t o_strides[4], int o_dtype, const void* q_idx,

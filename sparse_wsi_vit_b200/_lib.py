@@ -80,7 +80,7 @@ def _load():
     lib.swv_dsa_indexer_bwd.argtypes = [
         c_void_p, i64p, c_void_p, i64p, c_void_p, i64p, c_int, c_void_p, c_void_p, i64p, c_void_p, i64p, c_void_p,
         c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
-    lib.swv_dsa_module_bwd_bytes.argtypes = [c_int, c_int, c_int, c_int, POINTER(c_size_t)]
+    lib.swv_dsa_module_bwd_bytes.argtypes = [c_int, c_int, c_int, c_int, c_int, POINTER(c_size_t)]
     lib.swv_dsa_module_bwd.argtypes = (
         [c_void_p, i64p] * 5 + [c_int] + [c_void_p, i64p] * 2 + [c_int] + [c_void_p] * 12 + [c_int] * 8 +
         [c_void_p, c_size_t, c_void_p, c_void_p])

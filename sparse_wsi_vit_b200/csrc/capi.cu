@@ -58,7 +58,7 @@ int dsa_attn_bwd_impl(const void* d_out, const int64_t* dos, const void* q, cons
                       const int64_t* vls, const float* rw, const int64_t* rs, float* dq, float* dk, float* dv,
                       float* drw, int B, int H, int Tq, int Tk, int D, int top_k, int* status, cudaStream_t st,
                       const int* run_if);
-int dsa_module_bwd_bytes_impl(int B, int H, int Tq, int Tk, size_t* bytes);
+int dsa_module_bwd_bytes_impl(int B, int H, int Tq, int Tk, int top_k, size_t* bytes);
 int dsa_module_bwd_impl(const void* d_out, const int64_t* dos, const void* q, const int64_t* qs, const void* k,
                         const int64_t* ks, const void* v, const int64_t* vs, const void* o, const int64_t* os,
                         int o_dtype, const void* q_idx, const int64_t* qis, const void* k_idx, const int64_t* kis,
@@ -162,8 +162,8 @@ int swv_dsa_attn_bwd(const void* d_out, const int64_t d_out_strides[4], const vo
                                 Tq, Tk, D, top_k, status, static_cast<cudaStream_t>(stream), nullptr);
 }
 
-int swv_dsa_module_bwd_bytes(int B, int H, int Tq, int Tk, size_t* bytes) {
-  return swv::dsa_module_bwd_bytes_impl(B, H, Tq, Tk, bytes);
+int swv_dsa_module_bwd_bytes(int B, int H, int Tq, int Tk, int top_k, size_t* bytes) {
+  return swv::dsa_module_bwd_bytes_impl(B, H, Tq, Tk, top_k, bytes);
 }
 
 int swv_dsa_module_bwd(const void* d_out, const int64_t d_out_strides[4], const void* q, const int64_t q_strides[4],

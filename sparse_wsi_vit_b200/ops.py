@@ -416,7 +416,7 @@ def dsa_module_bwd(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores, mask)
     dq, dk, dv, drw = f32(B, H, Tq, D), f32(B, H, Tk, D), f32(B, H, Tk, D), f32(B, Tq, top_k)
     dqi, dki, dw = f32(B, Tq, IH, ID), f32(B, Tk, IH, ID), f32(IH)
     nws = ctypes.c_size_t()
-    check(lib.swv_dsa_module_bwd_bytes(B, H, Tq, Tk, ctypes.byref(nws)), "swv_dsa_module_bwd_bytes")
+    check(lib.swv_dsa_module_bwd_bytes(B, H, Tq, Tk, top_k, ctypes.byref(nws)), "swv_dsa_module_bwd_bytes")
     ws = torch.empty(nws.value, dtype=torch.uint8, device=dev)
     rc = lib.swv_dsa_module_bwd(
         d_out.data_ptr(), strides(d_out), q.data_ptr(), strides(q), k.data_ptr(), strides(k), v.data_ptr(), strides(v),
