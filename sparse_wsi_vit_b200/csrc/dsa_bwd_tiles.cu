@@ -9,23 +9,29 @@
 //   drw_ij = sum_heads g_ij   dq_idx = W sum_j drw_ij k_idx_j   dk_idx = W sum_i drw_ij q_idx_i
 //
 // Three sweeps over 128 x 64 tiles of (lane side) x (streamed side), one kernel:
-//   kStats : lanes = queries, keys streamed: exact row maximum and l in fp32 -> lse_i = m_i + log2 max(l_i, 1e-6)
-//   kDkv   : lanes = keys, queries streamed: dV, dK in TMEM accumulators; every head's g_ij stored in list
-//            order (the slot of a member is its rank in the row's bitmask), summed over the heads afterwards
-//            (reductions straight into drw took 6.3 ms instead of 4.9 ms at 16384 tokens, 8 heads)
-//   kDq    : lanes = queries, keys streamed: dQ in a TMEM accumulator
+//   kStats : lanes = queries, keys streamed: exact row maximum m_i and 1 / max(l_i, 1e-6) in fp32 (kept apart:
+//            one log-sum-exp of both would round by 2^-24 of its own size, a factor common to the whole row)
+//   kDkv   : lanes = keys, queries streamed: dV, dK; every head's g_ij stored in list order (the slot of a
+//            member is its rank in the row's bitmask), summed over the heads afterwards
+//   kDq    : lanes = queries, keys streamed: dQ
 // Every tile's logits S, routing weights R (TF32, from the collapsed indexer vectors: the forward's own
-// products) and dP = dO V^T come from tcgen05 products into one of two TMEM buffers; eight warps turn
+// products) and dP = dO V^T come from tcgen05 products into one of two TMEM buffers; sixteen warps turn
 // them into P and dS, which go back into the very columns they came from, as the A operand (TMEM) of the
 // gradient products.  P and dS are fp32 values: each is split into THREE bf16 terms (24 bits) that are
-// multiplied one after the other, so no product sees fewer bits than the CUDA-core form.  q, k, v are
+// multiplied one after the other, so no product sees fewer bits than the CUDA-core form.  The tensor cores
+// truncate at every accumulation step, always towards zero (2^-27 of the result per step, 9e-6 after the
+// 1128 steps of 6009 keys), so an accumulator holds ONE tile's products: the warps add it to fp32 registers
+// (round to nearest) before they hand over the next tile.  q, k, v are
 // bf16; dO must be exact in bf16 as well (it is whenever the next layer ran in bf16) -- where it is not,
 // these kernels return at once and the list kernel runs.
 //
-// Bound: the tensor pipe.  An M128 x N64 x K16 instruction takes ~60 cycles, so a 128 x 128 tile of one
-// head costs 128 (kDkv), 80 (kDq) and 24 (kStats) of them; exponentials and splits run beside them.
-// The list kernels move 3 rows and reduce 2 per selected pair (43.8 ms at 16384 tokens, 8 heads,
-// top-2048); at one key in 8 the tiles do 8 times the kept products and are still far ahead.
+// Bound: kDkv by the instructions of the sixteen warps (63 % of the issue slots), kStats and kDq by the chain
+// products -> terms -> gradient products of two buffers, at 60-100 cycles per M128 x N64 instruction (40 per
+// tile and head in kDkv, 28 in kDq, 12 in kStats).  16384 tokens, 8 heads, top-2048: kStats 1.6, kDkv 4.9, kDq
+// 3.2 ms; kDkv took 5.8 ms with eight warps, a branch around the list store, and a block barrier per tile for
+// the column data, while the accumulators still ran over the whole row.
+// The list kernels move 3 rows and reduce 2 per selected pair (43.8 ms on the same input); at one key in 8
+// the tiles do 8 times the kept products and are still far ahead.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -50,16 +56,16 @@ constexpr int kOffStage = 2 * kLBytes + kLRBytes;
 constexpr int kStageB = 2 * kSBytes + kSRBytes;
 constexpr int kOffCols = kOffStage + kBwdStages * kStageB;
 
-// per streamed query (kDkv), double-buffered: stabiliser, D, membership words and list positions
+// per streamed query (kDkv), double-buffered
 struct BwdCols {
-  float lse[kNW], di[kNW];
-  uint32_t word[4][kNW], base[4][kNW];
+  float4 f[kNW];                        // {row maximum, 1 / l, D, -}
+  uint2 mem[4][kNW];                    // per 32 keys: {membership word, list position of its first member}
 };
 struct BwdCtl {
   uint64_t l_full, full[kBwdStages], empty[kBwdStages];
-  uint64_t in_full[2], p_ready[2], acc_done, acc_final;   // acc_done: per tile (issuer); acc_final: once
+  uint64_t in_full[2], p_ready[2], acc_done;
   uint32_t tmem_base, abort_flag;
-  float xm[kTile][2], xl[kTile][2], xe[kTile][2];
+  float xm[4][kTile], xl[4][kTile], xe[4][kTile];
 };
 constexpr int kOffBwdCtl = kOffCols + 2 * static_cast<int>(sizeof(BwdCols));
 constexpr size_t kBwdSmem = 1024 + kOffBwdCtl + sizeof(BwdCtl) + 64;
@@ -71,7 +77,7 @@ struct BwdTileParams {
   const uint32_t* maskbits;
   const uint16_t* off;      // [B][nKT + 1][Tq] first list slot of row i with a key in tile kt or later
   const float* di;          // (B,H,Tq)
-  float* lse;               // (B,H,Tq): log2 domain
+  float *rmax, *linv;       // (B,H,Tq): row maximum of the members' logits (log2 domain), 1 / max(l, 1e-6)
   float *dq, *dk, *dv;
   float* gh;                // [H][B*Tq*top_k] the heads' g in list order
   int r_steps;              // 8-channel steps of the routing-weight product (the rest of the 64 channels is zero)
@@ -80,19 +86,30 @@ struct BwdTileParams {
   int* status;
 };
 
-// a pair of fp32 values as three bf16 pairs whose sum is the pair
+// A pair of fp32 values as three bf16 pairs whose sum is the pair: each term takes the next 8 of the 24
+// bits as they are (byte permutes; rounded conversions cost two issue slots each and gain nothing here).
 __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  hi = pack_bf16x2(a, b);
-  a -= __uint_as_float(hi << 16);
-  b -= __uint_as_float(hi & 0xffff0000u);
-  mid = pack_bf16x2(a, b);
-  a -= __uint_as_float(mid << 16);
-  b -= __uint_as_float(mid & 0xffff0000u);
-  lo = pack_bf16x2(a, b);
+  hi = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+  a -= __uint_as_float(__float_as_uint(a) & 0xffff0000u);
+  b -= __uint_as_float(__float_as_uint(b) & 0xffff0000u);
+  mid = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+  a -= __uint_as_float(__float_as_uint(a) & 0xffff0000u);
+  b -= __uint_as_float(__float_as_uint(b) & 0xffff0000u);
+  lo = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 
+// *p = x where `on`: one predicated store (a branch around it costs the warp its convergence bookkeeping)
+__device__ __forceinline__ void st_global_if(float* p, float x, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.global.f32 [%0], %1;\n\t}" ::"l"(p), "f"(x),
+               "r"(static_cast<uint32_t>(on))
+               : "memory");
+}
+
+constexpr int kBwdEpi = 16;             // warps that turn a tile's products into its terms, 16 columns each
+constexpr int bwd_threads(int mode) { return 64 + 32 * kBwdEpi + (mode == kDkv ? 64 : 0); }
+
 template <int MODE>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(bwd_threads(MODE), 1)
     dsa_bwd_tiles_kernel(const __grid_constant__ CUtensorMap tm_l1, const __grid_constant__ CUtensorMap tm_l2,
                          const __grid_constant__ CUtensorMap tm_lr, const __grid_constant__ CUtensorMap tm_s1,
                          const __grid_constant__ CUtensorMap tm_s2, const __grid_constant__ CUtensorMap tm_sr,
@@ -121,11 +138,10 @@ __global__ void __launch_bounds__(320, 1)
       mbar_init(&ctl->empty[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&ctl->in_full[s], 1);
-      mbar_init(&ctl->p_ready[s], 8);
+      mbar_init(&ctl->in_full[s], MODE == kDkv ? 3 : 1);    // the products and (kDkv) two warps of column data
+      mbar_init(&ctl->p_ready[s], kBwdEpi);
     }
     mbar_init(&ctl->acc_done, 1);
-    mbar_init(&ctl->acc_final, 1);
     ctl->abort_flag = 0;
     fence_barrier_init();
   }
@@ -181,9 +197,9 @@ __global__ void __launch_bounds__(320, 1)
         const uint64_t d1 = smem_desc_sw128(st), d2 = smem_desc_sw128(st + kSBytes);
 #pragma unroll
         for (int ks = 0; ks < kNW / 16; ++ks) {
-          // where the eight warps left the terms of these 16 streamed rows (see the epilogue)
+          // where the warps left the terms of these 16 streamed rows (see the epilogue)
           const uint32_t cs = buf + 16 * ks, cr = cs + 64, cp = cs + 128;
-          const bool acc = t > 0 || ks > 0;
+          const bool acc = ks > 0;
           if (MODE == kDkv) {
             umma_f16_ts(tmem_base + kColAcc, cs, d2 + ks * 128, kIdescAcc, acc);
             umma_f16_ts(tmem_base + kColAcc, cs + 8, d2 + ks * 128, kIdescAcc, 1);
@@ -232,13 +248,49 @@ __global__ void __launch_bounds__(320, 1)
         umma_commit(&ctl->in_full[t & 1]);
         if (MODE != kStats && t >= 1) ok = accumulate(t - 1);
       }
-      if (MODE != kStats && ok && accumulate(nS - 1)) umma_commit(&ctl->acc_final);
+      if (MODE != kStats && ok) accumulate(nS - 1);
+    }
+  } else if (MODE == kDkv && warp >= 2 + kBwdEpi) {
+    // ------------------------- two warps: the column data of the tiles, one streamed query per thread
+    const int cc = (warp & 1) * 32 + lane;
+    const int64_t bh = static_cast<int64_t>(b) * p.H + h;
+    for (int t = 0; t < nS; ++t) {
+      const int i = t * kNW + cc;
+      uint4 mw = make_uint4(0u, 0u, 0u, 0u);
+      uint32_t pos = 0;
+      float4 f = make_float4(__int_as_float(0x7f800000), 0.f, 0.f, 0.f);   // rows behind the end: sm = 2^-inf = 0
+      if (i < p.Tq) {
+        mw = __ldg(reinterpret_cast<const uint4*>(p.maskbits) +
+                   ((static_cast<int64_t>(b) * p.nQT + (i >> 7)) * p.nKT + lt) * kTile + (i & 127));
+        pos = (static_cast<uint32_t>(b) * p.Tq + i) * p.top_k +
+              __ldg(p.off + (static_cast<int64_t>(b) * (p.nKT + 1) + lt) * p.Tq + i);
+        f.x = __ldg(p.rmax + bh * p.Tq + i);
+        f.y = __ldg(p.linv + bh * p.Tq + i);
+        f.z = __ldg(p.di + bh * p.Tq + i);
+      }
+      // tile t - 2 has been turned into its terms: its column data are no longer read
+      bool ok = t < 2 || mbar_wait_bounded(&ctl->p_ready[t & 1], ((t >> 1) & 1) ^ 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        record_status(p.status, kDevWaitPReady);
+        break;
+      }
+      BwdCols& c = cols[t & 1];
+      c.f[cc] = f;
+      const uint32_t w[4] = {mw.x, mw.y, mw.z, mw.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        c.mem[q][cc] = make_uint2(w[q], pos);
+        pos += __popc(w[q]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->in_full[t & 1]);
     }
   } else {
-    // ------------------------------------------------- eight warps: (lane quarter, half of the columns)
-    const int ct = threadIdx.x - 64;
+    // ------------------------------------------ sixteen warps: (lane quarter, 16 of the 64 columns)
     const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;
+    const int grp = (warp - 2) >> 2;
+    const int c0 = grp * 16;                              // streamed rows c0 .. c0 + 15 = one k-step of the products
     const int row = quarter * 32 + lane;
     const int lrow = lt * kTile + row;                    // query (kStats, kDq) or key (kDkv)
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
@@ -246,114 +298,37 @@ __global__ void __launch_bounds__(320, 1)
     const float c2 = p.c2;
     const int64_t bh = static_cast<int64_t>(b) * p.H + h;
     const bool row_ok = lrow < (MODE == kDkv ? p.Tk : p.Tq);
+    constexpr int kAcc = MODE == kDkv ? 32 : 16;          // this warp's columns of the accumulators
+    const uint32_t acc_col = tmem_base + lane_off + kColAcc + grp * kAcc;
+    float acc[kAcc];
+#pragma unroll
+    for (int i = 0; i < kAcc; ++i) acc[i] = 0.f;
     bool ok = true;
+    // adds tile t's products; they are complete before the warps hand over tile t + 1
+    auto flush = [&](int t) {
+      if (!mbar_wait_bounded(&ctl->acc_done, t & 1, abort_flag)) {
+        record_status(p.status, kDevWaitPvDone);
+        ok = false;
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) return;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < kAcc; c += 16) {
+        uint32_t x[16];
+        tmem_ld16(acc_col + c, x);
+        tc_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[c + i] += __uint_as_float(x[i]);
+      }
+    };
 
     if constexpr (MODE == kDkv) {
-      // the column data of tile t: this thread's (quarter cq, query cc)
-      const int cq = ct >> 6, cc = ct & 63;
-      uint4 mw;
-      uint32_t off0 = 0;
-      float x0 = 0.f;
-      auto fetch = [&](int t) {
-        const int i = t * kNW + cc;
-        mw = make_uint4(0u, 0u, 0u, 0u);
-        off0 = 0;
-        x0 = cq == 0 ? -ninf : 0.f;                       // rows behind the end: sm = 2^-inf = 0
-        if (t < nS && i < p.Tq) {
-          mw = __ldg(reinterpret_cast<const uint4*>(p.maskbits) +
-                     ((static_cast<int64_t>(b) * p.nQT + (i >> 7)) * p.nKT + lt) * kTile + (i & 127));
-          off0 = __ldg(p.off + (static_cast<int64_t>(b) * (p.nKT + 1) + lt) * p.Tq + i);
-          if (cq < 2) x0 = __ldg((cq == 0 ? p.lse : p.di) + bh * p.Tq + i);
-        }
-      };
-      auto put = [&](int t) {
-        BwdCols& c = cols[t & 1];
-        const uint32_t w[4] = {mw.x, mw.y, mw.z, mw.w};
-        uint32_t mine = w[0], below = 0;
-#pragma unroll
-        for (int q = 1; q < 4; ++q) {
-          if (q <= cq) below += __popc(w[q - 1]);
-          if (q == cq) mine = w[q];
-        }
-        c.word[cq][cc] = mine;
-        c.base[cq][cc] = (static_cast<uint32_t>(b) * p.Tq + t * kNW + cc) * p.top_k + off0 + below;
-        if (cq == 0) c.lse[cc] = x0;
-        if (cq == 1) c.di[cc] = x0;
-      };
-      fetch(0);
-      put(0);
-      asm volatile("bar.sync 1, 256;" ::: "memory");
       const uint32_t lt_mask = (1u << lane) - 1u;
       float* gh = p.gh + static_cast<size_t>(h) * p.B * p.Tq * p.top_k;
       for (int t = 0; t < nS; ++t) {
         const BwdCols& c = cols[t & 1];
-        fetch(t + 1);
-        if (ok && !mbar_wait_bounded(&ctl->in_full[t & 1], (t >> 1) & 1, abort_flag)) {
-          record_status(p.status, kDevWaitAccFull);
-          ok = false;
-        }
-        ok = __all_sync(0xffffffffu, ok);
-        if (ok) {
-          tc_fence_after();
-          const uint32_t buf = tmem_base + lane_off + (t & 1) * kBufCols;
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int c0 = half * 32 + k * 16;            // streamed rows c0 .. c0 + 15 = one k-step of the products
-            uint32_t s[16], r[16], d[16];
-            tmem_ld16(buf + c0, s);
-            tmem_ld16(buf + 64 + c0, r);
-            tmem_ld16(buf + 128 + c0, d);
-            tc_wait_ld();
-            uint32_t pt[3][8], dt[3][8];
-#pragma unroll
-            for (int i = 0; i < 16; i += 2) {
-              float pv[2], dv[2];
-#pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const int j = c0 + i + e;
-                const uint32_t word = c.word[quarter][j];
-                const bool member = (word >> lane) & 1u;
-                const float sm = ex2_approx(fmaf(__uint_as_float(s[i + e]), c2, -c.lse[j]));
-                const float x = __uint_as_float(d[i + e]) - c.di[j];
-                if (member) gh[c.base[quarter][j] + __popc(word & lt_mask)] = sm * x;
-                // (selected as a product: sm of a pair that is not a member may be infinite)
-                pv[e] = member ? sm * fmaxf(__uint_as_float(r[i + e]), 0.f) : 0.f;
-                dv[e] = pv[e] * x;
-              }
-              split3(pv[0], pv[1], pt[0][i >> 1], pt[1][i >> 1], pt[2][i >> 1]);
-              split3(dv[0], dv[1], dt[0][i >> 1], dt[1][i >> 1], dt[2][i >> 1]);
-            }
-            tmem_st8(buf + c0, pt[0]);
-            tmem_st8(buf + c0 + 8, pt[1]);
-            tmem_st8(buf + 64 + c0, pt[2]);
-            tmem_st8(buf + 64 + c0 + 8, dt[0]);
-            tmem_st8(buf + 128 + c0, dt[1]);
-            tmem_st8(buf + 128 + c0 + 8, dt[2]);
-          }
-          tc_wait_st();
-          tc_fence_before();
-        }
-        __syncwarp();
-        if (ok && lane == 0) mbar_arrive(&ctl->p_ready[t & 1]);
-        put(t + 1);
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-      }
-    } else {
-      float neg_lse = ninf, di = 0.f;                     // rows behind the end: sm = 0
-      if (MODE == kDq && row_ok) {
-        neg_lse = -__ldg(p.lse + bh * p.Tq + lrow);
-        di = __ldg(p.di + bh * p.Tq + lrow);
-      }
-      float m = ninf, mx = ninf, l = 0.f;                 // kStats: stabiliser, exact maximum, sum
-      const uint32_t* mrow = p.maskbits + ((static_cast<int64_t>(b) * p.nQT + lt) * p.nKT * kTile + row) * 4 + half;
-      auto fetch = [&](int t) -> uint32_t {
-        return (t < nS && row_ok) ? __ldg(mrow + static_cast<int64_t>(t >> 1) * (kTile * 4) + (t & 1) * 2) : 0u;
-      };
-      uint32_t next = fetch(0);
-      for (int t = 0; t < nS; ++t) {
-        const uint32_t word = next;
-        next = fetch(t + 1);
-        if (ok && !mbar_wait_bounded(&ctl->in_full[t & 1], (t >> 1) & 1, abort_flag)) {
+        if (!mbar_wait_bounded(&ctl->in_full[t & 1], (t >> 1) & 1, abort_flag)) {
           record_status(p.status, kDevWaitAccFull);
           ok = false;
         }
@@ -361,18 +336,78 @@ __global__ void __launch_bounds__(320, 1)
         if (!ok) break;
         tc_fence_after();
         const uint32_t buf = tmem_base + lane_off + (t & 1) * kBufCols;
-        const int c0 = half * 32;
+        uint32_t s[16], r[16], d[16];
+        tmem_ld16(buf + c0, s);
+        tmem_ld16(buf + 64 + c0, r);
+        tmem_ld16(buf + 128 + c0, d);
+        tc_wait_ld();
+        uint32_t pt[3][8], dt[3][8];
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          float pv[2], dv[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float4 f = c.f[c0 + i + e];
+            const uint2 mem = c.mem[quarter][c0 + i + e];
+            const bool member = (mem.x >> lane) & 1u;
+            const float sm = ex2_approx(fmaf(__uint_as_float(s[i + e]), c2, -f.x)) * f.y;
+            const float x = __uint_as_float(d[i + e]) - f.z;
+            st_global_if(gh + (mem.y + __popc(mem.x & lt_mask)), sm * x, member);
+            // (selected as a product: sm of a pair that is not a member may be infinite)
+            pv[e] = member ? sm * fmaxf(__uint_as_float(r[i + e]), 0.f) : 0.f;
+            dv[e] = pv[e] * x;
+          }
+          split3(pv[0], pv[1], pt[0][i >> 1], pt[1][i >> 1], pt[2][i >> 1]);
+          split3(dv[0], dv[1], dt[0][i >> 1], dt[1][i >> 1], dt[2][i >> 1]);
+        }
+        tmem_st8(buf + c0, pt[0]);
+        tmem_st8(buf + c0 + 8, pt[1]);
+        tmem_st8(buf + 64 + c0, pt[2]);
+        tmem_st8(buf + 64 + c0 + 8, dt[0]);
+        tmem_st8(buf + 128 + c0, dt[1]);
+        tmem_st8(buf + 128 + c0 + 8, dt[2]);
+        if (t > 0) flush(t - 1);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (ok && lane == 0) mbar_arrive(&ctl->p_ready[t & 1]);
+      }
+    } else {
+      float neg_m = ninf, di = 0.f;                       // rows behind the end: sm = 0
+      if (MODE == kDq && row_ok) {
+        neg_m = -__ldg(p.rmax + bh * p.Tq + lrow);
+        di = __ldg(p.di + bh * p.Tq + lrow);
+      }
+      float m = ninf, mx = ninf, l = 0.f;                 // kStats: stabiliser, exact maximum, sum
+      const uint32_t* mrow =
+          p.maskbits + ((static_cast<int64_t>(b) * p.nQT + lt) * p.nKT * kTile + row) * 4 + (grp >> 1);
+      auto fetch = [&](int t) -> uint32_t {
+        return (t < nS && row_ok) ? __ldg(mrow + static_cast<int64_t>(t >> 1) * (kTile * 4) + (t & 1) * 2) >> ((grp & 1) * 16)
+                                  : 0u;
+      };
+      uint32_t next = fetch(0);
+      for (int t = 0; t < nS; ++t) {
+        const uint32_t word = next;
+        next = fetch(t + 1);
+        if (!mbar_wait_bounded(&ctl->in_full[t & 1], (t >> 1) & 1, abort_flag)) {
+          record_status(p.status, kDevWaitAccFull);
+          ok = false;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t buf = tmem_base + lane_off + (t & 1) * kBufCols;
+        uint32_t s[16], r[16];
+        tmem_ld16(buf + c0, s);
+        tmem_ld16(buf + 64 + c0, r);
         if constexpr (MODE == kStats) {
-          uint32_t s[32], r[32];
-          tmem_ld32(buf + c0, s);
-          tmem_ld32(buf + 64 + c0, r);
           tc_wait_ld();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl->p_ready[t & 1]);
           float mt = ninf;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
+          for (int i = 0; i < 16; ++i) {
             s[i] = ((word >> i) & 1u) ? __float_as_uint(__uint_as_float(s[i]) * c2) : __float_as_uint(ninf);
             mt = fmaxf(mt, __uint_as_float(s[i]));
           }
@@ -381,84 +416,73 @@ __global__ void __launch_bounds__(320, 1)
             l *= ex2_approx(m - mt);
             m = mt;
           }
-          const float neg_m = m == ninf ? 0.f : -m;
+          const float sub = m == ninf ? 0.f : -m;
           float l1 = 0.f;
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            l = fmaf(ex2_approx(__uint_as_float(s[i]) + neg_m), fmaxf(__uint_as_float(r[i]), 0.f), l);
-            l1 = fmaf(ex2_approx(__uint_as_float(s[i + 1]) + neg_m), fmaxf(__uint_as_float(r[i + 1]), 0.f), l1);
+          for (int i = 0; i < 16; i += 2) {
+            l = fmaf(ex2_approx(__uint_as_float(s[i]) + sub), fmaxf(__uint_as_float(r[i]), 0.f), l);
+            l1 = fmaf(ex2_approx(__uint_as_float(s[i + 1]) + sub), fmaxf(__uint_as_float(r[i + 1]), 0.f), l1);
           }
           l += l1;
         } else {
+          uint32_t d[16];
+          tmem_ld16(buf + 128 + c0, d);
+          tc_wait_ld();
+          uint32_t dt[3][8];
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int cc = c0 + k * 16;
-            uint32_t s[16], r[16], d[16];
-            tmem_ld16(buf + cc, s);
-            tmem_ld16(buf + 64 + cc, r);
-            tmem_ld16(buf + 128 + cc, d);
-            tc_wait_ld();
-            uint32_t dt[3][8];
+          for (int i = 0; i < 16; i += 2) {
+            float dv[2];
 #pragma unroll
-            for (int i = 0; i < 16; i += 2) {
-              float dv[2];
-#pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const float sm = ex2_approx(fmaf(__uint_as_float(s[i + e]), c2, neg_lse));
-                const float pv = ((word >> (k * 16 + i + e)) & 1u) ? sm * fmaxf(__uint_as_float(r[i + e]), 0.f) : 0.f;
-                dv[e] = pv * (__uint_as_float(d[i + e]) - di);
-              }
-              split3(dv[0], dv[1], dt[0][i >> 1], dt[1][i >> 1], dt[2][i >> 1]);
+            for (int e = 0; e < 2; ++e) {
+              const float sm = ex2_approx(fmaf(__uint_as_float(s[i + e]), c2, neg_m));   // (1 / l: with the output)
+              const float pv = ((word >> (i + e)) & 1u) ? sm * fmaxf(__uint_as_float(r[i + e]), 0.f) : 0.f;
+              dv[e] = pv * (__uint_as_float(d[i + e]) - di);
             }
-            tmem_st8(buf + 64 + cc + 8, dt[0]);
-            tmem_st8(buf + 128 + cc, dt[1]);
-            tmem_st8(buf + 128 + cc + 8, dt[2]);
+            split3(dv[0], dv[1], dt[0][i >> 1], dt[1][i >> 1], dt[2][i >> 1]);
           }
+          tmem_st8(buf + 64 + c0 + 8, dt[0]);
+          tmem_st8(buf + 128 + c0, dt[1]);
+          tmem_st8(buf + 128 + c0 + 8, dt[2]);
+          if (t > 0) flush(t - 1);
           tc_wait_st();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&ctl->p_ready[t & 1]);
+          if (ok && lane == 0) mbar_arrive(&ctl->p_ready[t & 1]);
         }
       }
       if constexpr (MODE == kStats) {
-        ctl->xm[row][half] = m;
-        ctl->xe[row][half] = mx;
-        ctl->xl[row][half] = l;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (half == 0 && row_ok && ok) {
-          const float mm = fmaxf(ctl->xe[row][0], ctl->xe[row][1]);
-          float lt_ = 0.f;
+        ctl->xm[grp][row] = m;
+        ctl->xe[grp][row] = mx;
+        ctl->xl[grp][row] = l;
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+        if (grp == 0 && row_ok && ok) {
+          const float mm = fmaxf(fmaxf(ctl->xe[0][row], ctl->xe[1][row]), fmaxf(ctl->xe[2][row], ctl->xe[3][row]));
+          float lsum = 0.f;
 #pragma unroll
-          for (int q = 0; q < 2; ++q)
-            if (ctl->xm[row][q] != ninf) lt_ = fmaf(ctl->xl[row][q], exp2f(ctl->xm[row][q] - mm), lt_);
+          for (int q = 0; q < 4; ++q)
+            if (ctl->xm[q][row] != ninf) lsum = fmaf(ctl->xl[q][row], exp2f(ctl->xm[q][row] - mm), lsum);
           // a row without members: +inf, all its weights are zero
-          p.lse[bh * p.Tq + lrow] = mm == ninf ? -ninf : mm + log2f(fmaxf(lt_, 1e-6f));
+          p.rmax[bh * p.Tq + lrow] = mm == ninf ? -ninf : mm;
+          p.linv[bh * p.Tq + lrow] = 1.f / fmaxf(lsum, 1e-6f);
         }
       }
     }
 
     if constexpr (MODE != kStats) {
-      if (ok && !mbar_wait_bounded(&ctl->acc_final, 0, abort_flag)) {
-        record_status(p.status, kDevWaitPvDone);
-        ok = false;
-      }
-      ok = __all_sync(0xffffffffu, ok);
-      if (ok) {
-        tc_fence_after();
-#pragma unroll
-        for (int a = 0; a < (MODE == kDkv ? 2 : 1); ++a) {
-          uint32_t o[32];
-          tmem_ld32(tmem_base + lane_off + kColAcc + a * 64 + half * 32, o);
-          tc_wait_ld();
-          if (!row_ok) continue;
-          float* dst = (MODE == kDq ? p.dq : (a == 0 ? p.dv : p.dk)) +
-                       (bh * (MODE == kDkv ? p.Tk : p.Tq) + lrow) * kHd + half * 32;
-          const float f = MODE == kDkv && a == 0 ? 1.f : p.scale;
-#pragma unroll
-          for (int i = 0; i < 32; i += 4)
-            *reinterpret_cast<float4*>(dst + i) = make_float4(__uint_as_float(o[i]) * f, __uint_as_float(o[i + 1]) * f,
-                                                              __uint_as_float(o[i + 2]) * f, __uint_as_float(o[i + 3]) * f);
+      if (ok) flush(nS - 1);
+      if (ok && row_ok) {
+        float* dst;
+        float f = p.scale;
+        if constexpr (MODE == kDkv) {
+          dst = (grp < 2 ? p.dv : p.dk) + (bh * p.Tk + lrow) * kHd + (grp & 1) * kAcc;
+          if (grp < 2) f = 1.f;
+        } else {
+          dst = p.dq + (bh * p.Tq + lrow) * kHd + grp * kAcc;
+          f *= __ldg(p.linv + bh * p.Tq + lrow);
         }
+#pragma unroll
+        for (int i = 0; i < kAcc; i += 4)
+          *reinterpret_cast<float4*>(dst + i) = make_float4(acc[i] * f, acc[i + 1] * f, acc[i + 2] * f, acc[i + 3] * f);
       }
     }
   }
@@ -663,7 +687,7 @@ __global__ void __launch_bounds__(320, 1)
 #pragma unroll
           for (int ks = 0; ks < kTile / 16; ++ks)
             umma_f16_ss(tmem_base, da + (ks >> 2) * (kTile * 128 / 16) + (ks & 3) * 2, db + ks * 128, kIdesc,
-                        t > 0 || term > 0 || ks > 0);
+                        term > 0 || ks > 0);
         }
         umma_commit(&ctl->empty[s]);
         umma_commit(&ctl->done);
@@ -705,12 +729,33 @@ __global__ void __launch_bounds__(320, 1)
       asm volatile("st.shared.u16 [%0], %1;" ::"r"(a + kTermBytes), "h"(static_cast<uint16_t>(mid)) : "memory");
       asm volatile("st.shared.u16 [%0], %1;" ::"r"(a + 2 * kTermBytes), "h"(static_cast<uint16_t>(lo)) : "memory");
     };
-    fetch(0);
-    for (int t = 0; t < nS; ++t) {
-      if (t > 0 && ok && !mbar_wait_bounded(&ctl->done, (t - 1) & 1, abort_flag)) {
+    // this thread's part of the sums, in registers (every accumulation in tensor memory truncates, see above)
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    const uint32_t acc_col = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (E / 2);
+    float acc[E / 2];
+#pragma unroll
+    for (int i = 0; i < E / 2; ++i) acc[i] = 0.f;
+    auto flush = [&](int t) {
+      if (!mbar_wait_bounded(&ctl->done, t & 1, abort_flag)) {
         record_status(p.status, kDevWaitPvDone);
         ok = false;
       }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) return;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < E / 2; c += 16) {
+        uint32_t x[16];
+        tmem_ld16(acc_col + c, x);
+        tc_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[c + i] += __uint_as_float(x[i]);
+      }
+      tc_fence_before();
+    };
+    fetch(0);
+    for (int t = 0; t < nS; ++t) {
+      if (t > 0 && ok) flush(t - 1);
 #pragma unroll
       for (int i = 0; i < 3 * kTermBytes / 16 / 256; ++i) sts128(g_addr + (i * 256 + ct) * 16, 0u, 0u, 0u, 0u);
       asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -724,27 +769,17 @@ __global__ void __launch_bounds__(320, 1)
       if (ok && lane == 0) mbar_arrive(&ctl->g_full);
       fetch(t + 1);
     }
-    if (ok && !mbar_wait_bounded(&ctl->done, (nS - 1) & 1, abort_flag)) {
-      record_status(p.status, kDevWaitPvDone);
-      ok = false;
-    }
-    ok = __all_sync(0xffffffffu, ok);
+    if (ok) flush(nS - 1);
     if (ok) {
-      tc_fence_after();
-      const int quarter = warp & 3, half = (warp - 2) >> 2;
       const int lrow = lt * kTile + quarter * 32 + lane;
       const int T = MODE == kLaneQ ? p.Tq : p.Tk;
       const bool row_ok = lrow < T;
-      const uint32_t acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (E / 2);
       float* dst = p.dx + (static_cast<int64_t>(b) * T + lrow) * E + half * (E / 2);
       const __nv_bfloat16* qrow = p.q_idx + b * p.qsb + lrow * p.qst + half * (E / 2);
       float dw = 0.f;
       int head = half * (E / 2) / p.ID;
-#pragma unroll 1
+#pragma unroll
       for (int c = 0; c < E / 2; c += 16) {
-        uint32_t o[16];
-        tmem_ld16(acc + c, o);
-        tc_wait_ld();
         uint4 qv[2];
         if (MODE == kLaneQ && row_ok) {
           qv[0] = __ldg(reinterpret_cast<const uint4*>(qrow + c));
@@ -764,7 +799,7 @@ __global__ void __launch_bounds__(320, 1)
             dw = 0.f;
             head = hh;
           }
-          x[i] = __uint_as_float(o[i]);
+          x[i] = acc[c + i];
           if (MODE == kLaneQ) dw = fmaf(x[i], __uint_as_float((i & 1) ? qw[i >> 1] & 0xffff0000u : qw[i >> 1] << 16), dw);
           x[i] *= __ldg(p.w + hh);
         }
@@ -791,7 +826,7 @@ __global__ void __launch_bounds__(320, 1)
 
 size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 struct BwdLayout {
-  size_t do16, di, lse, wq, wk, off, flag, gh, total;
+  size_t do16, di, rmax, linv, wq, wk, off, flag, gh, total;
 };
 BwdLayout bwd_layout(int B, int H, int Tq, int Tk, int top_k) {
   BwdLayout L;
@@ -800,7 +835,8 @@ BwdLayout bwd_layout(int B, int H, int Tq, int Tk, int top_k) {
   size_t o = 0;
   L.do16 = o; o += up256(rows * kHd * 2);
   L.di = o; o += up256(rows * 4);
-  L.lse = o; o += up256(rows * 4);
+  L.rmax = o; o += up256(rows * 4);
+  L.linv = o; o += up256(rows * 4);
   L.wq = o; o += up256(static_cast<size_t>(B) * Tq * kIdxDim * 4);
   L.wk = o; o += up256(static_cast<size_t>(B) * Tk * kIdxDim * 4);
   L.off = o; o += up256(static_cast<size_t>(B) * (nKT + 1) * Tq * 2);
@@ -816,7 +852,7 @@ int launch_bwd(const CUtensorMap& l1, const CUtensorMap& l2, const CUtensorMap& 
   SWV_CUDA_OK(cudaFuncSetAttribute(dsa_bwd_tiles_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(kBwdSmem)));
   const unsigned grid = static_cast<unsigned>(p.B) * p.H * (MODE == kDkv ? p.nKT : p.nQT);
-  dsa_bwd_tiles_kernel<MODE><<<grid, 320, kBwdSmem, st>>>(l1, l2, lr, s1, s2, sr, p);
+  dsa_bwd_tiles_kernel<MODE><<<grid, bwd_threads(MODE), kBwdSmem, st>>>(l1, l2, lr, s1, s2, sr, p);
   SWV_CUDA_OK(cudaGetLastError());
   return SWV_OK;
 }
@@ -939,7 +975,7 @@ int dsa_module_bwd_impl(const void* d_out, const int64_t* dos, const void* q, co
   }
   BwdTileParams p;
   p.B = B; p.H = H; p.Tq = Tq; p.Tk = Tk; p.nQT = nQT; p.nKT = nKT; p.top_k = top_k;
-  p.maskbits = maskbits; p.off = off; p.di = di; p.lse = reinterpret_cast<float*>(ws + L.lse);
+  p.maskbits = maskbits; p.off = off; p.di = di; p.rmax = reinterpret_cast<float*>(ws + L.rmax); p.linv = reinterpret_cast<float*>(ws + L.linv);
   p.dq = dq; p.dk = dk; p.dv = dv; p.gh = reinterpret_cast<float*>(ws + L.gh);
   p.r_steps = (ID + 7) / 8;
   p.scale = 1.0f / sqrtf(static_cast<float>(D));

@@ -191,3 +191,33 @@ def test_tile_backward_vs_oracle(swv, B, T, H, IH, ID, K, o_dtype, exact):
             assert _close(x[b], r)
         dw_ref += rdw
     assert _close(got[5], dw_ref, rel=1e-3)
+
+
+def test_tile_backward_long_sums_keep_fp32(swv):
+    """Gradients of a few queries over a long key range (128 tiles of the sweep) against fp64: the sums must not
+    lose bits with their length.  Bound 2^-19 in the 2-norm: every factor is good to about 2^-22 (the
+    approximate exponential, the products' fp32 sums) and rounded sums of independent terms do not grow;
+    accumulating the whole row in the tensor cores (which truncate at every step) gave 9e-6."""
+    T, K, R = 8192, 512, 8
+    g = torch.Generator(device=DEV).manual_seed(5)
+    rnd = lambda *s, scale=1.0: (torch.randn(*s, generator=g, device=DEV) * scale).to(torch.bfloat16)
+    q, k, v = rnd(1, 1, T, 64, scale=0.125), rnd(1, 1, T, 64), rnd(1, 1, T, 64)
+    qi, ki = rnd(1, T, 4, 32, scale=32 ** -0.5), rnd(1, T, 4, 32, scale=32 ** -0.5)
+    w = torch.randn(4, generator=g, device=DEV)
+    d_out = torch.zeros(1, 1, T, 64, dtype=torch.bfloat16, device=DEV)
+    d_out[:, :, :R] = rnd(1, 1, R, 64)
+    o, idx, valid, scores, sel = swv.ops._dsa_forward(q, k, v, qi, ki, w, K)
+    got = swv.ops.dsa_module_bwd(d_out, q, k, v, o, qi, ki, w, idx, valid, scores, sel[0])
+    swv.check_status(DEV)
+    f = lambda x: x.double()
+    ii = idx[0, :R].long()
+    rw = f(scores[0, :R] * valid[0, :R])
+    kk, vv, dd = f(k[0, 0])[ii], f(v[0, 0])[ii], f(d_out[0, 0, :R])
+    e = torch.softmax(torch.einsum("nd,nkd->nk", f(q[0, 0, :R]), kk) / 8, dim=1)
+    sm = e / (e * rw).sum(1, keepdim=True)
+    drw = sm * (torch.einsum("nd,nkd->nk", dd, vv) - (dd * f(o[0, 0, :R])).sum(1, keepdim=True))
+    dq = torch.einsum("nk,nkd->nd", rw * drw, kk) / 8
+    dqi = torch.einsum("nk,nkhd->nhd", drw, f(ki[0])[ii]) * f(w)[None, :, None]
+    for name, x, r in (("dq", got[0][0, 0, :R], dq), ("dq_idx", got[3][0, :R], dqi)):
+        err = float((f(x) - r).norm() / r.norm())
+        assert err < 2.0 ** -19, (name, err)
