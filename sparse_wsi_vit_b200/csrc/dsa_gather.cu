@@ -9,6 +9,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace swv {
@@ -141,17 +143,18 @@ __global__ void __launch_bounds__(128) dsa_attn_gather_kernel(const GatherParams
   }
 }
 
-// ------------------------------------------------------- 16-bit fast path
-// bf16 / fp16 q, k, v with unit inner stride and 16-byte aligned rows, D in {32, 64, 128}.
+// ------------------------------------------------------- rows of 16-byte chunks
+// q, k, v with unit inner stride and 16-byte aligned rows, D in {32, 64, 128}.
 // One CTA per (batch, query) and up to eight heads, one warp per head: the row of idx / valid /
-// rw is read ONCE for all heads (256 slots at a time through shared memory).  D / 8 lanes share a
-// selected row, each reading one 16-byte chunk of the key row (mixed-precision FMAs: bf16 x bf16
-// products are exact in fp32; the partial dot products are added across the row's lanes) and then of
-// the value row (p split into two 16-bit halves so that the products stay exact to 2^-17, fp32
-// accumulators per lane, folded once at the end).  The running maximum is exact (the accumulators
+// rw is read ONCE for all heads (256 slots at a time through shared memory).  As many lanes as a row has
+// 16-byte chunks share a selected row, each reading one chunk of the key row (16-bit types: mixed-precision
+// FMAs, bf16 x bf16 products are exact in fp32; the partial dot products are added across the row's lanes)
+// and then of the value row (16-bit types: p split into two 16-bit halves so that the products stay exact
+// to 2^-17; fp32 accumulators per lane, folded once at the end).  The running maximum is exact (the accumulators
 // are rescaled whenever it rises, a handful of times per row).  Every selected row crosses the
-// L2 -> SM path once per head: 2 * top_k * D * 2 bytes per (query, head), one byte per FLOP -- the
-// bound of this operator.
+// L2 -> SM path once per head: 2 * top_k * D elements per (query, head), the bound of this operator.
+// fp32, 4099 tokens, 6 heads of 64, 512 keys each (6.4 GB of rows): 3.46 ms in the lane-per-row kernel
+// above, 1.74 ms here (3.7 TB/s).
 template <bool BF16>
 __device__ __forceinline__ void fma_mixed2(float& acc0, float& acc1, uint32_t a, uint32_t b) {
   if (BF16) {
@@ -187,14 +190,17 @@ __device__ __forceinline__ void split16(float x, uint32_t& hi2, uint32_t& lo2) {
 
 constexpr int kRowsSlots = 256;      // slots staged per round
 
-// D / 8 lanes share one row (a lane reads ONE 16-byte chunk of it: 8 channels), so a warp-level load
-// touches 32 * 16 / (2 D) rows = whole 128-byte lines instead of 32 different lines -- the per-lane
-// form of this kernel ran at 99 % of the L1 pipe's tag rate.  G = 256 / D rows per step.
-template <int D, bool BF16>
+// A lane reads ONE 16-byte chunk of a row, so a warp-level load touches whole 128-byte lines instead of
+// 32 different lines -- the lane-per-row form of this kernel ran at 99 % of the L1 pipe's tag rate.
+// G rows per step, up to 16 steps at a time.
+template <int D, int DT>
 __global__ void __launch_bounds__(256) dsa_attn_gather_rows_kernel(const GatherParams p) {
-  constexpr int LPR = D / 8;           // lanes per row
+  constexpr bool F32 = DT == SWV_F32, BF16 = DT == SWV_BF16;
+  constexpr int CE = F32 ? 4 : 8;      // elements per chunk
+  constexpr int LPR = D / CE;          // lanes per row
   constexpr int G = 32 / LPR;          // rows per warp step
-  constexpr int STEPS = 32 / G;        // steps per 32 slots
+  constexpr int STEPS = LPR < 16 ? LPR : 16;
+  constexpr int CH = G * STEPS;        // slots per round of the loop below
   __shared__ int s_idx[kRowsSlots];
   __shared__ float s_w[kRowsSlots];    // routing weight (s_idx < 0 marks a slot that is not valid)
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -204,23 +210,23 @@ __global__ void __launch_bounds__(256) dsa_attn_gather_rows_kernel(const GatherP
   const int h = blockIdx.y * nwarps + wib;
   const bool head_ok = h < p.H;
   const int grp = lane / LPR, chunk = lane % LPR;
-  const uint16_t* q16 = static_cast<const uint16_t*>(p.q);
-  const uint16_t* k16 = static_cast<const uint16_t*>(p.k);
-  const uint16_t* v16 = static_cast<const uint16_t*>(p.v);
-  uint4 qv = make_uint4(0, 0, 0, 0);   // this lane's 8 channels of q
-  if (head_ok) qv = __ldg(reinterpret_cast<const uint4*>(q16 + b * p.qs[0] + h * p.qs[1] + qi * p.qs[2]) + chunk);
+  using E = typename std::conditional<F32, float, uint16_t>::type;
+  uint4 qv = make_uint4(0, 0, 0, 0);   // this lane's channels of q
+  if (head_ok)
+    qv = __ldg(reinterpret_cast<const uint4*>(static_cast<const E*>(p.q) + b * p.qs[0] + h * p.qs[1] + qi * p.qs[2]) + chunk);
   const int hk = head_ok ? h / p.kv_group : 0;
-  const uint16_t* kbase = k16 + b * p.ks[0] + hk * p.ks[1];
-  const uint16_t* vbase = v16 + b * p.vs[0] + hk * p.vs[1];
+  const E* kbase = static_cast<const E*>(p.k) + b * p.ks[0] + hk * p.ks[1];
+  const E* vbase = static_cast<const E*>(p.v) + b * p.vs[0] + hk * p.vs[1];
   const int32_t* idx_row = p.idx + b * p.is[0] + qi * p.is[1];
   const float* val_row = p.valid + b * p.vls[0] + qi * p.vls[1];
   const float* rw_row = p.rw + b * p.rs[0] + qi * p.rs[1];
   const float ninf = -__int_as_float(0x7f800000);
 
-  float o[8];                          // channels [8 * chunk, +8) summed over this lane's rows
+  float o[CE];                         // channels [CE * chunk, + CE) summed over this lane's rows
 #pragma unroll
-  for (int i = 0; i < 8; ++i) o[i] = 0.f;
+  for (int i = 0; i < CE; ++i) o[i] = 0.f;
   float m = ninf, l = 0.f;
+  auto exp_ = [](float x) { return F32 ? expf(x) : __expf(x); };
 
   for (int base = 0; base < p.top_k; base += kRowsSlots) {
     __syncthreads();
@@ -243,8 +249,8 @@ __global__ void __launch_bounds__(256) dsa_attn_gather_rows_kernel(const GatherP
     __syncthreads();
     if (!head_ok) continue;
     const int n_here = min(kRowsSlots, p.top_k - base);
-    for (int c0 = 0; c0 < n_here; c0 += 32) {
-      // logits of the 32 slots: step s handles slots c0 + s * G + grp (one per lane group)
+    for (int c0 = 0; c0 < n_here; c0 += CH) {
+      // logits of the CH slots: step s handles slots c0 + s * G + grp (one per lane group)
       float logit[STEPS];
       int ids[STEPS];
       float cmax = ninf;
@@ -255,10 +261,17 @@ __global__ void __launch_bounds__(256) dsa_attn_gather_rows_kernel(const GatherP
         float a0 = 0.f, a1 = 0.f;
         if (id >= 0) {
           const uint4 kv = __ldg(reinterpret_cast<const uint4*>(kbase + static_cast<int64_t>(id) * p.ks[2]) + chunk);
-          fma_mixed2<BF16>(a0, a1, qv.x, kv.x);
-          fma_mixed2<BF16>(a0, a1, qv.y, kv.y);
-          fma_mixed2<BF16>(a0, a1, qv.z, kv.z);
-          fma_mixed2<BF16>(a0, a1, qv.w, kv.w);
+          if constexpr (F32) {
+            a0 = fmaf(__uint_as_float(qv.x), __uint_as_float(kv.x), a0);
+            a1 = fmaf(__uint_as_float(qv.y), __uint_as_float(kv.y), a1);
+            a0 = fmaf(__uint_as_float(qv.z), __uint_as_float(kv.z), a0);
+            a1 = fmaf(__uint_as_float(qv.w), __uint_as_float(kv.w), a1);
+          } else {
+            fma_mixed2<BF16>(a0, a1, qv.x, kv.x);
+            fma_mixed2<BF16>(a0, a1, qv.y, kv.y);
+            fma_mixed2<BF16>(a0, a1, qv.z, kv.z);
+            fma_mixed2<BF16>(a0, a1, qv.w, kv.w);
+          }
         }
         float a = a0 + a1;
 #pragma unroll
@@ -270,27 +283,33 @@ __global__ void __launch_bounds__(256) dsa_attn_gather_rows_kernel(const GatherP
       for (int off = 16; off >= LPR; off >>= 1) cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, off));
       if (cmax > m) {                                    // warp-uniform
         if (m != ninf) {
-          const float f = __expf(m - cmax);
+          const float f = exp_(m - cmax);
           l *= f;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] *= f;
+          for (int i = 0; i < CE; ++i) o[i] *= f;
         }
         m = cmax;
       }
+      if (m == ninf) continue;                           // no finite logit so far
 #pragma unroll
       for (int s_ = 0; s_ < STEPS; ++s_) {
         const int id = ids[s_];
-        const float pj = id >= 0 ? __expf(logit[s_] - m) * s_w[c0 + s_ * G + grp] : 0.f;
+        const float pj = id >= 0 ? exp_(logit[s_] - m) * s_w[c0 + s_ * G + grp] : 0.f;
         if (pj != 0.f) {                                  // uniform within the lane group
           if (chunk == 0) l += pj;
-          uint32_t ph, pl;
-          split16<BF16>(pj, ph, pl);
           const uint4 vv = __ldg(reinterpret_cast<const uint4*>(vbase + static_cast<int64_t>(id) * p.vs[2]) + chunk);
           const uint32_t vw[4] = {vv.x, vv.y, vv.z, vv.w};
+          if constexpr (F32) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            fma_mixed2<BF16>(o[2 * c], o[2 * c + 1], ph, vw[c]);
-            fma_mixed2<BF16>(o[2 * c], o[2 * c + 1], pl, vw[c]);
+            for (int c = 0; c < 4; ++c) o[c] = fmaf(pj, __uint_as_float(vw[c]), o[c]);
+          } else {
+            uint32_t ph, pl;
+            split16<BF16>(pj, ph, pl);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              fma_mixed2<BF16>(o[2 * c], o[2 * c + 1], ph, vw[c]);
+              fma_mixed2<BF16>(o[2 * c], o[2 * c + 1], pl, vw[c]);
+            }
           }
         }
       }
@@ -303,33 +322,34 @@ __global__ void __launch_bounds__(256) dsa_attn_gather_rows_kernel(const GatherP
 #pragma unroll
   for (int off = 16; off >= LPR; off >>= 1) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] += __shfl_xor_sync(0xffffffffu, o[i], off);
+    for (int i = 0; i < CE; ++i) o[i] += __shfl_xor_sync(0xffffffffu, o[i], off);
   }
   if (grp == 0) {
     const float inv = 1.f / fmaxf(l, 1e-6f);
     const int64_t obase = b * p.os[0] + h * p.os[1] + qi * p.os[2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) st_out(p.o, p.o_dtype, obase + (chunk * 8 + i) * p.os[3], o[i] * inv);
+    for (int i = 0; i < CE; ++i) st_out(p.o, p.o_dtype, obase + (chunk * CE + i) * p.os[3], o[i] * inv);
   }
 }
 
 static bool rows_path_ok(const GatherParams& p, int dtype, int D) {
-  if (dtype == SWV_F32 || (D != 32 && D != 64 && D != 128)) return false;
+  if (D != 32 && D != 64 && D != 128) return false;
+  const int es = dtype == SWV_F32 ? 4 : 2;
   auto a16 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
   if (!a16(p.q) || !a16(p.k) || !a16(p.v)) return false;
   if (p.qs[3] != 1 || p.ks[3] != 1 || p.vs[3] != 1) return false;
   for (int i = 0; i < 3; ++i)
-    if ((p.qs[i] * 2) % 16 || (p.ks[i] * 2) % 16 || (p.vs[i] * 2) % 16) return false;
+    if ((p.qs[i] * es) % 16 || (p.ks[i] * es) % 16 || (p.vs[i] * es) % 16) return false;
   return true;
 }
 
-template <bool BF16>
+template <int DT>
 static int launch_gather_rows(const GatherParams& p, int D, cudaStream_t st) {
   const int warps = p.H < 8 ? p.H : 8;
   const dim3 grid(static_cast<unsigned>(p.B) * p.Tq, static_cast<unsigned>((p.H + warps - 1) / warps));
-  if (D == 32) dsa_attn_gather_rows_kernel<32, BF16><<<grid, 32 * warps, 0, st>>>(p);
-  else if (D == 64) dsa_attn_gather_rows_kernel<64, BF16><<<grid, 32 * warps, 0, st>>>(p);
-  else dsa_attn_gather_rows_kernel<128, BF16><<<grid, 32 * warps, 0, st>>>(p);
+  if (D == 32) dsa_attn_gather_rows_kernel<32, DT><<<grid, 32 * warps, 0, st>>>(p);
+  else if (D == 64) dsa_attn_gather_rows_kernel<64, DT><<<grid, 32 * warps, 0, st>>>(p);
+  else dsa_attn_gather_rows_kernel<128, DT><<<grid, 32 * warps, 0, st>>>(p);
   return cudaGetLastError() == cudaSuccess ? SWV_OK : SWV_ERR_CUDA;
 }
 
@@ -364,8 +384,10 @@ int dsa_attn_gather_impl(const void* q, const int64_t* qs, const void* k, const 
   p.B = B; p.H = H; p.Tq = Tq; p.Tk = Tk; p.D = D; p.top_k = top_k; p.kv_group = kv_group;
   p.scale = 1.0f / sqrtf(static_cast<float>(D));
   p.status = status;
-  if (rows_path_ok(p, dtype, D))
-    return dtype == SWV_BF16 ? launch_gather_rows<true>(p, D, st) : launch_gather_rows<false>(p, D, st);
+  if (rows_path_ok(p, dtype, D)) {
+    if (dtype == SWV_F32) return launch_gather_rows<SWV_F32>(p, D, st);
+    return dtype == SWV_BF16 ? launch_gather_rows<SWV_BF16>(p, D, st) : launch_gather_rows<SWV_F16>(p, D, st);
+  }
   if (dtype == SWV_F32) return launch_gather<float>(p, D, st);
   if (dtype == SWV_BF16) return launch_gather<__nv_bfloat16>(p, D, st);
   return launch_gather<__half>(p, D, st);

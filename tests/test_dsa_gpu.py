@@ -475,3 +475,26 @@ def test_two_sweep_selection_on_a_rank_share(swv, scale):
     swv.dsa_attention_gather(q_loc, k, v, idx, valid, scores * valid, o2)
     _check(swv)
     assert float((o1 - o2).abs().max()) < 2e-2
+
+
+@pytest.mark.parametrize("D,K,Tk,kvg", [(32, 1, 40, 1), (64, 257, 300, 3), (128, 300, 129, 1), (64, 31, 77, 1)])
+def test_gather_fp32_rows_vs_general_kernel(swv, D, K, Tk, kvg):
+    """fp32 rows of 16-byte chunks against the lane-per-row kernel (which unaligned rows take), on any-order
+    lists with repeats, slots that are not valid and a query without any: fp32 sums in another order, so
+    2^-20 of the largest value."""
+    B, H, Tq = 2, 3, 70
+    g = torch.Generator().manual_seed(D + K)
+    q = torch.randn(B, H, Tq, D, generator=g).to(_dev())
+    k, v = (torch.randn(B, H // kvg, Tk, D, generator=g).to(_dev()) for _ in range(2))
+    idx = torch.randint(0, Tk, (B, Tq, K), generator=g, dtype=torch.int32).to(_dev())
+    valid = (torch.rand(B, Tq, K, generator=g) < 0.8).float().to(_dev())
+    valid[:, 3] = 0
+    rw = torch.rand(B, Tq, K, generator=g).to(_dev()) + 0.1
+    o = torch.empty(B, H, Tq, D, device=_dev())
+    swv.dsa_attention_gather(q, k, v, idx, valid, rw, o, kv_group=kvg)
+    wide = lambda x: torch.nn.functional.pad(x, (0, 1))[..., :-1]           # rows that start at odd words
+    o2 = torch.empty_like(o)
+    swv.dsa_attention_gather(wide(q), wide(k), wide(v), idx, valid, rw, o2, kv_group=kvg)
+    _check(swv)
+    assert float(o[:, :, 3].abs().max()) == 0
+    assert float((o - o2).abs().max()) < 2.0 ** -20 * float(o2.abs().max())
