@@ -65,8 +65,10 @@ int swv_dsa_workspace_bytes(int B, int Tq, int Tk, size_t* bytes);
  * (49152 to 262144 keys, between about one key in 70 and one in 16 selected, candidate lists of at
  * most 12288 entries per row, i.e. top_k up to about 5000) it is larger than
  * swv_dsa_workspace_bytes: swv_dsa_indexer_topk_fwd then has room for per-row candidate lists and
- * selects in two sweeps over the score tiles instead of three (same results).  With the smaller
- * workspace the entry takes the three-sweep form. */
+ * selects in two sweeps over the score tiles instead of three (same results).  For short sequences
+ * (at most 4096 tiles of 128 x 128 scores over the batch, at most 16384 keys) it has room for the score
+ * matrix itself (64 KiB per tile, at most 256 MiB), from which every row is selected at once (same
+ * results).  With the smaller workspace the entry takes the three-sweep form. */
 int swv_dsa_workspace_bytes_topk(int B, int Tq, int Tk, int top_k, size_t* bytes);
 
 /* Bytes of the tile-major membership bitmask for B x Tq x Tk:

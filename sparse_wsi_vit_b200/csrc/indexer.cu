@@ -15,8 +15,11 @@
 //      instruction sequence) and writes idx / scores in ascending key order plus the
 //      tile-major membership bitmask.  Ties at the threshold go to the lower key index.
 //   4. fill_valid_kernel : valid[.., s] = s < min(K, Tk); zero padding of idx/scores.
-// The N x N score matrix never reaches global memory.
+// The score matrix never reaches global memory in these forms.  Up to kDenseTiles score tiles (8192 x 8192)
+// it does: indexer_tiles_kernel<SCORES> writes it once, with as many CTAs as the chip holds, and
+// dsa_select_dense_kernel selects every row from it (see there for the measurements).
 #include <cmath>
+#include <cstdint>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -125,6 +128,7 @@ __global__ void __launch_bounds__(128)
 // --------------------------------------------------------------- tile kernel
 constexpr int kModeHist = 0;
 constexpr int kModeEmit = 1;
+constexpr int kModeScores = 2;
 constexpr int kStages = 2;                         // wk ring depth
 constexpr int kTileBytes = kTile * kIdxDim * 4;    // 32 KiB fp32 tile (two 16 KiB K-halves)
 constexpr int kHistStride = 259;                   // words per histogram row (256 bins + 3: odd, bank spread)
@@ -153,7 +157,8 @@ struct IndexerParams {
                           // index), ascending, the first kMaxExcl of them
   // Key-range split: with few query tiles (a rank of a sequence-sharded run) `split` = 2 CTAs share
   // a query tile, each sweeping half of the key tiles; the part that finishes last merges.
-  int split, nKT0;               // CTAs per query tile; key tiles of part 0
+  int split, nKT0;               // CTAs per query tile; key tiles of part 0 (SCORES: of every part but the last)
+  uint32_t* dense;               // SCORES: bits of max(score, 0), [B*nQT*128][nKT*128]
   const uint32_t* flags_spec;    // [tiles] speculative pass failed: the candidate pass runs unsplit
   uint32_t* flags_unsplit;       // [tiles] written by the candidate pass: emit runs unsplit
   uint32_t* tickets;             // [tiles] arrival counter of a tile's parts (reset by the last one)
@@ -197,9 +202,12 @@ struct TileSmemCtl {
 constexpr int kRing = 32;
 constexpr int kRingStride = kRing + 1;             // words per row (+1: bank spread)
 constexpr int kStageBytes = 16 * 32 * 32 * 4 + 2 * kTile * 4 * 8 + 2 * kTile * kRingStride * 4;
+// (SCORES: a 4 KiB patch per epilogue warp)
+constexpr int mode_bytes(int mode) {
+  return mode == kModeHist ? kHistBytes : mode == kModeEmit ? kStageBytes : 16 * 32 * 32 * 4;
+}
 constexpr size_t tile_smem_bytes(int mode) {
-  return 1024 /*alignment slack*/ + kTileBytes * (1 + kStages) + (mode == kModeHist ? kHistBytes : kStageBytes) +
-         sizeof(TileSmemCtl) + 64;
+  return 1024 /*alignment slack*/ + kTileBytes * (1 + kStages) + mode_bytes(mode) + sizeof(TileSmemCtl) + 64;
 }
 
 // Bit pattern of max(x, 0) for a float x given as bits: as SIGNED integers the negative
@@ -277,8 +285,7 @@ __global__ void __launch_bounds__(576, 1)
   uint8_t* sm_q = smem;
   uint8_t* sm_k = smem + kTileBytes;
   uint32_t* sm_hist = reinterpret_cast<uint32_t*>(smem + kTileBytes * (1 + kStages));
-  TileSmemCtl* ctl = reinterpret_cast<TileSmemCtl*>(smem + kTileBytes * (1 + kStages) +
-                                                    (MODE == kModeHist ? kHistBytes : kStageBytes));
+  TileSmemCtl* ctl = reinterpret_cast<TileSmemCtl*>(smem + kTileBytes * (1 + kStages) + mode_bytes(MODE));
 
   const int tile = blockIdx.x / p.split;         // (batch, query tile)
   const int part = blockIdx.x - tile * p.split;  // which share of the key range
@@ -287,7 +294,7 @@ __global__ void __launch_bounds__(576, 1)
   // speculative pass failed for the tile; emit unless the candidate pass said otherwise; the
   // classic histogram passes never.  An unsplit tile is swept by part 0 alone.
   bool use_split = false;
-  if (p.split > 1) {
+  if (MODE != kModeScores && p.split > 1) {
     if (MODE == kModeEmit) use_split = p.collect != 0 || p.flags_unsplit[tile] == 0u;
     else if (p.kind == kKindSpec) use_split = true;
     else if (p.kind == kKindCand) use_split = p.flags_spec[tile] == 0u;
@@ -298,8 +305,10 @@ __global__ void __launch_bounds__(576, 1)
   const int lane = threadIdx.x & 31;
   const int b = tile / p.nQT;
   const int qt = tile % p.nQT;
-  const int kt0 = (use_split && part == 1) ? p.nKT0 : 0;                 // first key tile of this CTA
-  const int nKT = (use_split ? (part == 0 ? p.nKT0 : p.nKT - p.nKT0) : p.nKT);   // key tiles of this CTA
+  // first key tile and number of key tiles of this CTA
+  const int kt0 = MODE == kModeScores ? part * p.nKT0 : (use_split && part == 1) ? p.nKT0 : 0;
+  const int nKT = MODE == kModeScores ? min(p.nKT0, p.nKT - kt0)
+                                      : (use_split ? (part == 0 ? p.nKT0 : p.nKT - p.nKT0) : p.nKT);
   // The speculative pass first streams a sample of nSample key tiles twice (top byte, then second
   // byte of every row's estimated threshold; the same tiles for every part), then its key range.
   const bool estimate = MODE == kModeHist && p.kind == kKindEstimate;
@@ -395,7 +404,43 @@ __global__ void __launch_bounds__(576, 1)
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     bool ok = true;
 
-    if (MODE == kModeHist && (p.kind == kKindSpec || p.kind == kKindEstimate)) {
+    if constexpr (MODE == kModeScores) {
+      // every warp turns its 32 x 32 scores through its own patch (16-byte pieces, swizzled by the row) and
+      // writes four rows of 128 bytes per instruction
+      const int ch = ew >> 2;
+      const uint32_t patch = smem_u32(sm_hist) + static_cast<uint32_t>(ew) * 4096u;
+      const int64_t ld = static_cast<int64_t>(p.nKT) * kTile;
+      uint32_t* dst = p.dense + (static_cast<int64_t>(tile) * kTile + quarter * 32 + (lane >> 3)) * ld +
+                      static_cast<int64_t>(kt0) * kTile + ch * 32 + (lane & 7) * 4;
+      for (int j = 0; j < nKT; ++j) {
+        const int a = j & 1;
+        if (!mbar_wait_bounded(&ctl->acc_full[a], (j >> 1) & 1, abort_flag)) {
+          record_status(p.status, kDevWaitAccFull);
+          ok = false;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t r[32];
+        tmem_ld32(lane_base + a * kTile + ch * 32, r);
+        tc_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl->acc_empty[a]);
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          sts128(patch + lane * 128 + ((c ^ (lane & 7)) << 4), relu_bits(r[4 * c]), relu_bits(r[4 * c + 1]),
+                 relu_bits(r[4 * c + 2]), relu_bits(r[4 * c + 3]));
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int rr = i * 4 + (lane >> 3);
+          const uint4 x = lds128(patch + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4));
+          *reinterpret_cast<uint4*>(dst + i * 4 * ld + j * kTile) = x;
+        }
+        __syncwarp();
+      }
+    } else if (MODE == kModeHist && (p.kind == kKindSpec || p.kind == kKindEstimate)) {
       // Speculative fusion of the two first radix passes.  Phase 1 estimates, per row, the top 16
       // bits of the K-th largest score from a sample of key tiles (rank scaled to the sample; two
       // 8-bit histogram rounds).  Phase 2 streams all keys against a 2^24-wide window of bit
@@ -1158,6 +1203,227 @@ __global__ void __launch_bounds__(32 * kSelWarps) dsa_select_kernel(const Select
   }
 }
 
+// ---- exact top-k of every row of a score matrix in global memory (indexer_tiles_kernel<SCORES>); same outputs
+// and row state as the sweeps and fill_valid_kernel.  One CTA per row (of the padded query tiles): the row in
+// shared memory, a radix select, then every warp walks its share of the keys; 32 keys in a row are one word of
+// the membership bitmask.
+// Why: the sweeps give a query tile to one CTA, which takes ~4-6 us per key tile in its serial epilogue, so
+// short sequences leave the chip idle (1021 keys: 8 CTAs).  Whole indexer call with bitmask, sweeps -> here:
+// 1021 keys, top-512: 267 -> 32 us; 2048: 220 -> 48; 4099: 278 -> 107; 6007, top-1024: 419 -> 198; 8192,
+// top-2048: 415 -> 325.  Beyond, the matrix outgrows the L2 and the sweeps fill the chip: 12288 keys 697 us
+// with sweeps, 1056 here.
+struct DenseSelectParams {
+  int B, Tq, Tk, top_k, k_eff, nQT, nKT;
+  const uint32_t* dense;
+  int32_t* idx;
+  float *valid, *scores;
+  uint32_t *st_prefix, *st_kth, *st_neq;
+  int32_t* st_excl;
+  uint32_t* maskbits;          // may be null
+};
+constexpr int kDenseBins = 2048;
+__device__ __forceinline__ int dense_bin(uint32_t bin) { return static_cast<int>(bin + (bin >> 4)); }   // bank spread
+constexpr int kDenseHist = kDenseBins + kDenseBins / 16;
+
+template <int NT>
+__global__ void __launch_bounds__(NT) dsa_select_dense_kernel(const DenseSelectParams p) {
+  extern __shared__ __align__(16) uint32_t dsel_smem[];
+  const int n_pad = p.nKT * kTile, n = p.Tk;
+  uint32_t* sc_s = dsel_smem;
+  uint32_t* hist = sc_s + n_pad;
+  uint32_t* xch = hist + kDenseHist;
+  constexpr int NW = NT / 32;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tile = blockIdx.x >> 7, r = blockIdx.x & (kTile - 1);
+  const int b = tile / p.nQT, t = (tile - b * p.nQT) * kTile + r;
+  uint4* mask = p.maskbits == nullptr
+                    ? nullptr
+                    : reinterpret_cast<uint4*>(p.maskbits) + static_cast<int64_t>(tile) * p.nKT * kTile + r;
+  if (t >= p.Tq) {                               // a row behind the end: its scores are zero, every key a member
+    if (mask != nullptr)
+      for (int kt = tid; kt < p.nKT; kt += NT) {
+        uint32_t w[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int left = n - kt * kTile - c * 32;
+          w[c] = left >= 32 ? 0xffffffffu : left <= 0 ? 0u : (1u << left) - 1u;
+        }
+        mask[static_cast<int64_t>(kt) * kTile] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    return;
+  }
+  const int64_t row = static_cast<int64_t>(b) * p.Tq + t;
+  // the row, its largest value and how many of its scores are above zero (the padding columns are zero)
+  uint32_t vmax = 0, nz = 0;
+  {
+    const uint4* src = reinterpret_cast<const uint4*>(p.dense + static_cast<int64_t>(blockIdx.x) * n_pad);
+#pragma unroll 4
+    for (int i4 = tid; i4 < n_pad / 4; i4 += NT) {
+      const uint4 x = __ldg(src + i4);
+      reinterpret_cast<uint4*>(sc_s)[i4] = x;
+      vmax = max(max(vmax, max(x.x, x.y)), max(x.z, x.w));
+      nz += (x.x != 0u) + (x.y != 0u) + (x.z != 0u) + (x.w != 0u);
+    }
+    vmax = __reduce_max_sync(0xffffffffu, vmax);
+    nz = __reduce_add_sync(0xffffffffu, nz);
+    if (lane == 0) {
+      xch[16 + warp] = vmax;
+      xch[24 + warp] = nz;
+    }
+    for (int i = tid; i < kDenseHist; i += NT) hist[i] = 0u;
+    __syncthreads();
+    nz = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      vmax = max(vmax, xch[16 + w]);
+      nz += xch[24 + w];
+    }
+  }
+  uint32_t kth = static_cast<uint32_t>(p.k_eff), n_eq, thr = 0;
+  if (nz < kth) {                                // the threshold is zero
+    kth -= nz;
+    n_eq = static_cast<uint32_t>(n) - nz;
+  } else {
+    // k-th smallest u = vmax - v of the positive scores, in digits of 11 + 11 + 3 bits when it lies in a window
+    // of 2^25 bit patterns (down to a sixteenth of the largest score: 512 bins an octave, few lanes of a warp
+    // meet in one), else of 11 + 10 + 10 bits over all patterns (8 bins an octave).
+    uint32_t prefix = 0;
+    bool window = true;
+    for (int pass = 0; pass < 3; ++pass) {
+      const int shift = window ? (pass == 0 ? 14 : pass == 1 ? 3 : 0) : 20 - 10 * pass;
+      const int bits = window ? (pass == 2 ? 3 : 11) : (pass == 0 ? 11 : 10);
+      const uint32_t hi = static_cast<uint32_t>(shift + bits), digit_mask = (1u << bits) - 1u;
+      const uint32_t want = prefix >> hi;        // (hi <= 31)
+      for (int i4 = tid; i4 < n_pad / 4; i4 += NT) {
+        const uint4 x = reinterpret_cast<const uint4*>(sc_s)[i4];
+        const uint32_t v[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t u = vmax - v[e];
+          if (v[e] != 0u && (u >> hi) == want) atomicAdd(hist + dense_bin((u >> shift) & digit_mask), 1u);
+        }
+      }
+      __syncthreads();
+      // thread 0 owns the lowest bins
+      const int per = max(1, (1 << bits) / NT);
+      uint32_t c = 0;
+      for (int i = 0; i < per; ++i) c += hist[dense_bin(tid * per + i)];
+      uint32_t cum = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, cum, o);
+        if (lane >= o) cum += up;
+      }
+      if (lane == 31) xch[warp] = cum;
+      __syncthreads();
+      uint32_t all = 0, before = 0;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        if (w < warp) before += xch[w];
+        all += xch[w];
+      }
+      const bool found = all >= kth;
+      cum += before;
+      if (cum >= kth && cum - c < kth) {         // exactly one thread, if found
+        uint32_t below = cum - c;
+        for (int i = 0; i < per; ++i) {
+          const uint32_t h = hist[dense_bin(tid * per + i)];
+          if (below + h >= kth) {
+            xch[8] = static_cast<uint32_t>(tid * per + i);
+            xch[9] = below;
+            xch[10] = h;
+            break;
+          }
+          below += h;
+        }
+      }
+      __syncthreads();
+      if (found) {
+        prefix |= xch[8] << shift;
+        kth -= xch[9];
+        n_eq = xch[10];
+      } else {                                   // only the first pass over the window can miss
+        window = false;
+        pass = -1;
+      }
+      if (pass < 2)
+        for (int i = tid; i < kDenseHist; i += NT) hist[i] = 0u;
+      __syncthreads();
+    }
+    thr = vmax - prefix;
+  }
+  const uint32_t take = kth;                     // of the n_eq keys equal to the threshold that are selected
+  const uint32_t lt = (1u << lane) - 1u;
+  int32_t* idx_row = p.idx + row * p.top_k;
+  float* sc_row = p.scores + row * p.top_k;
+  const int share = (p.nKT + NW - 1) / NW * kTile;
+  const int lo_i = min(n, warp * share), hi_i = min(n, lo_i + share);
+  uint32_t gt = 0, eq = 0;
+  for (int i = lo_i + lane; i < hi_i; i += 32) {
+    const uint32_t v = sc_s[i];
+    gt += v > thr ? 1u : 0u;
+    eq += v == thr ? 1u : 0u;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    gt += __shfl_xor_sync(0xffffffffu, gt, o);
+    eq += __shfl_xor_sync(0xffffffffu, eq, o);
+  }
+  if (lane == 0) {
+    xch[32 + 2 * warp] = gt;
+    xch[33 + 2 * warp] = eq;
+  }
+  __syncthreads();
+  uint32_t out = 0, eq_seen = 0, ex_seen = 0;    // totals of the shares before this one
+  for (int w = 0; w < warp; ++w) {
+    const uint32_t e = xch[33 + 2 * w];
+    const uint32_t tk = min(e, take > eq_seen ? take - eq_seen : 0u);
+    out += xch[32 + 2 * w] + tk;
+    ex_seen += e - tk;
+    eq_seen += e;
+  }
+  for (int base = lo_i; base < hi_i; base += kTile) {
+    uint32_t words[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = base + c * 32 + lane;
+      const bool in = i < hi_i;
+      const uint32_t v = in ? sc_s[i] : 0u;
+      const bool is_eq = in && v == thr;
+      const uint32_t eq_mask = __ballot_sync(0xffffffffu, is_eq);
+      const uint32_t eq_rank = eq_seen + __popc(eq_mask & lt);
+      const bool sel = (in && v > thr) || (is_eq && eq_rank < take);
+      const uint32_t sel_mask = __ballot_sync(0xffffffffu, sel);
+      if (sel) {
+        const uint32_t slot = out + __popc(sel_mask & lt);      // (< k_eff: gt + take == k_eff)
+        idx_row[slot] = i;
+        sc_row[slot] = __uint_as_float(v);
+      } else if (is_eq) {
+        const uint32_t ex = ex_seen + __popc(eq_mask & ~sel_mask & lt);
+        if (ex < static_cast<uint32_t>(kMaxExcl)) p.st_excl[row * kMaxExcl + ex] = i;
+      }
+      out += __popc(sel_mask);
+      ex_seen += __popc(eq_mask & ~sel_mask);
+      eq_seen += __popc(eq_mask);
+      words[c] = sel_mask;
+    }
+    if (lane == 0 && mask != nullptr)
+      mask[static_cast<int64_t>(base >> 7) * kTile] = make_uint4(words[0], words[1], words[2], words[3]);
+  }
+  for (int s0 = tid; s0 < p.top_k; s0 += NT) {
+    p.valid[row * p.top_k + s0] = s0 < p.k_eff ? 1.f : 0.f;
+    if (s0 >= p.k_eff) {
+      idx_row[s0] = 0;
+      sc_row[s0] = 0.f;
+    }
+  }
+  if (tid == 0) {
+    p.st_prefix[row] = thr;
+    p.st_kth[row] = take;
+    p.st_neq[row] = n_eq;
+  }
+}
+
 // valid[b,t,s] = s < k_eff ; slots >= k_eff of idx / scores are zeroed.  VEC consecutive slots per
 // thread (VEC divides top_k, so a thread never crosses a row).
 template <int VEC>
@@ -1249,7 +1515,11 @@ static WorkspaceLayout workspace_layout(int B, int Tq, int Tk) {
 
 // The short form of the selection (estimate, collect, select) needs candidate lists behind the base
 // layout: 2.0-2.5 k candidates per row (1.3-1.7 k expected), divided over the parts of a split key range.
+constexpr int kDenseTiles = 4096;        // score tiles (256 MiB) up to which the score matrix is written out ...
+constexpr int kDenseKeyTiles = 128;      // ... and key tiles of a row (64 KiB of shared memory in the select)
 struct FastLayout {
+  bool dense_ok;           // short sequences: room for the score matrix
+  size_t dense_off;
   bool ok;                 // the shape qualifies
   int cand_cap;            // per (row, part)
   int est_rank;            // rank in the sample at which the estimate pass takes a row's lower bound
@@ -1292,6 +1562,10 @@ static FastLayout fast_layout(int B, int Tq, int Tk, int top_k) {
   F.cnt_off = off;
   off += align_up(rows * L.split * 4, 1024);
   F.total = F.ok ? off : L.total;
+  const int64_t nQT = (Tq + kTile - 1) / kTile, nKT = (Tk + kTile - 1) / kTile;
+  F.dense_ok = !F.ok && nKT <= kDenseKeyTiles && B * nQT * nKT <= kDenseTiles;
+  F.dense_off = L.total;
+  if (F.dense_ok) F.total += static_cast<size_t>(B * nQT * nKT) * kTile * kTile * 4;
   return F;
 }
 
@@ -1422,9 +1696,6 @@ int dsa_indexer_topk_impl(const void* q_idx, const int64_t* qs, const void* k_id
   p.ghist = reinterpret_cast<uint32_t*>(ws + L.ghist_off);
   p.glist = reinterpret_cast<uint16_t*>(ws + L.glist_off);
   p.gcnt = reinterpret_cast<uint32_t*>(ws + L.gcnt_off);
-  if (L.split > 1)
-    SWV_CUDA_OK(cudaMemsetAsync(p.tickets, 0, static_cast<size_t>(B) * p.nQT * 4, st));
-
   SWV_CUDA_OK(cudaFuncSetAttribute(indexer_tiles_kernel<kModeHist>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(tile_smem_bytes(kModeHist))));
   SWV_CUDA_OK(cudaFuncSetAttribute(indexer_tiles_kernel<kModeEmit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1436,9 +1707,41 @@ int dsa_indexer_topk_impl(const void* q_idx, const int64_t* qs, const void* k_id
   //   bytes 2-3: one candidate-list pass; tiles whose list overflowed (massive ties) redo the two
   //              classic histogram passes.
   const size_t hs = tile_smem_bytes(kModeHist);
-  p.collect = 0; p.est_rank = 0; p.cand_cap = 0;
+  p.collect = 0; p.est_rank = 0; p.cand_cap = 0; p.dense = nullptr;
   p.cand_idx = nullptr; p.cand_sc = nullptr; p.cand_cnt = nullptr;
   const FastLayout F = fast_layout(B, Tq, Tk, top_k);
+  if (L.split > 1) SWV_CUDA_OK(cudaMemsetAsync(p.tickets, 0, static_cast<size_t>(B) * p.nQT * 4, st));
+  if (F.dense_ok && allow_split && workspace_bytes >= F.total) {
+    // Parts per query tile: the fewest rounds of CTAs, at two tiles' time of start-up each.
+    const int64_t tiles = static_cast<int64_t>(B) * p.nQT, n_sm = sm_count();
+    int64_t best = INT64_MAX;
+    for (int parts = 1; parts <= p.nKT; ++parts) {
+      const int per = (p.nKT + parts - 1) / parts;
+      const int64_t cost = (tiles * ((p.nKT + per - 1) / per) + n_sm - 1) / n_sm * (per + 2);
+      if (cost < best) {
+        best = cost;
+        p.nKT0 = per;
+      }
+    }
+    p.split = (p.nKT + p.nKT0 - 1) / p.nKT0;
+    p.dense = reinterpret_cast<uint32_t*>(ws + F.dense_off);
+    SWV_CUDA_OK(cudaFuncSetAttribute(indexer_tiles_kernel<kModeScores>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(tile_smem_bytes(kModeScores))));
+    indexer_tiles_kernel<kModeScores>
+        <<<static_cast<unsigned>(tiles * p.split), 576, tile_smem_bytes(kModeScores), st>>>(tm_q, tm_k, p);
+    DenseSelectParams sp;
+    sp.B = B; sp.Tq = Tq; sp.Tk = Tk; sp.top_k = top_k; sp.k_eff = top_k < Tk ? top_k : Tk;
+    sp.nQT = p.nQT; sp.nKT = p.nKT; sp.dense = p.dense; sp.idx = idx; sp.valid = valid; sp.scores = scores;
+    sp.st_prefix = p.st_prefix; sp.st_kth = p.st_kth; sp.st_neq = p.st_neq; sp.st_excl = p.st_excl;
+    sp.maskbits = maskbits;
+    const size_t sel_smem = (static_cast<size_t>(p.nKT) * kTile + kDenseHist + 64) * 4;
+    // a short row does not feed eight warps (4099 keys: 107 against 114 us; 8192: 382 against 325)
+    auto* select = p.nKT <= 40 ? dsa_select_dense_kernel<128> : dsa_select_dense_kernel<256>;
+    SWV_CUDA_OK(cudaFuncSetAttribute(select, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sel_smem)));
+    select<<<static_cast<unsigned>(tiles * kTile), p.nKT <= 40 ? 128 : 256, sel_smem, st>>>(sp);
+    SWV_CUDA_OK(cudaGetLastError());
+    return SWV_OK;
+  }
   if (F.ok && allow_split && workspace_bytes >= F.total) {
     // Sparse top-k on a long key range, and the caller brought the larger workspace
     // (swv_dsa_workspace_bytes_topk): TWO sweeps instead of three.

@@ -477,6 +477,45 @@ def test_two_sweep_selection_on_a_rank_share(swv, scale):
     assert float((o1 - o2).abs().max()) < 2e-2
 
 
+@pytest.mark.parametrize("B,Tq,Tk,K,ID,ties,want_mask", [
+    (1, 1, 1, 1, 64, False, True),            # one key
+    (1, 127, 127, 200, 32, False, True),      # less than a tile, more slots than keys
+    (2, 128, 128, 64, 64, True, True),        # exactly one tile, batch, ties
+    (1, 129, 1021, 512, 32, False, False),    # ragged tiles, no bitmask
+    (3, 257, 2049, 1000, 64, True, True),     # one key beyond a tile, massive ties at the threshold
+    (1, 130, 16384, 77, 64, False, True),     # the most key tiles a row may have
+    (1, 8192, 8192, 2048, 64, False, True),   # the most score tiles
+])
+def test_dense_selection_equals_the_sweeps(swv, B, Tq, Tk, K, ID, ties, want_mask):
+    """Short sequences: the selection from the written score matrix against the sweeps (which run when the
+    caller's workspace has no room for the matrix): lists, scores, valid and bitmask bit for bit, and the row
+    state through the attention that reads it."""
+    g = torch.Generator().manual_seed(Tk + K)
+    qi, ki = torch.randn(B, Tq, 4, ID, generator=g) / 8, torch.randn(B, Tk, 4, ID, generator=g) / 8
+    if ties:
+        qi, ki = (qi * 4).round() / 4, (ki * 4).round() / 4
+    qi, ki = qi.to(torch.bfloat16).to(_dev()), ki.to(torch.bfloat16).to(_dev())
+    w = torch.randn(4, generator=g).to(_dev())
+    base, full = swv.ops.workspace_bytes(B, Tq, Tk), swv.ops.workspace_bytes(B, Tq, Tk, K)
+    assert full > base
+    q = torch.randn(B, 2, Tq, 64, generator=g).to(torch.bfloat16).to(_dev())
+    k, v = (torch.randn(B, 2, Tk, 64, generator=g).to(torch.bfloat16).to(_dev()) for _ in range(2))
+    res = []
+    for nbytes in (base, full):
+        ws = torch.full((nbytes,), 255, dtype=torch.uint8, device=_dev())
+        out = swv.dsa_indexer_topk(qi, ki, w, K, want_mask=want_mask, workspace=ws)
+        bits = o = None
+        if want_mask:
+            nqt, nkt = -(-Tq // 128), -(-Tk // 128)
+            bits = out[3][0].reshape(B, nqt, nkt, 128, 4).permute(0, 1, 3, 2, 4).reshape(B, nqt * 128, nkt * 4)[:, :Tq]
+            o = torch.zeros((B, 2, Tq, 64), dtype=torch.float32, device=_dev())
+            swv.dsa_attention_masked(q, k, v, out[3], o)
+        res.append((*out[:3], bits, o))
+    _check(swv)
+    for name, x, y in zip(("idx", "valid", "scores", "bitmask", "attention"), *res):
+        assert x is None or torch.equal(x, y), name
+
+
 @pytest.mark.parametrize("D,K,Tk,kvg", [(32, 1, 40, 1), (64, 257, 300, 3), (128, 300, 129, 1), (64, 31, 77, 1)])
 def test_gather_fp32_rows_vs_general_kernel(swv, D, K, Tk, kvg):
     """fp32 rows of 16-byte chunks against the lane-per-row kernel (which unaligned rows take), on any-order
