@@ -165,6 +165,7 @@ def test_encoder_train_steps_reduce_the_loss(swv):
     (1, 517, 2, 4, 64, 96, torch.float32, False),     # gradients with more bits than bf16: the list kernel takes over
     (1, 260, 1, 2, 32, 300, torch.bfloat16, True),    # more slots than keys, one 64-channel projection block
     (1, 391, 2, 3, 64, 33, torch.bfloat16, True),     # 192 projection channels: indexer gradients on the list kernel
+    (2, 1100, 1, 4, 32, 48, torch.bfloat16, True),    # few tiles: the indexer gradients' streamed range in two parts
 ])
 def test_tile_backward_vs_oracle(swv, B, T, H, IH, ID, K, o_dtype, exact):
     """The tensor-core backward on the selection of the library's own indexer, against the oracle's
