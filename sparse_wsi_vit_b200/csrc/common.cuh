@@ -4,6 +4,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cuda.h>
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include "../../include/swv_b200.h"
@@ -144,6 +145,55 @@ inline int make_tmap_4d(CUtensorMap* out, const void* base, CUtensorMapDataType 
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? SWV_OK : SWV_ERR_TENSORMAP;
+}
+
+// 2-D rotary embedding of one channel pair of every head, (y[0], y[1]) = (x[0], x[1]) turned by the angle with
+// this sine and cosine (in place where y is x); explicit rounding order, so that every kernel that rotates gives
+// the same bits.  `vec`: every pair lies on an address that is a multiple of its size (one access instead of
+// two).  Four heads are read before the first of them is written: one memory latency for four.
+template <typename T>
+__device__ __forceinline__ float2 rope_load(const T* x, bool vec) {
+  if constexpr (sizeof(T) == 4) {
+    return vec ? *reinterpret_cast<const float2*>(x) : make_float2(x[0], x[1]);
+  } else {
+    if (!vec) return make_float2(__bfloat162float(x[0]), __bfloat162float(x[1]));
+    const uint32_t v = *reinterpret_cast<const uint32_t*>(x);
+    return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+  }
+}
+template <typename T>
+__device__ __forceinline__ void rope_store(T* y, float2 x, float cs, float sn, bool vec) {
+  const float o0 = __fmaf_rn(x.x, cs, -__fmul_rn(x.y, sn)), o1 = __fmaf_rn(x.y, cs, __fmul_rn(x.x, sn));
+  if constexpr (sizeof(T) == 4) {
+    if (vec) {
+      *reinterpret_cast<float2*>(y) = make_float2(o0, o1);
+    } else {
+      y[0] = o0;
+      y[1] = o1;
+    }
+  } else if (vec) {
+    *reinterpret_cast<__nv_bfloat162*>(y) = __floats2bfloat162_rn(o0, o1);
+  } else {
+    y[0] = __float2bfloat16_rn(o0);
+    y[1] = __float2bfloat16_rn(o1);
+  }
+}
+template <typename T>
+__device__ __forceinline__ void rope_heads(const T* x, int64_t xs_h, T* y, int64_t ys_h, int H, float cs, float sn,
+                                           bool vec) {
+  for (int h0 = 0; h0 < H; h0 += 4) {
+    float2 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (h0 + i < H) v[i] = rope_load(x + (h0 + i) * xs_h, vec);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (h0 + i < H) rope_store(y + (h0 + i) * ys_h, v[i], cs, sn, vec);
+  }
+}
+// whether every pair of a tensor (element size es, strides of its outer dimensions) lies on a multiple of its size
+inline bool rope_vec_ok(const void* p, int64_t s0, int64_t s1, int64_t s2, int es) {
+  return reinterpret_cast<uintptr_t>(p) % (2 * es) == 0 && s0 % 2 == 0 && s1 % 2 == 0 && s2 % 2 == 0;
 }
 
 }  // namespace swv

@@ -38,6 +38,24 @@ def test_prologue_equals_separate_rope_and_collapse(dtype):
     assert torch.equal(untouched, qkv) and torch.equal(idx2, idx_r) and torch.equal(sc2, sc_r)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H,hd", [(1, 4), (5, 64), (4, 128)])
+def test_rope_of_odd_strides_equals_aligned(dtype, H, hd):
+    """Channel pairs on odd addresses (one element at a time) against the same values on aligned rows, in place
+    and out of place, for head counts around the four that are read at a time: the same bits."""
+    import sparse_wsi_vit_b200 as swv
+    T, C = 131, 3
+    g = torch.Generator().manual_seed(H)
+    x = torch.randn(T, H, hd, generator=g).to(dtype).to(DEV)
+    coords = (torch.rand(T, 2, generator=g) * 50).to(DEV)
+    ref = swv.rope2d(x, coords, 50.0, skip_tokens=C)
+    odd = torch.zeros(T, H, hd + 1, dtype=dtype, device=DEV)[..., 1:]
+    odd.copy_(x)
+    assert torch.equal(swv.rope2d(odd, coords, 50.0, skip_tokens=C), ref)
+    swv.rope2d(odd, coords, 50.0, skip_tokens=C, out=odd)
+    assert torch.equal(odd, ref) and torch.equal(ref[:C], x[:C])
+
+
 def test_inference_module_uses_one_projection_gemm_and_matches_training_path():
     """Without gradients the three Linears run as one GEMM over concatenated weights and the prologue
     launch replaces the separate RoPE / collapse steps; with gradients the module takes the separate,
