@@ -7,7 +7,7 @@ are the library-defined ones frozen in ``oracle/nsa.py`` (parity unpinned).
   selection  : `swv_nsa_select_blocks_fwd`: block importance recomputed on the tensor cores from
                q, the compressed keys and the log-sum-exp, then an arg-max kernel per query;
   selected   : `swv_nsa_selected_attn_fwd`: one warp per (kv group, query) reads each selected
-               key / value row once for all heads of the group (the heads are the rows of
+               key / value row once for all heads of the group (the heads are the columns of
                warp-level tensor-core tiles);
   window     : the block-sparse kernel in token-pattern mode (|i-j| <= window/2);
   gate       : in the one-call form (`swv_nsa_attn_fwd`) every branch kernel applies its sigmoid gate

@@ -1,5 +1,7 @@
 """NSA-style attention (compressed / selected / sliding-window + gate) against the library-defined
 CPU oracle (parity unpinned: the reference has no NSA code)."""
+import math
+
 import pytest
 import torch
 
@@ -111,3 +113,33 @@ def test_selection_on_plateaus_takes_the_lowest_blocks(T):
     # so only the bf16 rounding of the inputs and the fp32 sums are left
     mean = v[0, 0, :min(T, n * 64)].float().mean(0)
     assert (o_sel[0] - mean).abs().max() < 1e-4
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_selected_branch_dominant_key_is_not_rounded(D):
+    """Two keys per query carry all the weight: one in the first selected block, a larger one (by x = 0.3 .. 5
+    in the log2 domain) in the last.  P is rounded to bf16 relative to the row's maximum, so the larger key's
+    probability is exactly 1 and only the smaller one's rounding (2^-9 of it) is left, beside the 2^-22 of the
+    approximate exponential and the fp32 sums: |error| <= 2^-9 w_small |v_small| + 2^-18 max|v|, w = its weight."""
+    from sparse_wsi_vit_b200.nsa import selected_attention
+    R, blk = 64, 64
+    T = 4 * blk
+    g = torch.Generator().manual_seed(D)
+    k = torch.zeros(1, 1, T, D)
+    k[..., 0] = -64.0                                     # every other key: weight 2^-60 and less
+    k[0, 0, 3] = 0.0
+    k[0, 0, 3, 1] = 1.0                                   # logit of the small key: channel 1 of the query
+    k[0, 0, 200] = 0.0
+    k[0, 0, 200, 2] = 1.0                                 # of the large key: channel 2
+    x = torch.linspace(0.3, 5.0, R) * D ** 0.5 * math.log(2.0)
+    q = torch.zeros(1, 1, R, D)
+    q[..., 0], q[0, 0, :, 2] = D ** 0.5, x
+    q, k = q.to(torch.bfloat16), k.to(torch.bfloat16)
+    v = torch.randn(1, 1, T, D, generator=g).to(torch.bfloat16)
+    blocks = torch.tensor([0, 1, 3], dtype=torch.int32).repeat(R, 1)[None, None]
+    o = selected_attention(q.to(DEV), k.to(DEV), v.to(DEV), blocks.to(DEV), blk)[0, 0].cpu().double()
+    keys = torch.cat([torch.arange(b * blk, (b + 1) * blk) for b in (0, 1, 3)])
+    w = torch.softmax(q[0, 0].double() @ k[0, 0, keys].double().T / D ** 0.5, dim=1)
+    vd = v[0, 0].double()
+    bound = 2.0 ** -9 * w[:, 3:4] * vd[3].abs() + 2.0 ** -18 * vd.abs().max()
+    assert bool(((o - w @ vd[keys]).abs() <= bound).all())
