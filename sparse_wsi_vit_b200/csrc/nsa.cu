@@ -237,8 +237,9 @@ __global__ void __launch_bounds__(320, 2)
 }
 
 // ------------------------------------------------------------------- select
-// One warp per (b, g, t).  Importance values are >= 0; entries behind the last selection block count as
-// -2.  Ties go to the lower block index; output ascending.
+// One warp per (b, g, t).  Importance values are >= 0 (a NaN counts as 0, so that every row has its k_eff
+// blocks); entries behind the last selection block count as -2.  Ties go to the lower block index; output
+// ascending.
 //
 // Short form (k_eff <= 32, at most 32 * NPL blocks, the row in registers, entry i * 32 + lane): the
 // k-th largest of the 32 lane maxima is a lower bound of the k-th largest entry, and on real rows only a
@@ -248,6 +249,12 @@ __global__ void __launch_bounds__(320, 2)
 // kv heads, 1024 blocks: 0.64 -> 0.17 ms).
 constexpr int kSelCand = 64;
 
+// entry e of an importance row: blocks without compressed tokens (e >= n_pad) have none
+__device__ __forceinline__ float nsa_importance(const float* src, int e, int n_pad, int n_s) {
+  return e >= n_s ? -2.f : e < n_pad ? fmaxf(__ldg(src + e), 0.f) : 0.f;
+}
+
+// (every row holds at least k_eff values >= 0)
 __device__ __forceinline__ void nsa_argmax_loop(float* v, int n, int k_eff, int lane, int32_t* dst) {
   for (int s = 0; s < k_eff; ++s) {
     float best = -3.f;
@@ -293,8 +300,7 @@ __global__ void __launch_bounds__(128) nsa_select_short_kernel(const float* __re
   float mx = -2.f;
 #pragma unroll
   for (int i = 0; i < NPL; ++i) {
-    const int e = i * 32 + lane;
-    v[i] = e < n_s ? (e < n_pad ? __ldg(src + e) : 0.f) : -2.f;
+    v[i] = nsa_importance(src, i * 32 + lane, n_pad, n_s);
     mx = fmaxf(mx, v[i]);
   }
   // the k-th largest lane maximum: the one whose rank (ties by lane) is k - 1
@@ -359,7 +365,7 @@ __global__ void __launch_bounds__(128) nsa_select_kernel(const float* __restrict
   const int n = (n_s + 31) & ~31;                     // scanned range, a multiple of 32
   float* v = sel_sm + wib * n;
   const float* src = imp + r * n_pad;
-  for (int i = lane; i < n; i += 32) v[i] = i < n_s ? (i < n_pad ? src[i] : 0.f) : -2.f;
+  for (int i = lane; i < n; i += 32) v[i] = nsa_importance(src, i, n_pad, n_s);
   __syncwarp();
   nsa_argmax_loop(v, n, k_eff, lane, blocks + r * k_eff);
 }
@@ -376,9 +382,14 @@ struct NsaSelParams {
   // Gated form (whole-pass call): o is the running gated sum of the branches and this branch adds
   // sigmoid(gate[b,t,h,1]) * (its rows) to it; gate (B,Tq,Hq,3) fp32, null = plain store.
   const float* gate;
-  int B, Hq, Hkv, G, Tq, Tk, n_sel, sel_block;
+  int B, Hq, Hkv, G, Tq, Tk, n_sel, sel_block, n_blk;      // n_blk: blocks the keys fill
   float scale_log2;
 };
+
+// First key of a listed block; an index outside the keys counts as the block behind them (no key attended).
+__device__ __forceinline__ int nsa_block_key0(const NsaSelParams& p, int blk) {
+  return min(static_cast<uint32_t>(blk), static_cast<uint32_t>(p.n_blk)) * p.sel_block;
+}
 
 template <int D, int GMAX>
 __global__ void __launch_bounds__(128) nsa_selected_attn_kernel(const NsaSelParams p) {
@@ -415,7 +426,7 @@ __global__ void __launch_bounds__(128) nsa_selected_attn_kernel(const NsaSelPara
 
   const int chunks_per_block = p.sel_block / 32;
   for (int s = 0; s < p.n_sel; ++s) {
-    const int key_block0 = blk[s] * p.sel_block;
+    const int key_block0 = nsa_block_key0(p, blk[s]);
     for (int c = 0; c < chunks_per_block; ++c) {
       const int key = key_block0 + c * 32 + lane;
       const bool ok = key < p.Tk;
@@ -613,7 +624,7 @@ __global__ void __launch_bounds__(32 * NsaSelCfg<D>::kWarps, 1)
   auto issue = [&](int which, int stage) {                   // which: 0 = K, 1 = V
     Stream& x = str[which];
     if (x.row < total) {
-      const int key0 = x.blk * p.sel_block + x.in_block * Cfg::kStep;
+      const int key0 = nsa_block_key0(p, x.blk) + x.in_block * Cfg::kStep;
       const int64_t rs = which ? p.vs[2] : p.ks[2];
       const uint32_t dst = cdst + (which * 2 + stage) * Cfg::kStageBytes;
       if (key0 + Cfg::kStep <= p.Tk) {
@@ -668,7 +679,7 @@ __global__ void __launch_bounds__(32 * NsaSelCfg<D>::kWarps, 1)
     for (int n = 0; n < D / 16; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
     float m[2] = {ninf, ninf}, l[2] = {0.f, 0.f};            // heads 2 t4, 2 t4 + 1
     const int32_t* list = p.blocks + r * p.n_sel;
-    int key0 = __ldg(list) * p.sel_block, in_block = 0;
+    int key0 = nsa_block_key0(p, __ldg(list)), in_block = 0;
     int blk_next = p.n_sel > 1 ? __ldg(++list) : 0;          // (loaded a block ahead of its use)
     for (int step = 0; step < n_steps; ++step, ++it) {
       const int stage = it & 1;
@@ -769,7 +780,7 @@ __global__ void __launch_bounds__(32 * NsaSelCfg<D>::kWarps, 1)
       key0 += Cfg::kStep;
       if (++in_block == steps_per_block) {
         in_block = 0;
-        key0 = blk_next * p.sel_block;
+        key0 = nsa_block_key0(p, blk_next);
         if (step + 1 + steps_per_block < n_steps) blk_next = __ldg(++list);
       }
     }
@@ -942,6 +953,7 @@ int nsa_selected_attn_impl(const void* q, const int64_t* qs, const void* k, cons
   for (int i = 0; i < 4; ++i) { p.qs[i] = qs[i]; p.ks[i] = ks[i]; p.vs[i] = vs[i]; }
   p.blocks = blocks; p.o = o; p.gate = gate;
   p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.G = G; p.Tq = Tq; p.Tk = Tk; p.n_sel = n_sel; p.sel_block = sel_block;
+  p.n_blk = (Tk + sel_block - 1) / sel_block;
   p.scale_log2 = 1.4426950408889634f / sqrtf(static_cast<float>(D));
   const int64_t total = static_cast<int64_t>(B) * Hkv * Tq;
   const unsigned grid = static_cast<unsigned>((total + 3) / 4);

@@ -143,3 +143,46 @@ def test_selected_branch_dominant_key_is_not_rounded(D):
     vd = v[0, 0].double()
     bound = 2.0 ** -9 * w[:, 3:4] * vd[3].abs() + 2.0 ** -18 * vd.abs().max()
     assert bool(((o - w @ vd[keys]).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("T,topk", [(3000, 16), (16384, 16), (4000, 40), (66000, 16)])
+def test_selection_with_nan_rows_lists_valid_blocks(T, topk):
+    """A NaN query (its own row) and a NaN key (every row): NaN importances count as 0, so each row still lists
+    k_eff ascending blocks of the sequence, the lowest ones of a row without any other importance.  Block counts
+    with and without padding entries in the short form's registers, and both ways to the arg-max loop."""
+    import sparse_wsi_vit_b200 as swv
+    from sparse_wsi_vit_b200.nsa import nsa_attention
+    g = torch.Generator().manual_seed(T)
+    q, k, v = (torch.randn(1, h, T, 64, generator=g).to(torch.bfloat16).to(DEV) for h in (2, 1, 1))
+    gate = torch.zeros(1, T, 2, 3, device=DEV)
+    n = -(-T // 64)
+    run = lambda q, k: nsa_attention(q, k, v, gate, sel_topk=topk, window=128, return_parts=True)
+    blocks = run(q, k)[4]
+    q1 = q.clone()
+    q1[:, :, 7] = float("nan")
+    got, lowest = run(q1, k), torch.arange(min(topk, n), device=DEV)
+    assert torch.equal(got[4][0, 0, 7], lowest.int()) and bool(got[2][0, :, 7].isnan().all())
+    keep = torch.arange(T, device=DEV) != 7
+    assert torch.equal(got[4][:, :, keep], blocks[:, :, keep])
+    k1 = k.clone()
+    k1[:, :, T // 2] = float("nan")
+    b = run(q, k1)[4]
+    swv.check_status(DEV)
+    assert bool((b[..., 1:] > b[..., :-1]).all()) and int(b.min()) >= 0 and int(b.max()) < n
+
+
+@pytest.mark.parametrize("aligned", [True, False])
+def test_selected_branch_ignores_blocks_outside_the_keys(aligned):
+    """Block indices below 0 and behind the last block attend nothing and nothing is read through them, on
+    tensor-core tiles and (odd query strides) on CUDA cores."""
+    from sparse_wsi_vit_b200.nsa import selected_attention
+    T, D = 300, 64
+    g = torch.Generator().manual_seed(8)
+    q = torch.randn(1, 4, T, D + 1, generator=g).to(torch.bfloat16).to(DEV)[..., :D]
+    k, v = (torch.randn(1, 2, T, D, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
+    q = q.contiguous() if aligned else q
+    run = lambda blocks: selected_attention(q, k, v, torch.tensor(blocks, dtype=torch.int32, device=DEV).repeat(2, T, 1)[None], 64)
+    want = run([1, 4])
+    assert torch.isfinite(want).all()
+    for blocks in ([1, 4, -1, 5, -2 ** 31, 2 ** 31 - 1], [-7, 1, 9, 4, 6, 2 ** 30]):
+        assert torch.equal(run(blocks), want)
