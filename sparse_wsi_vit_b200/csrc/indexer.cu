@@ -1244,13 +1244,20 @@ __global__ void __launch_bounds__(NT) dsa_select_dense_kernel(const DenseSelectP
     return;
   }
   const int64_t row = static_cast<int64_t>(b) * p.Tq + t;
-  // the row, its largest value and how many of its scores are above zero (the padding columns are zero)
+  // the row, its largest value and how many of its scores are above zero; the columns behind the keys become
+  // zero (they hold the products with zero vectors, which are NaN where a query is infinite)
   uint32_t vmax = 0, nz = 0;
   {
     const uint4* src = reinterpret_cast<const uint4*>(p.dense + static_cast<int64_t>(blockIdx.x) * n_pad);
 #pragma unroll 4
     for (int i4 = tid; i4 < n_pad / 4; i4 += NT) {
-      const uint4 x = __ldg(src + i4);
+      uint4 x = __ldg(src + i4);
+      if (i4 * 4 + 4 > n) {
+        if (i4 * 4 >= n) x.x = 0u;
+        if (i4 * 4 + 1 >= n) x.y = 0u;
+        if (i4 * 4 + 2 >= n) x.z = 0u;
+        x.w = 0u;
+      }
       reinterpret_cast<uint4*>(sc_s)[i4] = x;
       vmax = max(max(vmax, max(x.x, x.y)), max(x.z, x.w));
       nz += (x.x != 0u) + (x.y != 0u) + (x.z != 0u) + (x.w != 0u);

@@ -516,6 +516,30 @@ def test_dense_selection_equals_the_sweeps(swv, B, Tq, Tk, K, ID, ties, want_mas
         assert x is None or torch.equal(x, y), name
 
 
+@pytest.mark.parametrize("Tq,Tk,K", [(5, 1, 4), (129, 129, 128), (40, 1021, 700), (300, 640, 500), (130, 4097, 3000)])
+def test_dense_selection_of_infinite_and_nan_rows(swv, Tq, Tk, K):
+    """Queries of +-inf and NaN and a NaN key: the columns behind the last key (products with zero vectors, NaN
+    for an infinite query) are no keys, so every slot below min(K, Tk) is written, ascending and in range, as the
+    sweeps list them (bit patterns of the scores in order, ties to the lower key)."""
+    g = torch.Generator().manual_seed(Tk)
+    qi, ki = (torch.randn(1, n, 2, 32, generator=g).to(torch.bfloat16) for n in (Tq, Tk))
+    qi[0, 0, 0, 3], qi[0, 1, 1, 3], qi[0, 2, 0, 3], qi[0, 3] = float("inf"), -float("inf"), float("nan"), 0.0
+    if Tk > 600:
+        ki[0, Tk - 2, 0, 0] = float("nan")
+    qi, ki, w = qi.to(_dev()), ki.to(_dev()), torch.tensor([1.0, 0.5], device=_dev())
+    n, res = min(K, Tk), []
+    for nbytes in (swv.ops.workspace_bytes(1, Tq, Tk), swv.ops.workspace_bytes(1, Tq, Tk, K)):
+        out = tuple(torch.full((1, Tq, K), -7, dtype=t, device=_dev()) for t in (torch.int32, torch.float32, torch.float32))
+        ws = torch.full((nbytes,), 255, dtype=torch.uint8, device=_dev())
+        swv.dsa_indexer_topk(qi, ki, w, K, out=out, workspace=ws)
+        _check(swv)
+        idx = out[0][0, :, :n]
+        assert bool((idx[:, 1:] > idx[:, :-1]).all()) and int(idx.min()) >= 0 and int(idx.max()) < Tk
+        res.append((out[0], out[1], out[2].view(torch.int32)))
+    for name, x, y in zip(("idx", "valid", "scores"), *res):
+        assert torch.equal(x, y), name
+
+
 @pytest.mark.parametrize("D,K,Tk,kvg", [(32, 1, 40, 1), (64, 257, 300, 3), (128, 300, 129, 1), (64, 31, 77, 1)])
 def test_gather_fp32_rows_vs_general_kernel(swv, D, K, Tk, kvg):
     """fp32 rows of 16-byte chunks against the lane-per-row kernel (which unaligned rows take), on any-order
