@@ -772,6 +772,8 @@ __global__ void __launch_bounds__(576, 1)
       const bool warp_partial = __any_sync(0xffffffffu, partial);
       const uint32_t thr_min = partial ? thr + 1u : thr;        // member iff bits >= thr_min (+ chosen ties)
       const int thr_signed = thr_min == 0u ? static_cast<int>(0x80000000u) : static_cast<int>(thr_min);
+      // (cut ties at the largest pattern, a row of NaN scores: no score lies above the threshold)
+      const uint32_t above = thr_min == 0x80000000u ? 0u : 0xFFFFFFFFu;
       // A second part starts behind part 0's share of the row: the keys above the threshold in part
       // 0's range plus the ties part 0 takes (ties are taken in ascending key order).
       uint32_t eq_seen = 0;
@@ -863,6 +865,7 @@ __global__ void __launch_bounds__(576, 1)
             w &= vm;
             e &= vm;
           }
+          w &= above;
         }
         const uint32_t x = xchg + static_cast<uint32_t>((a * kTile + row) * 4) * 8u;
         sts64(x + ch * 8, w, e);

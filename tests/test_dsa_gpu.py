@@ -530,13 +530,16 @@ def test_dense_selection_of_infinite_and_nan_rows(swv, Tq, Tk, K):
     n, res = min(K, Tk), []
     for nbytes in (swv.ops.workspace_bytes(1, Tq, Tk), swv.ops.workspace_bytes(1, Tq, Tk, K)):
         out = tuple(torch.full((1, Tq, K), -7, dtype=t, device=_dev()) for t in (torch.int32, torch.float32, torch.float32))
+        mask = torch.zeros(swv.ops.mask_bytes(1, Tq, Tk) // 4, dtype=torch.int32, device=_dev())
         ws = torch.full((nbytes,), 255, dtype=torch.uint8, device=_dev())
-        swv.dsa_indexer_topk(qi, ki, w, K, out=out, workspace=ws)
+        swv.dsa_indexer_topk(qi, ki, w, K, want_mask=True, out=out, mask=mask, workspace=ws)
         _check(swv)
         idx = out[0][0, :, :n]
         assert bool((idx[:, 1:] > idx[:, :-1]).all()) and int(idx.min()) >= 0 and int(idx.max()) < Tk
-        res.append((out[0], out[1], out[2].view(torch.int32)))
-    for name, x, y in zip(("idx", "valid", "scores"), *res):
+        nqt, nkt = -(-Tq // 128), -(-Tk // 128)
+        bits = mask.reshape(nqt, nkt, 128, 4).permute(0, 2, 1, 3).reshape(nqt * 128, nkt * 4)[:Tq]
+        res.append((out[0], out[1], out[2].view(torch.int32), bits))
+    for name, x, y in zip(("idx", "valid", "scores", "bitmask"), *res):
         assert torch.equal(x, y), name
 
 
