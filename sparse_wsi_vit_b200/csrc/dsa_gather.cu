@@ -111,9 +111,9 @@ __global__ void __launch_bounds__(128) dsa_attn_gather_kernel(const GatherParams
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) gm = fmaxf(gm, __shfl_xor_sync(0xffffffffu, gm, off));
     const float m_new = fmaxf(m, gm);
-    if (m_new == ninf) continue;   // no valid slot so far (uniform across the warp)
     const float alpha = (m == m_new) ? 1.f : expf(m - m_new);
-    float pj = ok ? expf(logit - m_new) * w : 0.f;
+    // (no logit above -inf so far: those are zero, a NaN stays NaN)
+    float pj = ok ? expf(logit - (m_new == ninf ? 0.f : m_new)) * w : 0.f;
     float ps = pj;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, off);
@@ -290,11 +290,12 @@ __global__ void __launch_bounds__(256) dsa_attn_gather_rows_kernel(const GatherP
         }
         m = cmax;
       }
-      if (m == ninf) continue;                           // no finite logit so far
+      // no logit above -inf so far: fp32 rows count those as zero like the kernel above; a NaN stays NaN
+      const float m_sub = F32 && m == ninf ? 0.f : m;
 #pragma unroll
       for (int s_ = 0; s_ < STEPS; ++s_) {
         const int id = ids[s_];
-        const float pj = id >= 0 ? exp_(logit[s_] - m) * s_w[c0 + s_ * G + grp] : 0.f;
+        const float pj = id >= 0 ? exp_(logit[s_] - m_sub) * s_w[c0 + s_ * G + grp] : 0.f;
         if (pj != 0.f) {                                  // uniform within the lane group
           if (chunk == 0) l += pj;
           const uint4 vv = __ldg(reinterpret_cast<const uint4*>(vbase + static_cast<int64_t>(id) * p.vs[2]) + chunk);

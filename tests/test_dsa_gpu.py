@@ -564,3 +564,32 @@ def test_gather_fp32_rows_vs_general_kernel(swv, D, K, Tk, kvg):
     _check(swv)
     assert float(o[:, :, 3].abs().max()) == 0
     assert float((o - o2).abs().max()) < 2.0 ** -20 * float(o2.abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_gather_keeps_nan(swv, D, dtype, aligned):
+    """A NaN query (every logit NaN) and lists that begin with 32 times a NaN key: those rows come out NaN in every
+    channel, from the row kernel and (odd strides) the lane-per-row kernel; the others do not notice."""
+    Tq, Tk, K = 20, 90, 70
+    g = torch.Generator().manual_seed(D)
+    q, k, v = (torch.randn(1, 2, n, D + 1, generator=g).to(dtype).to(_dev())[..., :D] for n in (Tq, Tk, Tk))
+    if aligned:
+        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+    idx = torch.randint(1, Tk, (1, Tq, K), generator=g, dtype=torch.int32).to(_dev())
+    valid = torch.ones(1, Tq, K, device=_dev())
+    valid[:, 5, ::3] = 0
+    rw = torch.rand(1, Tq, K, generator=g).to(_dev()) + 0.1
+    clean = torch.empty(1, 2, Tq, D, device=_dev())
+    swv.dsa_attention_gather(q, k, v, idx, valid, rw, clean)
+    assert torch.isfinite(clean).all()
+    q[:, :, 5] = float("nan")
+    k[:, :, 0] = float("nan")
+    idx[:, 9, :32] = 0
+    o = torch.empty_like(clean)
+    swv.dsa_attention_gather(q, k, v, idx, valid, rw, o)
+    _check(swv)
+    assert bool(o[:, :, [5, 9]].isnan().all())
+    keep = [i for i in range(Tq) if i not in (5, 9)]
+    assert torch.equal(o[:, :, keep], clean[:, :, keep])
