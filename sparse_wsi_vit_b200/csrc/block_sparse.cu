@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(kBsaThreads, BsaCfg<BS, D>::kCtas)
         for (int c = 0; c < nch; ++c) {
           const int64_t u = bh * units + (c == 0 ? qb : p.nQB + ubase + c - 1);
           const float2 ml = __ldcg(p.part_ml + u * BS + row);
-          if (ml.x != ninf) l += ml.y * ex2_approx(ml.x - wgt_m);
+          l += ml.y * (ml.x == wgt_m ? 1.f : ex2_approx(ml.x - wgt_m));    // (a chunk without keys: 0 * 0)
         }
       }
       const float inv = l > 0.f ? 1.f / l : 0.f;
@@ -527,8 +527,7 @@ __global__ void __launch_bounds__(kBsaThreads, BsaCfg<BS, D>::kCtas)
           for (int k = 0; row_ok && k < nch; ++k) {
             const int64_t u = bh * units + (k == 0 ? qb : p.nQB + ubase + k - 1);
             const float mk = __ldcg(p.part_ml + u * BS + row).x;
-            if (mk == ninf) continue;
-            const float f = ex2_approx(mk - wgt_m);
+            const float f = mk == wgt_m ? 1.f : ex2_approx(mk - wgt_m);    // (no chunk is left out: a NaN stays NaN)
             const float4* po = reinterpret_cast<const float4*>(p.part_o + (u * BS + row) * D + c * 16);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {

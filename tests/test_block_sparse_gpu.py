@@ -78,6 +78,39 @@ def test_long_lists_are_divided(swv, nb, D, block, long_rows):
     assert (again[1][0].cpu() - ref)[:, seen].abs().max() < 1e-3
 
 
+@pytest.mark.parametrize("mode,block,D", [(0, 64, 64), (1, 128, 64), (1, 64, 128), (0, 128, 128)])
+def test_divided_lists_batch_groups_and_nan(swv, mode, block, D):
+    """Divided lists in a batch, with grouped queries and with the token pattern; then a NaN query in a long list
+    (every chunk of its row is NaN with a stabiliser of -inf): the row comes out NaN as from one sweep, the
+    others do not notice."""
+    B, H, G, nb = 2, 4, 2, 30
+    T = nb * block - 21
+    if mode:
+        rp, ci = swv.patterns.static_window_blocks(T, 3, 5, 2, block)
+    else:
+        rp, ci = swv.patterns._to_csr([range(nb) if r == 0 else [r] for r in range(nb)])
+    g = torch.Generator().manual_seed(block + D)
+    q = torch.randn(B, H, T, D, generator=g).to(torch.bfloat16)
+    k, v = (torch.randn(B, H // G, T, D, generator=g).to(torch.bfloat16) for _ in range(2))
+    kw = dict(mode=mode, num_cls=3, window=5, dilation=2) if mode else {}
+    run = lambda q: swv.block_sparse_attention(*_dev(q, k, v), torch.from_numpy(rp).to(DEV), torch.from_numpy(ci).to(DEV),
+                                               block, out_dtype=torch.float32, kv_group=G, return_lse=True, **kw)
+    o, lse = run(q)
+    mask = S.static_window_mask(T, 3, 5, 2) if mode else S.expand_block_mask(rp, ci, block, T, T, rows=None)
+    for b in range(B):
+        ref = S.masked_attention(q[b].float(), k[b].float().repeat_interleave(G, 0), v[b].float().repeat_interleave(G, 0), mask)
+        diff = (o[b].cpu() - ref).abs()
+        assert diff.max() < 2e-2 and diff.mean() < 1e-3
+    q1 = q.clone()
+    q1[1, 2, 1] = float("nan")
+    o1, lse1 = run(q1)
+    swv.check_status(DEV)
+    assert bool(o1[1, 2, 1].isnan().all())
+    keep = torch.ones(B, H, T, dtype=torch.bool, device=DEV)
+    keep[1, 2, 1] = False
+    assert torch.equal(o1[keep], o[keep]) and torch.equal(lse1[keep], lse[keep])
+
+
 def test_empty_rows_and_full_list(swv):
     T, H, D, block = 512, 2, 64, 128
     q, k, v = _qkv(T, H, D, seed=3)
