@@ -32,6 +32,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace swv {
@@ -40,7 +42,7 @@ struct BsaParams {
   int B, H, Tq, Tk, nQB;
   const int32_t* row_ptr;   // [nQB + 1]
   const int32_t* col_idx;   // [nnz] key block index
-  int mode, num_cls, window, dilation;
+  int mode, num_cls, reach, dilation;   // reach = window * dilation, at most Tq + Tk
   int kv_group;             // query heads per key/value head (grouped-query attention), >= 1
   float* lse;               // optional (B,H,Tq): natural-log sum of exponentials per row, -inf for empty rows
   // Optional gated epilogue (the NSA branches): the rows are scaled by sigmoid(gate[b,t,h,gate_idx])
@@ -362,7 +364,7 @@ __global__ void __launch_bounds__(kBsaThreads, BsaCfg<BS, D>::kCtas)
     const uint32_t o_col = s_col + Cfg::kColO;
     const float sc = p.scale_log2;
     const float ninf = -__int_as_float(0x7f800000);
-    const int reach = p.window * p.dilation;
+    const int reach = p.reach;
     const int dil = p.dilation > 0 ? p.dilation : 1;
 
     float m_used = ninf;
@@ -750,7 +752,9 @@ int block_sparse_attn_impl(const void* q, const int64_t* qs, const void* k, cons
   p.B = B; p.H = H; p.Tq = Tq; p.Tk = Tk;
   p.nQB = (Tq + block - 1) / block;
   p.row_ptr = row_ptr; p.col_idx = col_idx;
-  p.mode = mode; p.num_cls = num_cls; p.window = window; p.dilation = dilation;
+  p.mode = mode; p.num_cls = num_cls; p.dilation = dilation;
+  // (the bound keeps every sum of a position and the reach within 32 bits)
+  p.reach = static_cast<int>(std::min<int64_t>(static_cast<int64_t>(window) * dilation, static_cast<int64_t>(Tq) + Tk));
   p.kv_group = kv_group; p.lse = lse;
   p.gate = gate; p.gate_idx = gate_idx; p.acc_in = acc_in;
   p.o = o; p.osb = os[0]; p.osh = os[1]; p.ost = os[2]; p.o_dtype = o_dtype;

@@ -111,6 +111,19 @@ def test_divided_lists_batch_groups_and_nan(swv, mode, block, D):
     assert torch.equal(o1[keep], o[keep]) and torch.equal(lse1[keep], lse[keep])
 
 
+def test_window_beyond_32_bits_sees_everything_in_reach(swv):
+    """window * dilation past the range of an int: the reach is bounded by the sequence, not wrapped."""
+    T = 300
+    q, k, v = _qkv(T, 2, 64, seed=12)
+    rp, ci = swv.patterns._to_csr([range(3)] * 3)
+    lists = _dev(torch.from_numpy(rp), torch.from_numpy(ci))
+    run = lambda w, d: swv.block_sparse_attention(*_dev(q, k, v), *lists, 128, mode=1, num_cls=1, window=w, dilation=d)
+    assert torch.equal(run(2 ** 31 - 1, 1), run(T, 1))
+    assert torch.equal(run(2 ** 20, 2 ** 12), run(1, 2 ** 12))
+    assert torch.equal(run(2 ** 30, 3), run(T, 3))
+    swv.check_status(DEV)
+
+
 def test_empty_rows_and_full_list(swv):
     T, H, D, block = 512, 2, 64, 128
     q, k, v = _qkv(T, H, D, seed=3)
