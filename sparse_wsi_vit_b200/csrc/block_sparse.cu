@@ -57,11 +57,12 @@ struct BsaParams {
   float scale_log2;
   // Long lists: a query block with more than `chunk` key blocks is divided over ceil(n / chunk) CTAs
   // (chunk = 0: never).  The first `extra` CTAs of every (batch, head) serve the second and later
-  // chunks.  Partial rows go to `part_o` / `part_ml` (indexed by the chunk's unit), the CTA that
-  // takes the last ticket of the row block adds them up.
+  // chunks.  Partial rows go to `part_o` / `part_ml`, a later chunk's to the slot of its extra unit, the
+  // first chunk's to slot extra + (its list's first extra unit); the CTA that takes the last ticket of the
+  // row block adds them up.
   int chunk, extra;
-  float* part_o;            // [B*H][nQB + extra][BS rows][D] unnormalised fp32 rows
-  float2* part_ml;          // [B*H][nQB + extra][BS rows] (stabiliser, probability sum)
+  float* part_o;            // [B*H][2 * extra][BS rows][D] unnormalised fp32 rows
+  float2* part_ml;          // [B*H][2 * extra][BS rows] (stabiliser, probability sum)
   uint32_t* tickets;        // [B*H][nQB], zero before the launch
   int* status;
 };
@@ -231,7 +232,8 @@ __global__ void __launch_bounds__(kBsaThreads, BsaCfg<BS, D>::kCtas)
     const int a = static_cast<int>(static_cast<int64_t>(nblk) * ch / nch);
     const int z = static_cast<int>(static_cast<int64_t>(nblk) * (ch + 1) / nch);
     // A later chunk looks at the list's first block before its own: it starts from the same stabiliser
-    // as the first chunk, so its probabilities round to bf16 exactly as they would in one sweep.
+    // as the first chunk, so its probabilities round to bf16 as they would in one sweep unless a block
+    // between the two would have raised it.
     peek = ch > 0;
     first_blk = list0;
     list0 += a - (peek ? 1 : 0);
@@ -475,10 +477,10 @@ __global__ void __launch_bounds__(kBsaThreads, BsaCfg<BS, D>::kCtas)
 
     // One chunk of a long list: leave the unnormalised rows, take a ticket; the last CTA of the query
     // block goes on with the sum over all chunks.
-    const int64_t units = p.nQB + p.extra;
+    auto slot = [&](int c) { return (bh * 2 + (c == 0)) * static_cast<int64_t>(p.extra) + ubase + (c == 0 ? 0 : c - 1); };
     bool writer = true;
     if (nch > 1) {
-      const int64_t u = bh * units + (ch == 0 ? qb : p.nQB + ubase + ch - 1);
+      const int64_t u = slot(ch);
       if (ok) {
         if (row_ok) p.part_ml[u * BS + row] = make_float2(m_used, l);
         float* po = p.part_o + (u * BS + row) * D;
@@ -504,12 +506,12 @@ __global__ void __launch_bounds__(kBsaThreads, BsaCfg<BS, D>::kCtas)
       float wgt_m = m_used;
       if (nch > 1 && row_ok) {
         for (int c = 0; c < nch; ++c) {
-          const int64_t u = bh * units + (c == 0 ? qb : p.nQB + ubase + c - 1);
+          const int64_t u = slot(c);
           wgt_m = fmaxf(wgt_m, __ldcg(p.part_ml + u * BS + row).x);
         }
         l = 0.f;
         for (int c = 0; c < nch; ++c) {
-          const int64_t u = bh * units + (c == 0 ? qb : p.nQB + ubase + c - 1);
+          const int64_t u = slot(c);
           const float2 ml = __ldcg(p.part_ml + u * BS + row);
           l += ml.y * (ml.x == wgt_m ? 1.f : ex2_approx(ml.x - wgt_m));    // (a chunk without keys: 0 * 0)
         }
@@ -527,7 +529,7 @@ __global__ void __launch_bounds__(kBsaThreads, BsaCfg<BS, D>::kCtas)
 #pragma unroll
           for (int i = 0; i < 16; ++i) acc[i] = 0.f;
           for (int k = 0; row_ok && k < nch; ++k) {
-            const int64_t u = bh * units + (k == 0 ? qb : p.nQB + ubase + k - 1);
+            const int64_t u = slot(k);
             const float mk = __ldcg(p.part_ml + u * BS + row).x;
             const float f = mk == wgt_m ? 1.f : ex2_approx(mk - wgt_m);    // (no chunk is left out: a NaN stays NaN)
             const float4* po = reinterpret_cast<const float4*>(p.part_o + (u * BS + row) * D + c * 16);
@@ -699,7 +701,7 @@ static BsaSplit bsa_split(int B, int H, int nQB, int nKB, int block, int D, int6
   s.chunk = static_cast<int>(chunk);
   s.extra = static_cast<int>(nnz / chunk);          // sum over rows of ceil(n / chunk) - 1 <= nnz / chunk
   if (s.extra == 0) s.chunk = 0;
-  const size_t rows = static_cast<size_t>(B) * H * (nQB + s.extra) * block;
+  const size_t rows = static_cast<size_t>(B) * H * 2 * s.extra * block;     // (a divided list has an extra unit or more)
   s.o_bytes = rows * D * sizeof(float);
   s.ml_bytes = rows * sizeof(float2);
   s.ticket_bytes = static_cast<size_t>(B) * H * nQB * sizeof(uint32_t);

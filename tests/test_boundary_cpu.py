@@ -76,6 +76,12 @@ def test_size_queries(swv):
     assert topk_extra(300000, 8192) == 0                               # beyond 262144 keys
     assert L.swv_dsa_workspace_bytes_topk(1, 1, 1, 0, ctypes.byref(n)) == -4
     assert L.swv_dsa_workspace_bytes_topk(1, 1, 1, 1, None) == -1
+    # divided block lists: partial rows of the divided lists only.  512 blocks of 128, six a list and one list of
+    # all 512: at most nnz / chunk extra units (chunk >= the even share of all work), two slots each
+    nnz = 512 * 6 - 6 + 506
+    assert L.swv_block_sparse_workspace_bytes(1, 16, 65536, 65536, 128, 128, nnz, ctypes.byref(n)) == 0
+    assert 0 < n.value <= 16 * (2 * 20 * 128 * (128 * 4 + 8) + 512 * 4)
+    assert L.swv_block_sparse_workspace_bytes(1, 16, 65536, 65536, 128, 128, 0, ctypes.byref(n)) == 0 and n.value == 0
     # NSA sizes
     assert L.swv_nsa_importance_bytes(1, 2, 65536, 4095, 16, 64, ctypes.byref(n)) == 0
     assert n.value == 2 * 65536 * 1024 * 4
