@@ -19,7 +19,6 @@ import torch
 from . import _lib
 from ._lib import SwvError, check, dtype_code, lib, strides
 
-_scratch: dict = {}
 _status: dict = {}
 _CHECK = os.environ.get("SWV_CHECK_STATUS", "0") == "1"
 
@@ -51,13 +50,10 @@ def check_status(dev, what="kernel"):
         raise SwvError(f"{what}: {_lib.strerror(code)} (device status {code})")
 
 
-def _buffer(kind, dev, nbytes):
-    key = (kind, dev.index)
-    buf = _scratch.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(int(nbytes), dtype=torch.uint8, device=dev)
-        _scratch[key] = buf
-    return buf
+def _workspace(dev, nbytes):
+    """Device memory of one call.  The caching allocator reuses it in the order of the stream it was allocated
+    on, so calls on other streams or threads never share it."""
+    return torch.empty(int(nbytes), dtype=torch.uint8, device=dev)
 
 
 def workspace_bytes(B, Tq, Tk, top_k=None):
@@ -91,7 +87,7 @@ def dsa_prologue(qkv_q, qkv_k, q_idx, k_idx, w, coords=None, coord_high=1.0, the
     if k_idx.dtype != q_idx.dtype:
         k_idx = k_idx.to(q_idx.dtype)
     dev = q_idx.device
-    ws = torch.empty(workspace_bytes(B, T, T, top_k), dtype=torch.uint8, device=dev)
+    ws = _workspace(dev, workspace_bytes(B, T, T, top_k))
     w32 = w.detach().to(torch.float32).contiguous()
     cptr, qp, kp, qs, ks, qdt, H, D = None, None, None, None, None, 0, 1, 4
     if coords is not None:
@@ -136,11 +132,7 @@ def dsa_indexer_topk(q_idx, k_idx, w, top_k, want_mask=False, out=None, mask=Non
     else:
         idx, valid, scores = out
     nws = workspace_bytes(B, Tq, Tk, top_k)
-    # a selection handle keeps its own workspace (the attention reads it); plain calls share one
-    if workspace is not None:
-        ws = workspace
-    else:
-        ws = torch.empty(nws, dtype=torch.uint8, device=dev) if want_mask else _buffer("ws", dev, nws)
+    ws = workspace if workspace is not None else _workspace(dev, nws)
     mptr = None
     if want_mask:
         if mask is None:
@@ -202,7 +194,7 @@ def dsa_attention_masked(q, k, v, selection, o):
     st = status_word(dev)
     nscr = ctypes.c_size_t()
     check(lib.swv_dsa_attn_scratch_bytes(B, H, Tq, Tk, ctypes.byref(nscr)), "swv_dsa_attn_scratch_bytes")
-    scr = _buffer("attn_scratch", dev, nscr.value) if nscr.value else None
+    scr = _workspace(dev, nscr.value) if nscr.value else None
     rc = lib.swv_dsa_attn_masked_fwd(
         q.data_ptr(), strides(q), k.data_ptr(), strides(k), v.data_ptr(), strides(v), mask.data_ptr(),
         ws.data_ptr(), o.data_ptr(), strides(o), dtype_code(o.dtype), B, H, Tq, Tk, D,
@@ -233,7 +225,7 @@ def dsa_attention_lists(q, k, v, idx, rw, selection, o):
     nscr = ctypes.c_size_t()
     check(lib.swv_dsa_attn_lists_scratch_bytes(B, H, Tq, Tk, top_k, ctypes.byref(nscr)),
           "swv_dsa_attn_lists_scratch_bytes")
-    scr = _buffer("attn_lists_scratch", dev, nscr.value)
+    scr = _workspace(dev, nscr.value)
     rc = lib.swv_dsa_attn_lists_fwd(
         q.data_ptr(), strides(q), k.data_ptr(), strides(k), v.data_ptr(), strides(v), idx.data_ptr(), rw.data_ptr(),
         top_k, mask.data_ptr(), ws.data_ptr(), o.data_ptr(), strides(o), dtype_code(o.dtype), B, H, Tq, Tk, D,
@@ -417,7 +409,7 @@ def dsa_module_bwd(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores, mask)
     dqi, dki, dw = f32(B, Tq, IH, ID), f32(B, Tk, IH, ID), f32(IH)
     nws = ctypes.c_size_t()
     check(lib.swv_dsa_module_bwd_bytes(B, H, Tq, Tk, top_k, ctypes.byref(nws)), "swv_dsa_module_bwd_bytes")
-    ws = torch.empty(nws.value, dtype=torch.uint8, device=dev)
+    ws = _workspace(dev, nws.value)
     rc = lib.swv_dsa_module_bwd(
         d_out.data_ptr(), strides(d_out), q.data_ptr(), strides(q), k.data_ptr(), strides(k), v.data_ptr(), strides(v),
         o.data_ptr(), strides(o), dtype_code(o.dtype), q_idx.data_ptr(), strides(q_idx), k_idx.data_ptr(), strides(k_idx),
@@ -561,7 +553,7 @@ def block_sparse_attention(q, k, v, row_ptr, col_idx, block, mode=0, num_cls=0, 
     nws = ctypes.c_size_t()
     check(lib.swv_block_sparse_workspace_bytes(B, H, Tq, Tk, D, block, nnz, ctypes.byref(nws)),
           "swv_block_sparse_workspace_bytes")
-    ws = torch.empty(nws.value, dtype=torch.uint8, device=dev) if nws.value else None
+    ws = _workspace(dev, nws.value) if nws.value else None
     rc = lib.swv_block_sparse_attn_ws_fwd(
         q.data_ptr(), strides(q), k.data_ptr(), strides(k), v.data_ptr(), strides(v), row_ptr.data_ptr(),
         col_idx.data_ptr(), nnz, block, mode, num_cls, window, dilation, kv_group,

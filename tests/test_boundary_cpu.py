@@ -195,3 +195,47 @@ def test_backward_has_no_cpu_path(swv):
     with pytest.raises(swv._lib.SwvError):
         swv.ops.dsa_attention_bwd(z.transpose(1, 2), z.transpose(1, 2), z.transpose(1, 2), z.transpose(1, 2),
                                   z.transpose(1, 2), i, f, f)
+
+
+@pytest.mark.parametrize("op", ["indexer", "attention", "nsa"])
+def test_calls_in_flight_do_not_share_a_workspace(swv, monkeypatch, op):
+    """Two threads whose launches are in flight at the same time (the launch replaced by a host function that
+    waits for the other one) must have been given different workspaces."""
+    import threading
+
+    from sparse_wsi_vit_b200 import nsa, ops
+    launch, at = {"indexer": ("swv_dsa_indexer_topk_fwd", 16), "attention": ("swv_dsa_attn_lists_fwd", 19),
+                  "nsa": ("swv_nsa_attn_fwd", 19)}[op]
+    both, seen = threading.Barrier(2, timeout=20), []
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(swv._lib.lib, name) if name != launch else self.launch
+
+        def launch(self, *args):
+            seen.append(args[at])
+            both.wait()
+            return 0
+
+    for m in (ops, nsa):
+        monkeypatch.setattr(m, "lib", Lib())
+        monkeypatch.setattr(m, "_require_cuda", lambda *ts: None)
+        monkeypatch.setattr(m, "_stream", lambda dev: None)
+    t = lambda *s, dt=torch.bfloat16: torch.zeros(*s, dtype=dt)
+    x = t(1, 2, 300, 64)
+
+    def call():
+        if op == "indexer":
+            ops.dsa_indexer_topk(t(1, 300, 4, 32), t(1, 300, 4, 32), torch.ones(4), 8)
+        elif op == "attention":
+            lists = t(1, 300, 8, dt=torch.int32), t(1, 300, 8, dt=torch.float32)
+            ops.dsa_attention_lists(x, x, x, *lists, (t(64, dt=torch.int32), t(64, dt=torch.uint8)), t(1, 2, 300, 64))
+        else:
+            nsa.nsa_attention(x, x, x, t(1, 300, 2, 3))
+
+    threads = [threading.Thread(target=call) for _ in range(2)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert len(seen) == 2 and seen[0] != seen[1]
