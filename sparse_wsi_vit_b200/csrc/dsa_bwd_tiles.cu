@@ -20,9 +20,10 @@
 // gradient products.  P and dS are fp32 values: each is split into THREE bf16 terms (24 bits) that are
 // multiplied one after the other, so no product sees fewer bits than the CUDA-core form.  The tensor cores
 // truncate at every accumulation step, always towards zero (2^-27 of the result per step, 9e-6 after the
-// 1128 steps of 6009 keys), so an accumulator holds ONE tile's products: the warps add it to fp32 registers
-// (round to nearest) before they hand over the next tile.  q, k, v are
-// bf16; dO must be exact in bf16 as well (it is whenever the next layer ran in bf16) -- where it is not,
+// 1128 steps of 6009 keys), so an accumulator holds ONE tile's products, those of the smallest terms first:
+// the warps add it to fp32 registers (round to nearest) before they hand over the next tile.  Error against
+// fp64 (1024 to 16384 tokens): 1.4e-7 to 3.5e-7 of every gradient (dq_idx 7.8e-7 at 1024 tokens with the
+// largest terms first), the list kernels 4.1e-7 to 8.4e-7.  q, k, v are bf16; dO must be exact in bf16 as well (it is whenever the next layer ran in bf16) -- where it is not,
 // these kernels return at once and the list kernel runs.
 //
 // Bound: kDkv by the instructions of the sixteen warps (63 % of the issue slots), kStats and kDq by the chain
@@ -196,20 +197,19 @@ __global__ void __launch_bounds__(bwd_threads(MODE), 1)
         const uint32_t buf = tmem_base + (t & 1) * kBufCols;
         const uint32_t st = st0 + (t % kBwdStages) * kStageB;
         const uint64_t d1 = smem_desc_sw128(st), d2 = smem_desc_sw128(st + kSBytes);
+        // Smallest terms first: every accumulation truncates at the size of the sum so far, so only the
+        // products of the leading terms (four of the twelve) do it at the size of the result.
 #pragma unroll
-        for (int ks = 0; ks < kNW / 16; ++ks) {
-          // where the warps left the terms of these 16 streamed rows (see the epilogue)
-          const uint32_t cs = buf + 16 * ks, cr = cs + 64, cp = cs + 128;
-          const bool acc = ks > 0;
-          if (MODE == kDkv) {
-            umma_f16_ts(tmem_base + kColAcc, cs, d2 + ks * 128, kIdescAcc, acc);
-            umma_f16_ts(tmem_base + kColAcc, cs + 8, d2 + ks * 128, kIdescAcc, 1);
-            umma_f16_ts(tmem_base + kColAcc, cr, d2 + ks * 128, kIdescAcc, 1);
+        for (int term = 2; term >= 0; --term) {
+#pragma unroll
+          for (int ks = 0; ks < kNW / 16; ++ks) {
+            // where the warps left the terms of these 16 streamed rows (see the epilogue): six groups of 8 columns
+            const bool acc = term < 2 || ks > 0;
+            const uint32_t c1 = buf + 16 * ks + (term == 0 ? 0 : term == 1 ? 8 : 64);
+            const uint32_t c2 = buf + 16 * ks + (term == 0 ? 72 : term == 1 ? 128 : 136);
+            if (MODE == kDkv) umma_f16_ts(tmem_base + kColAcc, c1, d2 + ks * 128, kIdescAcc, acc);
+            umma_f16_ts(tmem_base + kColAcc + (MODE == kDkv ? 64 : 0), c2, d1 + ks * 128, kIdescAcc, acc);
           }
-          const uint32_t a2 = tmem_base + kColAcc + (MODE == kDkv ? 64 : 0);
-          umma_f16_ts(a2, cr + 8, d1 + ks * 128, kIdescAcc, acc);
-          umma_f16_ts(a2, cp, d1 + ks * 128, kIdescAcc, 1);
-          umma_f16_ts(a2, cp + 8, d1 + ks * 128, kIdescAcc, 1);
         }
         umma_commit(&ctl->empty[t % kBwdStages]);
         umma_commit(&ctl->acc_done);
@@ -686,12 +686,12 @@ __global__ void __launch_bounds__(320, 1)
         tc_fence_after();
         const uint64_t db = smem_desc_sw128(b0 + s * kBBytes, kTile * 128);
 #pragma unroll
-        for (int term = 0; term < 3; ++term) {
+        for (int term = 2; term >= 0; --term) {                // (smallest terms first, see above)
           const uint64_t da = smem_desc_sw128(a0 + term * kTermBytes);
 #pragma unroll
           for (int ks = 0; ks < kTile / 16; ++ks)
             umma_f16_ss(tmem_base, da + (ks >> 2) * (kTile * 128 / 16) + (ks & 3) * 2, db + ks * 128, kIdesc,
-                        term > 0 || ks > 0);
+                        term < 2 || ks > 0);
         }
         umma_commit(&ctl->empty[s]);
         umma_commit(&ctl->done);

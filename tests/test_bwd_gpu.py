@@ -222,3 +222,34 @@ def test_tile_backward_long_sums_keep_fp32(swv):
     for name, x, r in (("dq", got[0][0, 0, :R], dq), ("dq_idx", got[3][0, :R], dqi)):
         err = float((f(x) - r).norm() / r.norm())
         assert err < 2.0 ** -19, (name, err)
+
+
+@pytest.mark.parametrize("T,K", [(1024, 512), (3001, 512)])
+def test_tile_backward_is_as_exact_as_the_lists(swv, T, K):
+    """Both forms of the module backward against fp64 on the same lists: the tensor cores truncate each
+    accumulation, which must not cost the tiles more than the CUDA-core kernels' rounded sums lose."""
+    H, ID = 2, 64
+    g = torch.Generator(device=DEV).manual_seed(T)
+    rnd = lambda *s, scale=1.0: (torch.randn(*s, generator=g, device=DEV) * scale).to(torch.bfloat16)
+    q, k, v, do = (rnd(1, H, T, 64, scale=x) for x in (0.125, 1.0, 1.0, 1.0))
+    qi, ki = rnd(1, T, 4, ID, scale=ID ** -0.5), rnd(1, T, 4, ID, scale=ID ** -0.5)
+    w = torch.randn(4, generator=g, device=DEV)
+    o, idx, valid, scores, sel = swv.ops._dsa_forward(q, k, v, qi, ki, w, K)
+    tiles = swv.ops.dsa_module_bwd(do, q, k, v, o, qi, ki, w, idx, valid, scores, sel[0])
+    dq, dk, dv, drw = swv.ops.dsa_attention_bwd(do, q, k, v, o, idx, valid, scores * valid)
+    lists = (dq, dk, dv) + swv.ops.dsa_indexer_bwd(drw, qi, ki, w, idx, valid)
+    swv.check_status(DEV)
+    f = lambda x: x[0].double()
+    rw = torch.zeros(T, T, dtype=torch.float64, device=DEV).scatter_(1, idx[0].long(), f(scores))
+    mem = torch.zeros(T, T, dtype=torch.bool, device=DEV).scatter_(1, idx[0].long(), True)
+    logit = (f(q) @ f(k).transpose(1, 2) / 8).masked_fill(~mem, float("-inf"))
+    e = torch.exp(logit - logit.max(-1, keepdim=True).values)
+    sm = e / (e * rw).sum(-1, keepdim=True).clamp_min(1e-6)
+    gr = sm * (f(do) @ f(v).transpose(1, 2) - (f(do) * f(o)).sum(-1, keepdim=True))
+    dg = gr.sum(0)
+    dqi = (dg @ f(ki).reshape(T, -1)).reshape(T, 4, ID)
+    ref = [(rw * gr) @ f(k) / 8, (rw * gr).transpose(1, 2) @ f(q) / 8, (sm * rw).transpose(1, 2) @ f(do),
+           dqi * w.double()[:, None], (dg.T @ f(qi).reshape(T, -1)).reshape(T, 4, ID) * w.double()[:, None]]
+    for name, a, b, r in zip(("dq", "dk", "dv", "dq_idx", "dk_idx"), tiles, lists, ref):
+        ea, eb = (float((f(x) - r).norm() / r.norm()) for x in (a, b))
+        assert ea <= eb, (name, ea, eb)
