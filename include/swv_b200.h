@@ -206,14 +206,15 @@ int swv_dsa_attn_bwd(const void* d_out, const int64_t d_out_strides[4], const vo
                      const int64_t rw_strides[3], float* dq, float* dk, float* dv, float* drw, int B, int H, int Tq,
                      int Tk, int D, int top_k, int* status, void* stream);
 
-/* Both backward steps of a DSA layer in one call, for the lists and the membership bitmask that
- * swv_dsa_indexer_topk_fwd wrote for the same q_idx, k_idx and w: the gradients of swv_dsa_attn_bwd with
+/* Both backward steps of a DSA layer in one call, for the lists that swv_dsa_indexer_topk_fwd wrote for the
+ * same q_idx, k_idx and w (maskbits: the membership bitmask it wrote with them, or NULL: rebuilt from the lists): the gradients of swv_dsa_attn_bwd with
  * rw = scores * valid, and those of swv_dsa_indexer_bwd with d_scores = drw, computed on tensor-core
  * tiles with every fp32 factor split into three bf16 terms.  q, k, v bf16 with D == 64 and 16-byte
  * rows; d_out and o in o_dtype, unit inner stride.  Where d_out holds values with more bits than bf16 the
  * attention part runs on the list kernel instead (decided on the device).  idx, valid, scores, drw
  * (B,Tq,top_k) and all gradients fp32 contiguous; ID <= 64; top_k <= 65535; B*Tq*top_k < 2^32.
- * `workspace`: swv_dsa_module_bwd_bytes() bytes, 256-byte aligned.
+ * The work grows with Tq * Tk, that of the two list entries with Tq * top_k: the tiles win above about one
+ * key in 40.  `workspace`: swv_dsa_module_bwd_bytes() bytes, 256-byte aligned.
  */
 int swv_dsa_module_bwd_bytes(int B, int H, int Tq, int Tk, int top_k, size_t* bytes);
 int swv_dsa_module_bwd(const void* d_out, const int64_t d_out_strides[4], const void* q, const int64_t q_strides[4],

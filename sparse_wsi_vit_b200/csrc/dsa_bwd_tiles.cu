@@ -1,5 +1,5 @@
 // Backward of a DSA layer on the tensor cores, for selections this library's own indexer made
-// (ascending key lists with their membership bitmask): gradients of the routing-weighted attention
+// (ascending key lists; their membership bitmask is rebuilt from them): gradients of the routing-weighted attention
 // (src/sparse_wsi_vit/models/deepseek_sparse_attention_kernels/kernels.py:569-762) and of the indexer
 // (:128-339), the same formulas as the list kernels in dsa_bwd.cu, which serve every other case.
 //
@@ -263,8 +263,13 @@ __global__ void __launch_bounds__(bwd_threads(MODE), 1)
       if (i < p.Tq) {
         mw = __ldg(reinterpret_cast<const uint4*>(p.maskbits) +
                    ((static_cast<int64_t>(b) * p.nQT + (i >> 7)) * p.nKT + lt) * kTile + (i & 127));
-        pos = (static_cast<uint32_t>(b) * p.Tq + i) * p.top_k +
-              __ldg(p.off + (static_cast<int64_t>(b) * (p.nKT + 1) + lt) * p.Tq + i);
+        const int first = __ldg(p.off + (static_cast<int64_t>(b) * (p.nKT + 1) + lt) * p.Tq + i);
+        pos = (static_cast<uint32_t>(b) * p.Tq + i) * p.top_k + first;
+        // (a bitmask that does not belong to the list: nothing is stored outside the row)
+        if (first + __popc(mw.x) + __popc(mw.y) + __popc(mw.z) + __popc(mw.w) > p.top_k) {
+          record_status(p.status, kDevBadIndex);
+          mw = make_uint4(0u, 0u, 0u, 0u);
+        }
         f.x = __ldg(p.rmax + bh * p.Tq + i);
         f.y = __ldg(p.linv + bh * p.Tq + i);
         f.z = __ldg(p.di + bh * p.Tq + i);
@@ -541,28 +546,57 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// off[b][kt][i] = first slot of row i whose key lies in tile kt or later (kt = 0 .. nKT); one warp per
-// row of the ascending lists (`n` slots are valid in every row).
+// off[b][kt][i] = first slot of row i whose key lies in tile kt or later (kt = 0 .. nKT); one warp per row of
+// the ascending lists (`n` slots are valid in every row).  With `mask` also the tile-major membership bitmask:
+// the CTA's eight rows fill a window of 32 key tiles in shared memory and write it in runs of 128 bytes, so that
+// a layer need not keep the T^2 / 8 bytes from its forward to its backward.
 __global__ void __launch_bounds__(256)
-    dsa_bwd_offsets_kernel(const int32_t* __restrict__ idx, int top_k, int n, int B, int T, int nKT,
-                           uint16_t* __restrict__ off) {
-  const int64_t r = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (r >= static_cast<int64_t>(B) * T) return;
+    dsa_bwd_offsets_kernel(const int32_t* __restrict__ idx, int top_k, int n, int B, int T, int Tk, int nKT,
+                           uint16_t* __restrict__ off, uint4* __restrict__ mask, int* status) {
+  constexpr int kWin = 32;                               // key tiles per window
+  __shared__ __align__(16) uint32_t words[kWin][8][4];
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t r0 = static_cast<int64_t>(blockIdx.x) * 8, r = r0 + wib, rows = static_cast<int64_t>(B) * T;
+  if (r >= rows) n = 0;
   const int b = static_cast<int>(r / T), t = static_cast<int>(r % T);
   const int32_t* row = idx + r * top_k;
   uint16_t* dst = off + static_cast<int64_t>(b) * (nKT + 1) * T + t;
   int carry = -1;                                        // tile of the slot before this group
-  for (int s0 = 0; s0 < n; s0 += 32) {
-    const int s = s0 + lane;
-    const int kt = s < n ? min(max(__ldg(row + s) >> 7, 0), nKT - 1) : nKT;
-    int before = __shfl_up_sync(0xffffffffu, kt, 1);
-    if (lane == 0) before = carry;
-    if (s < n)
-      for (int q = before + 1; q <= kt; ++q) dst[static_cast<int64_t>(q) * T] = static_cast<uint16_t>(s);
-    carry = __shfl_sync(0xffffffffu, kt, min(31, n - 1 - s0));
+  int s0 = -32, key = 0;
+  bool placed = true;                                    // this lane's slot has its bit
+  for (int win = 0; win < nKT; win += kWin) {
+    reinterpret_cast<uint4*>(words)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    for (;;) {
+      if (!placed && (key >> 7) < win + kWin) {
+        if (key >= win * kTile) atomicOr(&words[(key >> 7) - win][wib][(key >> 5) & 3], 1u << (key & 31));
+        else record_status(status, kDevBadIndex);        // (not ascending)
+        placed = true;
+      }
+      if (!__all_sync(0xffffffffu, placed) || s0 + 32 >= n) break;     // the rest lies behind the window, or the row is done
+      s0 += 32;
+      const int s = s0 + lane;
+      placed = s >= n;
+      key = placed ? 0 : min(max(__ldg(row + s), 0), Tk - 1);
+      const int kt = placed ? nKT : key >> 7;
+      int before = __shfl_up_sync(0xffffffffu, kt, 1);
+      if (lane == 0) before = carry;
+      if (!placed)
+        for (int q = before + 1; q <= kt; ++q) dst[static_cast<int64_t>(q) * T] = static_cast<uint16_t>(s);
+      carry = __shfl_sync(0xffffffffu, kt, min(31, n - 1 - s0));
+    }
+    __syncthreads();
+    const int kt = win + (threadIdx.x >> 3), rr = threadIdx.x & 7;
+    if (mask != nullptr && kt < nKT && r0 + rr < rows) {
+      const int bb = static_cast<int>((r0 + rr) / T), tt = static_cast<int>((r0 + rr) % T);
+      const int nQT = (T + kTile - 1) / kTile;
+      mask[((static_cast<int64_t>(bb) * nQT + tt / kTile) * nKT + kt) * kTile + tt % kTile] =
+          *reinterpret_cast<const uint4*>(words[threadIdx.x >> 3][rr]);
+    }
+    __syncthreads();
   }
-  for (int q = carry + 1 + lane; q <= nKT; q += 32) dst[static_cast<int64_t>(q) * T] = static_cast<uint16_t>(n);
+  if (r < rows)
+    for (int q = carry + 1 + lane; q <= nKT; q += 32) dst[static_cast<int64_t>(q) * T] = static_cast<uint16_t>(n);
 }
 
 // drw = sum over the heads of their g, heads in ascending order (slots behind the valid ones are zero)
@@ -830,7 +864,7 @@ __global__ void __launch_bounds__(320, 1)
 
 size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 struct BwdLayout {
-  size_t do16, di, rmax, linv, wq, wk, off, flag, gh, total;
+  size_t do16, di, rmax, linv, wq, wk, off, flag, mask, gh, total;
 };
 BwdLayout bwd_layout(int B, int H, int Tq, int Tk, int top_k) {
   BwdLayout L;
@@ -845,6 +879,7 @@ BwdLayout bwd_layout(int B, int H, int Tq, int Tk, int top_k) {
   L.wk = o; o += up256(static_cast<size_t>(B) * Tk * kIdxDim * 4);
   L.off = o; o += up256(static_cast<size_t>(B) * (nKT + 1) * Tq * 2);
   L.flag = o; o += 256;
+  L.mask = o; o += up256(static_cast<size_t>(B) * ((Tq + kTile - 1) / kTile) * nKT * kTile * 16);
   L.gh = o; o += up256(rows * top_k * 4);
   L.total = o;
   return L;
@@ -941,7 +976,7 @@ int dsa_module_bwd_impl(const void* d_out, const int64_t* dos, const void* q, co
                         const uint32_t* maskbits, float* dq, float* dk, float* dv, float* drw, float* dq_idx,
                         float* dk_idx, float* dw, int B, int H, int Tq, int Tk, int D, int IH, int ID, int top_k,
                         void* workspace, size_t workspace_bytes, int* status, cudaStream_t st) {
-  if (!d_out || !q || !k || !v || !o || !q_idx || !k_idx || !w || !idx || !valid || !scores || !maskbits || !dq || !dk ||
+  if (!d_out || !q || !k || !v || !o || !q_idx || !k_idx || !w || !idx || !valid || !scores || !dq || !dk ||
       !dv || !drw || !dq_idx || !dk_idx || !dw || !workspace || !status)
     return SWV_ERR_NULL;
   if (B < 1 || H < 1 || Tq < 1 || Tk < 1 || top_k < 1 || IH < 1 || ID < 1) return SWV_ERR_SHAPE;
@@ -981,8 +1016,10 @@ int dsa_module_bwd_impl(const void* d_out, const int64_t* dos, const void* q, co
   rc = dsa_collapse_impl(k_idx, kis, idx_dtype, w, wk, B, Tk, IH, ID, st);
   if (rc != SWV_OK) return rc;
   const int64_t rows = static_cast<int64_t>(B) * Tq;
+  uint4* own_mask = maskbits == nullptr ? reinterpret_cast<uint4*>(ws + L.mask) : nullptr;
+  if (own_mask != nullptr) maskbits = reinterpret_cast<const uint32_t*>(own_mask);
   dsa_bwd_offsets_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, st>>>(idx, top_k, top_k < Tk ? top_k : Tk, B, Tq,
-                                                                              nKT, off);
+                                                                              Tk, nKT, off, own_mask, status);
   SWV_CUDA_OK(cudaGetLastError());
 
   // maps with 128-row boxes (lane side) and 64-row boxes (streamed side)

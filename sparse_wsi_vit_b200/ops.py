@@ -388,11 +388,12 @@ def dsa_indexer_bwd(d_scores, q_idx, k_idx, w, idx, valid):
     return dq, dk, dw
 
 
-def dsa_module_bwd(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores, mask):
+def dsa_module_bwd(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores, mask=None):
     """``dsa_attention_bwd`` (with ``rw = scores * valid``) and ``dsa_indexer_bwd`` of its ``drw`` in one call
-    on tensor-core tiles, for lists and bitmask of this library's indexer on the same projections; bf16
-    q, k, v with head_dim 64.  Returns fp32 ``dq, dk, dv, dq_idx, dk_idx, dw``."""
-    _require_cuda(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores, mask)
+    on tensor-core tiles, for lists of this library's indexer on the same projections (``mask``: the bitmask of
+    its selection handle; rebuilt from the lists without it); bf16 q, k, v with head_dim 64.  Returns fp32
+    ``dq, dk, dv, dq_idx, dk_idx, dw``."""
+    _require_cuda(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores)
     B, H, Tq, D = q.shape
     Tk, top_k = k.shape[2], idx.shape[-1]
     IH, ID = q_idx.shape[2:]
@@ -413,13 +414,31 @@ def dsa_module_bwd(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores, mask)
     rc = lib.swv_dsa_module_bwd(
         d_out.data_ptr(), strides(d_out), q.data_ptr(), strides(q), k.data_ptr(), strides(k), v.data_ptr(), strides(v),
         o.data_ptr(), strides(o), dtype_code(o.dtype), q_idx.data_ptr(), strides(q_idx), k_idx.data_ptr(), strides(k_idx),
-        dtype_code(q_idx.dtype), w32.data_ptr(), idx.data_ptr(), valid.data_ptr(), scores.data_ptr(), mask.data_ptr(),
-        dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), drw.data_ptr(), dqi.data_ptr(), dki.data_ptr(), dw.data_ptr(),
+        dtype_code(q_idx.dtype), w32.data_ptr(), idx.data_ptr(), valid.data_ptr(), scores.data_ptr(),
+        None if mask is None else mask.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), drw.data_ptr(), dqi.data_ptr(), dki.data_ptr(), dw.data_ptr(),
         B, H, Tq, Tk, D, IH, ID, top_k, ws.data_ptr(), nws.value, status_word(dev).data_ptr(), _stream(dev))
     check(rc, "swv_dsa_module_bwd")
     if _CHECK:
         check_status(dev, "swv_dsa_module_bwd")
     return dq, dk, dv, dqi, dki, dw
+
+
+# The tile form of the module backward does a constant amount of work per (query, key) pair of the whole sequence,
+# the list kernels per selected pair.  Measured on B200, both forms, 8 heads / 6 heads (ms, tiles against lists):
+# 65536 tokens 168 : 227 at top-2048, 167 : 108 at 1024; 32768 tokens 42.2 : 54.3 / 31.5 : 37.6 at 1024, 42.0 : 27.0 /
+# 31.2 : 18.6 at 512; 8192 tokens 3.19 : 3.51 / 2.29 : 2.43 at 256, 3.17 : 1.79 at 128.  The two meet at one key in 40,
+# and some 30 keys later for the tiles' extra launches, which short sequences feel (2048 tokens: 0.36 : 0.59 at 128,
+# 0.38 : 0.35 at 64).
+TILE_BWD_KEYS_PER_SELECTED = 40
+TILE_BWD_MIN_SELECTED = 30
+
+
+def tile_backward_pays(Tq, Tk, top_k, B=1):
+    """Whether ``dsa_module_bwd`` serves lists of this size faster than the two list kernels, and can address
+    them (16-bit slots, 32-bit positions)."""
+    if top_k > 65535 or B * Tq * top_k >= 1 << 32:
+        return False
+    return TILE_BWD_KEYS_PER_SELECTED * (min(top_k, Tk) - TILE_BWD_MIN_SELECTED) >= Tk
 
 
 class LightningIndexerFunction(torch.autograd.Function):
@@ -476,17 +495,17 @@ class DSAModuleFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, q_idx, k_idx, w, top_k, out_dtype):
-        o, idx, valid, scores, sel = _dsa_forward(q.detach(), k.detach(), v.detach(), q_idx.detach(), k_idx.detach(),
-                                                  w.detach(), top_k, out_dtype=out_dtype)
-        ctx.save_for_backward(q, k, v, q_idx, k_idx, w, idx, valid, scores, o, None if sel is None else sel[0])
+        o, idx, valid, scores, _ = _dsa_forward(q.detach(), k.detach(), v.detach(), q_idx.detach(), k_idx.detach(),
+                                                w.detach(), top_k, out_dtype=out_dtype)
+        ctx.save_for_backward(q, k, v, q_idx, k_idx, w, idx, valid, scores, o)
         return o
 
     @staticmethod
     def backward(ctx, d_out):
-        q, k, v, q_idx, k_idx, w, idx, valid, scores, o, mask = ctx.saved_tensors
-        # the tile form addresses lists by 16-bit slots and 32-bit positions
-        if mask is not None and idx.shape[-1] < 65536 and idx.numel() < 1 << 32 and q_idx.shape[-1] <= 64:
-            dq, dk, dv, dqi, dki, dw = dsa_module_bwd(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores, mask)
+        q, k, v, q_idx, k_idx, w, idx, valid, scores, o = ctx.saved_tensors
+        if (q.dtype == torch.bfloat16 and q.shape[-1] == 64 and q_idx.shape[-1] <= 64 and
+                tile_backward_pays(idx.shape[1], k.shape[2], idx.shape[-1], idx.shape[0])):
+            dq, dk, dv, dqi, dki, dw = dsa_module_bwd(d_out, q, k, v, o, q_idx, k_idx, w, idx, valid, scores)
         else:
             dq, dk, dv, drw = dsa_attention_bwd(d_out.contiguous(), q, k, v, o, idx, valid, scores * valid)
             # d scores = d rw * valid; the indexer backward multiplies by valid itself (valid is 0 or 1)

@@ -239,3 +239,14 @@ def test_calls_in_flight_do_not_share_a_workspace(swv, monkeypatch, op):
     for th in threads:
         th.join()
     assert len(seen) == 2 and seen[0] != seen[1]
+
+
+def test_backward_form_follows_the_measured_times(swv):
+    """(tokens, top_k) with the time of the list kernels over that of the tiles, 8 heads: the faster form is chosen
+    wherever the two differ by more than a tenth; sizes the tiles cannot address stay with the lists."""
+    pays = swv.ops.tile_backward_pays
+    for T, K, ratio in ((1024, 16, 0.53), (1024, 128, 1.52), (2048, 16, 0.39), (2048, 128, 1.67), (4096, 64, 0.54),
+                        (4096, 256, 1.94), (8192, 128, 0.57), (8192, 256, 1.10), (16384, 256, 0.65), (16384, 512, 1.27),
+                        (32768, 512, 0.64), (32768, 1024, 1.28), (65536, 1024, 0.65), (65536, 2048, 1.35)):
+        assert pays(T, T, K) == (ratio > 1), (T, K)
+    assert pays(300, 300, 5000) and not pays(70000, 70000, 65536) and not pays(65536, 65536, 32768, B=2)

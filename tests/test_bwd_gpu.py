@@ -253,3 +253,44 @@ def test_tile_backward_is_as_exact_as_the_lists(swv, T, K):
     for name, a, b, r in zip(("dq", "dk", "dv", "dq_idx", "dk_idx"), tiles, lists, ref):
         ea, eb = (float((f(x) - r).norm() / r.norm()) for x in (a, b))
         assert ea <= eb, (name, ea, eb)
+
+
+@pytest.mark.parametrize("B,T,K", [(1, 100, 7), (3, 131, 40), (1, 4097, 300), (2, 4500, 20)])
+def test_tile_backward_rebuilds_the_bitmask(swv, B, T, K):
+    """Without the bitmask of the forward the backward builds it from the lists: the same gradients bit for bit
+    (dw is summed in arrival order).  Rows of several batches in one CTA, a list that ends inside a group of
+    32 slots, lists over more than one window of 32 key tiles with empty tiles between."""
+    g = torch.Generator().manual_seed(T)
+    bf = torch.bfloat16
+    q, k, v, do = (torch.randn(B, 1, T, 64, generator=g).to(bf).to(DEV) for _ in range(4))
+    qi, ki = (torch.randn(B, T, 4, 32, generator=g).to(bf).to(DEV) for _ in range(2))
+    w = torch.randn(4, generator=g).to(DEV)
+    o, idx, valid, scores, sel = swv.ops._dsa_forward(q, k, v, qi, ki, w, K)
+    args = (do, q, k, v, o, qi, ki, w, idx, valid, scores)
+    with_mask, without = swv.ops.dsa_module_bwd(*args, sel[0]), swv.ops.dsa_module_bwd(*args)
+    swv.check_status(DEV)
+    for name, a, b in zip(("dq", "dk", "dv", "dq_idx", "dk_idx"), with_mask, without):
+        assert torch.equal(a, b), name
+    assert _close(without[5], with_mask[5].cpu())
+
+
+def test_module_backward_form_and_memory(swv, monkeypatch):
+    """The module takes the tiles for dense selections and the two list kernels for sparse ones, and keeps nothing
+    of the size of the bitmask (T^2 / 8 bytes) from its forward to its backward."""
+    calls, real = [], swv.ops.dsa_module_bwd
+    monkeypatch.setattr(swv.ops, "dsa_module_bwd", lambda *a, **kw: calls.append(1) or real(*a, **kw))
+    T, grads = 3000, {}
+    for K in (256, 64):
+        torch.manual_seed(0)
+        m = swv.DeepSeekSparseAttention(d_model=64, attention_heads=1, indexer_heads=4, indexer_dim=32, top_k=K).to(DEV)
+        x = torch.randn(1, T, 64, generator=torch.Generator().manual_seed(1)).to(DEV)
+        kept = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: kept.append(t) or t, lambda t: t):
+            with torch.autocast("cuda", dtype=torch.bfloat16):
+                y = m(x)
+        n = len(calls)
+        y.float().square().mean().backward()
+        swv.check_status(DEV)
+        assert (len(calls) > n) == (K == 256)
+        assert [tuple(t.shape) for t in kept if t.dtype == torch.int32] == [(1, T, K)]
+        assert all(torch.isfinite(p.grad).all() for p in m.parameters())
