@@ -76,12 +76,13 @@ constexpr uint32_t kColAcc = 384;       // dV (or dQ) 64 | dK 64
 
 struct BwdTileParams {
   int B, H, Tq, Tk, nQT, nKT, top_k;
+  int h0, Hn;               // heads of this launch: h0 .. h0 + Hn - 1
   const uint32_t* maskbits;
   const uint16_t* off;      // [B][nKT + 1][Tq] first list slot of row i with a key in tile kt or later
   const float* di;          // (B,H,Tq)
   float *rmax, *linv;       // (B,H,Tq): row maximum of the members' logits (log2 domain), 1 / max(l, 1e-6)
   float *dq, *dk, *dv;
-  float* gh;                // [H][B*Tq*top_k] the heads' g in list order
+  float* gh;                // [Hn][B*Tq*top_k] the heads' g in list order
   int r_steps;              // 8-channel steps of the routing-weight product (the rest of the 64 channels is zero)
   float scale, c2;          // 1/sqrt(D), and times log2 e
   const int* skip_if;       // non-zero: nothing to do here
@@ -129,8 +130,8 @@ __global__ void __launch_bounds__(bwd_threads(MODE), 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nLT = MODE == kDkv ? p.nKT : p.nQT;
   const int lt = blockIdx.x % nLT;                       // lane-side tile
-  const int h = (blockIdx.x / nLT) % p.H;
-  const int b = blockIdx.x / (nLT * p.H);
+  const int h = p.h0 + (blockIdx.x / nLT) % p.Hn;
+  const int b = blockIdx.x / (nLT * p.Hn);
   const int nS = ((MODE == kDkv ? p.Tq : p.Tk) + kNW - 1) / kNW;   // streamed tiles
 
   if (threadIdx.x == 0) {
@@ -331,7 +332,7 @@ __global__ void __launch_bounds__(bwd_threads(MODE), 1)
 
     if constexpr (MODE == kDkv) {
       const uint32_t lt_mask = (1u << lane) - 1u;
-      float* gh = p.gh + static_cast<size_t>(h) * p.B * p.Tq * p.top_k;
+      float* gh = p.gh + static_cast<size_t>(h - p.h0) * p.B * p.Tq * p.top_k;
       for (int t = 0; t < nS; ++t) {
         const BwdCols& c = cols[t & 1];
         if (!mbar_wait_bounded(&ctl->in_full[t & 1], (t >> 1) & 1, abort_flag)) {
@@ -599,15 +600,16 @@ __global__ void __launch_bounds__(256)
     for (int q = carry + 1 + lane; q <= nKT; q += 32) dst[static_cast<int64_t>(q) * T] = static_cast<uint16_t>(n);
 }
 
-// drw = sum over the heads of their g, heads in ascending order (slots behind the valid ones are zero)
+// drw = sum over the heads of their g, heads in ascending order (slots behind the valid ones are zero); `add`:
+// the sum goes on from the heads before these
 __global__ void __launch_bounds__(256)
     dsa_bwd_sum_heads_kernel(const float* __restrict__ gh, float* __restrict__ drw, int64_t n, int H, int top_k,
-                             int n_valid, const int* __restrict__ skip_if) {
+                             int n_valid, bool add, const int* __restrict__ skip_if) {
   if (skip_if != nullptr && *skip_if != 0) return;
   const int64_t i = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) * 4;
   if (i >= n) return;
   if (((n | top_k | n_valid) & 3) == 0) {
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 a = add ? *reinterpret_cast<const float4*>(drw + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     if (static_cast<int>(i % top_k) < n_valid)
       for (int h = 0; h < H; ++h) {
         const float4 x = __ldcs(reinterpret_cast<const float4*>(gh + h * n + i));
@@ -616,7 +618,7 @@ __global__ void __launch_bounds__(256)
     *reinterpret_cast<float4*>(drw + i) = a;
   } else {
     for (int64_t e = i; e < i + 4 && e < n; ++e) {
-      float a = 0.f;
+      float a = add ? drw[e] : 0.f;
       if (static_cast<int>(e % top_k) < n_valid)
         for (int h = 0; h < H; ++h) a += gh[h * n + e];
       drw[e] = a;
@@ -863,7 +865,12 @@ __global__ void __launch_bounds__(320, 1)
 }
 
 size_t up256(size_t x) { return (x + 255) / 256 * 256; }
+// Room for the heads' list gradients: as many heads as fit go through one dK / dV launch, their sum is added to
+// that of the heads before (the same order of additions whatever the number).  16384 tokens, 8 heads, top-2048
+// fill it; a sequence whose single head is larger takes one head at a time, the size of drw itself.
+constexpr size_t kGhBytes = size_t(1) << 30;
 struct BwdLayout {
+  int heads;
   size_t do16, di, rmax, linv, wq, wk, off, flag, mask, gh, total;
 };
 BwdLayout bwd_layout(int B, int H, int Tq, int Tk, int top_k) {
@@ -880,7 +887,9 @@ BwdLayout bwd_layout(int B, int H, int Tq, int Tk, int top_k) {
   L.off = o; o += up256(static_cast<size_t>(B) * (nKT + 1) * Tq * 2);
   L.flag = o; o += 256;
   L.mask = o; o += up256(static_cast<size_t>(B) * ((Tq + kTile - 1) / kTile) * nKT * kTile * 16);
-  L.gh = o; o += up256(rows * top_k * 4);
+  const size_t head = static_cast<size_t>(B) * Tq * top_k * 4;
+  L.heads = static_cast<int>(std::max<size_t>(1, std::min<size_t>(H, kGhBytes / head)));
+  L.gh = o; o += up256(L.heads * head);
   L.total = o;
   return L;
 }
@@ -890,7 +899,7 @@ int launch_bwd(const CUtensorMap& l1, const CUtensorMap& l2, const CUtensorMap& 
                const CUtensorMap& s2, const CUtensorMap& sr, const BwdTileParams& p, cudaStream_t st) {
   SWV_CUDA_OK(cudaFuncSetAttribute(dsa_bwd_tiles_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(kBwdSmem)));
-  const unsigned grid = static_cast<unsigned>(p.B) * p.H * (MODE == kDkv ? p.nKT : p.nQT);
+  const unsigned grid = static_cast<unsigned>(p.B) * p.Hn * (MODE == kDkv ? p.nKT : p.nQT);
   dsa_bwd_tiles_kernel<MODE><<<grid, bwd_threads(MODE), kBwdSmem, st>>>(l1, l2, lr, s1, s2, sr, p);
   SWV_CUDA_OK(cudaGetLastError());
   return SWV_OK;
@@ -1040,6 +1049,7 @@ int dsa_module_bwd_impl(const void* d_out, const int64_t* dos, const void* q, co
   BwdTileParams p;
   p.B = B; p.H = H; p.Tq = Tq; p.Tk = Tk; p.nQT = nQT; p.nKT = nKT; p.top_k = top_k;
   p.maskbits = maskbits; p.off = off; p.di = di; p.rmax = reinterpret_cast<float*>(ws + L.rmax); p.linv = reinterpret_cast<float*>(ws + L.linv);
+  p.h0 = 0; p.Hn = H;
   p.dq = dq; p.dk = dk; p.dv = dv; p.gh = reinterpret_cast<float*>(ws + L.gh);
   p.r_steps = (ID + 7) / 8;
   p.scale = 1.0f / sqrtf(static_cast<float>(D));
@@ -1047,12 +1057,15 @@ int dsa_module_bwd_impl(const void* d_out, const int64_t* dos, const void* q, co
   p.skip_if = exact ? nullptr : flag;
   p.status = status;
   if ((rc = launch_bwd<kStats>(mq[0], mq[0], mwq[0], mk[1], mk[1], mwk[1], p, st)) != SWV_OK) return rc;
-  if ((rc = launch_bwd<kDkv>(mk[0], mv[0], mwk[0], mq[1], md[1], mwq[1], p, st)) != SWV_OK) return rc;
   if ((rc = launch_bwd<kDq>(mq[0], md[0], mwq[0], mk[1], mv[1], mwk[1], p, st)) != SWV_OK) return rc;
   const int64_t n = rows * top_k;
-  dsa_bwd_sum_heads_kernel<<<static_cast<unsigned>((n + 1023) / 1024), 256, 0, st>>>(p.gh, drw, n, H, top_k,
-                                                                                  top_k < Tk ? top_k : Tk, p.skip_if);
-  SWV_CUDA_OK(cudaGetLastError());
+  for (; p.h0 < H; p.h0 += L.heads) {
+    p.Hn = std::min(L.heads, H - p.h0);
+    if ((rc = launch_bwd<kDkv>(mk[0], mv[0], mwk[0], mq[1], md[1], mwq[1], p, st)) != SWV_OK) return rc;
+    dsa_bwd_sum_heads_kernel<<<static_cast<unsigned>((n + 1023) / 1024), 256, 0, st>>>(
+        p.gh, drw, n, p.Hn, top_k, top_k < Tk ? top_k : Tk, p.h0 > 0, p.skip_if);
+    SWV_CUDA_OK(cudaGetLastError());
+  }
 
   // indexer: tiles for bf16 projections whose heads lie side by side, else the list kernel
   const int E = IH * ID;
@@ -1070,7 +1083,7 @@ int dsa_module_bwd_impl(const void* d_out, const int64_t* dos, const void* q, co
     ip.dx = dq_idx; ip.dw = dw; ip.status = status;
     // the heads' gradients have been summed: their room takes the partial sums
     float* part = p.gh;
-    const size_t nf = static_cast<size_t>(n) * H;
+    const size_t nf = static_cast<size_t>(n) * L.heads;
     if (E == 64) rc = launch_idx<kLaneQ, 64>(tk, ip, part, nf, st);
     else if (E == 128) rc = launch_idx<kLaneQ, 128>(tk, ip, part, nf, st);
     else rc = launch_idx<kLaneQ, 256>(tk, ip, part, nf, st);

@@ -82,6 +82,12 @@ def test_size_queries(swv):
     assert L.swv_block_sparse_workspace_bytes(1, 16, 65536, 65536, 128, 128, nnz, ctypes.byref(n)) == 0
     assert 0 < n.value <= 16 * (2 * 20 * 128 * (128 * 4 + 8) + 512 * 4)
     assert L.swv_block_sparse_workspace_bytes(1, 16, 65536, 65536, 128, 128, 0, ctypes.byref(n)) == 0 and n.value == 0
+    # module backward: the heads' list gradients take 1 GiB at most, or one head's lists
+    size = lambda *a: (L.swv_dsa_module_bwd_bytes(*a, ctypes.byref(n)), n.value)[1]
+    per_row = 64 * 2 + 3 * 4                       # bf16 d_out and three fp32 row values per head
+    base = lambda H, T: T * (H * per_row + 2 * 64 * 4 + (T // 128 + 1) * 2 + T // 8)
+    for H, T, K, heads in ((8, 16384, 2048, 8), (12, 16384, 2048, 8), (8, 65536, 2048, 2), (12, 65536, 16384, 1)):
+        assert 0 <= size(1, H, T, T, K) - base(H, T) - heads * T * K * 4 <= 4096
     # NSA sizes
     assert L.swv_nsa_importance_bytes(1, 2, 65536, 4095, 16, 64, ctypes.byref(n)) == 0
     assert n.value == 2 * 65536 * 1024 * 4

@@ -294,3 +294,23 @@ def test_module_backward_form_and_memory(swv, monkeypatch):
         assert (len(calls) > n) == (K == 256)
         assert [tuple(t.shape) for t in kept if t.dtype == torch.int32] == [(1, T, K)]
         assert all(torch.isfinite(p.grad).all() for p in m.parameters())
+
+
+def test_tile_backward_in_head_groups(swv):
+    """More heads than the room for their list gradients holds (1 GiB: three heads of 8200 tokens with 8192 slots):
+    every head's gradients are those of a call with fewer heads, bit for bit, and the indexer's follow the sum
+    over all heads, which goes on in the same order (2^-20: the one-group calls are added in another)."""
+    T, K, H = 8200, 8192, 5
+    g = torch.Generator(device=DEV).manual_seed(3)
+    rnd = lambda *s, scale=1.0: (torch.randn(*s, generator=g, device=DEV) * scale).to(torch.bfloat16)
+    q, k, v, do = (rnd(1, H, T, 64, scale=x) for x in (0.125, 1.0, 1.0, 1.0))
+    qi, ki = rnd(1, T, 2, 32, scale=0.18), rnd(1, T, 2, 32, scale=0.18)
+    w = torch.randn(2, generator=g, device=DEV)
+    o, idx, valid, scores, _ = swv.ops._dsa_forward(q, k, v, qi, ki, w, K)
+    run = lambda h: swv.ops.dsa_module_bwd(*(x[:, h] for x in (do, q, k, v, o)), qi, ki, w, idx, valid, scores)
+    every, parts = run(slice(0, H)), (run(slice(0, 3)), run(slice(3, H)))
+    swv.check_status(DEV)
+    for i in range(3):
+        assert torch.equal(every[i], torch.cat([p[i] for p in parts], dim=1))
+    for i in (3, 4):
+        assert _close(every[i], (parts[0][i] + parts[1][i]).cpu(), rel=2.0 ** -20)
