@@ -50,7 +50,8 @@ extern "C" {
 #define SWV_BF16 1
 #define SWV_F16 2
 
-/* Library ABI version (major*100 + minor). */
+/* Library ABI version (major*100 + minor).  103: swv_block_sparse_attn_ws_fwd, swv_dsa_module_bwd and their size
+ * queries. */
 int swv_version(void);
 
 /* Text for a negative return code or a positive device status code. */

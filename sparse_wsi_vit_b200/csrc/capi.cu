@@ -84,7 +84,7 @@ int nsa_attn_impl(const void* q, const int64_t* qs, const void* k, const int64_t
 
 extern "C" {
 
-int swv_version(void) { return 102; }
+int swv_version(void) { return 103; }
 
 const char* swv_strerror(int code) {
   switch (code) {
