@@ -249,10 +249,12 @@ __global__ void __launch_bounds__(320, 2)
 // kv heads, 1024 blocks: 0.64 -> 0.17 ms).
 constexpr int kSelCand = 64;
 
-// entry e of an importance row: blocks without compressed tokens (e >= n_pad) have none
-__device__ __forceinline__ float nsa_importance(const float* src, int e, int n_pad, int n_s) {
-  return e >= n_s ? -2.f : e < n_pad ? fmaxf(__ldg(src + e), 0.f) : 0.f;
+// entry e of an importance row (blocks without compressed tokens, e >= n_pad, have none), in two steps so that
+// a thread's loads are all in flight before the first is looked at (in one: 0.53 instead of 0.17 ms)
+__device__ __forceinline__ float nsa_importance_load(const float* src, int e, int n_pad, int n_s) {
+  return e < min(n_pad, n_s) ? __ldg(src + e) : 0.f;
 }
+__device__ __forceinline__ float nsa_importance(float raw, int e, int n_s) { return e < n_s ? fmaxf(raw, 0.f) : -2.f; }
 
 // (every row holds at least k_eff values >= 0)
 __device__ __forceinline__ void nsa_argmax_loop(float* v, int n, int k_eff, int lane, int32_t* dst) {
@@ -299,8 +301,10 @@ __global__ void __launch_bounds__(128) nsa_select_short_kernel(const float* __re
   float v[NPL];
   float mx = -2.f;
 #pragma unroll
+  for (int i = 0; i < NPL; ++i) v[i] = nsa_importance_load(src, i * 32 + lane, n_pad, n_s);
+#pragma unroll
   for (int i = 0; i < NPL; ++i) {
-    v[i] = nsa_importance(src, i * 32 + lane, n_pad, n_s);
+    v[i] = nsa_importance(v[i], i * 32 + lane, n_s);
     mx = fmaxf(mx, v[i]);
   }
   // the k-th largest lane maximum: the one whose rank (ties by lane) is k - 1
@@ -365,7 +369,7 @@ __global__ void __launch_bounds__(128) nsa_select_kernel(const float* __restrict
   const int n = (n_s + 31) & ~31;                     // scanned range, a multiple of 32
   float* v = sel_sm + wib * n;
   const float* src = imp + r * n_pad;
-  for (int i = lane; i < n; i += 32) v[i] = nsa_importance(src, i, n_pad, n_s);
+  for (int i = lane; i < n; i += 32) v[i] = nsa_importance(nsa_importance_load(src, i, n_pad, n_s), i, n_s);
   __syncwarp();
   nsa_argmax_loop(v, n, k_eff, lane, blocks + r * k_eff);
 }
