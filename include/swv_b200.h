@@ -214,7 +214,8 @@ int swv_dsa_attn_bwd(const void* d_out, const int64_t d_out_strides[4], const vo
  * rows; d_out and o in o_dtype, unit inner stride.  Where d_out holds values with more bits than bf16 the
  * attention part runs on the list kernel instead (decided on the device).  idx, valid, scores, drw
  * (B,Tq,top_k) and all gradients fp32 contiguous; ID <= 64; top_k <= 65535; B*Tq*top_k < 2^32.
- * The work grows with Tq * Tk, that of the two list entries with Tq * top_k: the tiles win above about one
+ * A pair that is not selected is multiplied with zero, so a NaN or an infinity in one row can reach every
+ * gradient of its head.  The work grows with Tq * Tk, that of the two list entries with Tq * top_k: the tiles win above about one
  * key in 40.  `workspace`: swv_dsa_module_bwd_bytes() bytes, 256-byte aligned.
  */
 int swv_dsa_module_bwd_bytes(int B, int H, int Tq, int Tk, int top_k, size_t* bytes);

@@ -26,13 +26,16 @@
 // largest terms first), the list kernels 4.1e-7 to 8.4e-7.  q, k, v are bf16; dO must be exact in bf16 as well (it is whenever the next layer ran in bf16) -- where it is not,
 // these kernels return at once and the list kernel runs.
 //
-// Bound: kDkv by the instructions of the sixteen warps (63 % of the issue slots), kStats and kDq by the chain
-// products -> terms -> gradient products of two buffers, at 60-100 cycles per M128 x N64 instruction (40 per
-// tile and head in kDkv, 28 in kDq, 12 in kStats).  16384 tokens, 8 heads, top-2048: kStats 1.6, kDkv 4.9, kDq
-// 3.2 ms; kDkv took 5.8 ms with eight warps, a branch around the list store, and a block barrier per tile for
-// the column data, while the accumulators still ran over the whole row.
-// The list kernels move 3 rows and reduce 2 per selected pair (43.8 ms on the same input); at one key in 8
-// the tiles do 8 times the kept products and are still far ahead.
+// A pair that is not a member is multiplied with zero, not skipped: a NaN or an infinity in one row of q, k, v or
+// dO can reach every gradient of its head (the list kernels keep it to the selected pairs).
+//
+// Bound: kDkv by the instructions of the sixteen warps (63 % of the issue slots, tensor pipe 21 % of the time),
+// kStats and kDq by the chain products -> terms -> gradient products of two buffers (47 and 42 % of the issue
+// slots, tensor pipe 20 and 23 %; ncu at 8192 tokens).  16384 tokens, 8 heads, top-2048: kStats 1.6, kDkv 4.9,
+// kDq 3.2 ms; kDkv took 5.8 ms with eight warps, a branch around the list store, and a block barrier per tile
+// for the column data, while the accumulators still ran over the whole row.
+// The list kernels move 3 rows and reduce 2 per selected pair: 43.7 + 13.4 ms with the indexer's part on the
+// same input against 11.4 ms.  They do T * K work, the tiles T^2: the two meet at about one key in 40.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 

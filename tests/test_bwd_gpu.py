@@ -314,3 +314,28 @@ def test_tile_backward_in_head_groups(swv):
         assert torch.equal(every[i], torch.cat([p[i] for p in parts], dim=1))
     for i in (3, 4):
         assert _close(every[i], (parts[0][i] + parts[1][i]).cpu(), rel=2.0 ** -20)
+
+
+def test_tile_backward_with_a_nan_query(swv):
+    """One NaN query (its lists and weights are finite): its gradient and those of the keys it selected are NaN,
+    the other queries' gradients are what they are without it, and no wait runs out."""
+    T, K, H = 700, 64, 2
+    g = torch.Generator().manual_seed(2)
+    bf = torch.bfloat16
+    q, k, v, do = (torch.randn(1, H, T, 64, generator=g).to(bf).to(DEV) for _ in range(4))
+    qi, ki = (torch.randn(1, T, 4, 32, generator=g).to(bf).to(DEV) for _ in range(2))
+    w = torch.randn(4, generator=g).to(DEV)
+    o, idx, valid, scores, _ = swv.ops._dsa_forward(q, k, v, qi, ki, w, K)
+    run = lambda q, o: swv.ops.dsa_module_bwd(do, q, k, v, o, qi, ki, w, idx, valid, scores)
+    clean = run(q, o)
+    q, o = q.clone(), o.clone()
+    q[0, 1, 5], o[0, 1, 5] = float("nan"), float("nan")
+    got = run(q, o)
+    swv.check_status(DEV)
+    assert bool(got[0][0, 1, 5].isnan().all())
+    keep = torch.ones(1, H, T, dtype=torch.bool, device=DEV)
+    keep[0, 1, 5] = False
+    assert torch.equal(got[0][keep], clean[0][keep])
+    sel = idx[0, 5].long()
+    assert bool(got[1][0, 1, sel].isnan().all()) and bool(got[2][0, 1, sel].isnan().all())
+    assert torch.equal(got[1][0, 0], clean[1][0, 0]) and torch.equal(got[2][0, 0], clean[2][0, 0])
