@@ -113,7 +113,7 @@ class DeepSeekSparseAttention(nn.Module):
         qkv, q_idx, k_idx = self._project(x)
         if torch.is_grad_enabled() and (qkv.requires_grad or q_idx.requires_grad or
                                         self.indexer_head_weights.requires_grad):
-            # training: one differentiable op (fused forward, the two backward kernels chained)
+            # training: one differentiable op (fused forward, its backward on tiles or list kernels)
             qt, kt, vt = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]            # (B, T, H, D)
             if coords is not None:
                 if B != 1:

@@ -489,9 +489,10 @@ class DSAAttentionFunction(torch.autograd.Function):
 
 class DSAModuleFunction(torch.autograd.Function):
     """The module's whole attention step as ONE differentiable op: the forward is the fused path
-    (indexer + top-k + dense tensor-core attention, ``dsa_sparse_attention``), the backward chains
-    the two backward kernels the way autograd chains the reference's two Functions through
-    ``routing_weights = scores * valid`` (deepseek_sparse_attention.py:63-85)."""
+    (indexer + top-k + dense tensor-core attention, ``dsa_sparse_attention``), the backward is that of
+    the reference's two Functions chained through ``routing_weights = scores * valid``
+    (deepseek_sparse_attention.py:63-85): ``dsa_module_bwd`` where ``tile_backward_pays``, else the two
+    list kernels one after the other."""
 
     @staticmethod
     def forward(ctx, q, k, v, q_idx, k_idx, w, top_k, out_dtype):
