@@ -13,7 +13,8 @@
 //                           keys and every head of the group S = Q_h Kc^T on the tensor cores
 //                           (TMA rings -> tcgen05 -> two TMEM accumulators), eight epilogue warps
 //                           turn scores into probabilities and add them up per selection block.
-//   nsa_select_kernel     : one warp per (b, g, t): iterative arg-max over the importance row.
+//   nsa_select_short_kernel, nsa_select_kernel : one warp per (b, g, t): the n_sel largest of an importance row,
+//                           ranked among the few that can be, or by iterative arg-max.
 //   nsa_selected_attn_mma_kernel : one warp per (b, g, t), the G heads as columns of mma.sync tiles: every
 //                           selected key / value row is read once for the whole group
 //                           (nsa_selected_attn_kernel: the same on CUDA cores, for unaligned layouts).

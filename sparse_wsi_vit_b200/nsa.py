@@ -5,7 +5,7 @@ are the library-defined ones frozen in ``oracle/nsa.py`` (parity unpinned).
   compressed : `swv_pool_tokens` (mean pooling) + the block-sparse tensor-core kernel over ALL
                compressed tokens, grouped-query (kv_group), returning the log-sum-exp per row;
   selection  : `swv_nsa_select_blocks_fwd`: block importance recomputed on the tensor cores from
-               q, the compressed keys and the log-sum-exp, then an arg-max kernel per query;
+               q, the compressed keys and the log-sum-exp, then one warp selects per query;
   selected   : `swv_nsa_selected_attn_fwd`: one warp per (kv group, query) reads each selected
                key / value row once for all heads of the group (the heads are the columns of
                warp-level tensor-core tiles);
